@@ -3,14 +3,16 @@
 //   Quality_Fastest    -> icbc Level1: box fit + least squares
 //   Quality_Normal     -> icbc Level8: 4- and 3-colour cluster fit over all orderings
 //   Quality_Production -> icbc Level9: Level8 + endpoint refinement
-// One thread encodes one 4x4 block. The block's texels, its reduced colour set and its summed-area
-// table live in shared memory laid out [element][thread], so the data-dependent element indices of
-// the cluster-fit search never conflict on banks. The ordering index of the search loop is the
-// same in every thread of a warp, so ordering records are read as constant-cache broadcasts.
+// The cluster fits (k_bc1) take two blocks per warp and search one block's orderings with all its lanes,
+// through the scan of ntg_scan.cuh; Level1 (k_bc1_box) and the learned path's kernels take one block per
+// thread, the block's texels, reduced colours and summed-area table in shared memory.
 // Built with --fmad=false: results are bit-identical to the reference's scalar build.
+#include <memory>
+
 #include "ntg.h"
 #include "ntg_device.cuh"
 #include "ntg_internal.h"
+#include "ntg_scan.cuh"
 
 namespace ntg {
 
@@ -74,12 +76,22 @@ __device__ __forceinline__ f3 round_ept(f3 n, float f) {
 __device__ __forceinline__ bool is_black(f3 c) { return c.x < 1.0f / 8 && c.y < 1.0f / 8 && c.z < 1.0f / 8; }
 __device__ __forceinline__ f3 xyz(float4 v) { return mk3(v.x, v.y, v.z); }
 
+// v / 255 for the whole numbers 0..255
+static __constant__ float c_unit8[256];
+
 struct Pal3 { f3 p[4]; };
 __device__ __forceinline__ void palette_f(unsigned c0, unsigned c1, Pal3 &pf) {
     Pal8 p;
     palette_d3d10(c0, c1, p);
 #pragma unroll
     for (int i = 0; i < 4; i++) pf.p[i] = mk3(p.r[i] / 255.0f, p.g[i] / 255.0f, p.b[i] / 255.0f);
+}
+// The same where all lanes of a half-warp have the same end points: the quotients from a table.
+__device__ __forceinline__ void palette_half(unsigned c0, unsigned c1, Pal3 &pf) {
+    Pal8 p;
+    palette_d3d10(c0, c1, p);
+#pragma unroll
+    for (int i = 0; i < 4; i++) pf.p[i] = mk3(c_unit8[p.r[i]], c_unit8[p.g[i]], c_unit8[p.b[i]]);
 }
 
 // compute_indices4 (src/nvtt/icbc.h:2803-2835)
@@ -404,43 +416,6 @@ __device__ __forceinline__ float four_eval(const Lane<float4> &sat, uint32_t o, 
     return four_eval_v(v0, v1, sat[c2], sum, wsum, metric, a, b);
 }
 
-// The first strict minimum over all orderings wins, as in the scalar build. The search keeps the
-// index of the best ordering; its endpoints are recomputed once at the end. Over a ZERO table the
-// orderings are walked as the nest the table lists them in (last end t = 1..n, first end 0..t,
-// second end first..t: build_device_tables), so that the last and first ends' entries stay loaded.
-template <bool ZERO = false>
-__device__ void cluster_fit_four(const Lane<float4> &sat, int n, f3 metric, f3 &start, f3 &end) {
-    const float4 s = sat[ZERO ? n : n - 1];
-    const f3 sum = xyz(s);
-    const float wsum = s.w;
-    float best = FLT_MAX;
-    int bi = -1;
-    if (ZERO) {
-        int i = 0;
-        for (int t = 1; t <= n; t++) {
-            const float4 v2 = sat[t];
-            for (int c0 = 0; c0 <= t; c0++) {
-                const float4 v0 = sat[c0];
-                for (int c1 = c0; c1 <= t; c1++, i++) {
-                    f3 a, b;
-                    const float e = four_eval_v(v0, sat[c1], v2, sum, wsum, metric, a, b);
-                    if (e < best) { best = e; bi = i; }
-                }
-            }
-        }
-    } else {
-        const int total = c_tab.four_total[n - 1];
-        for (int i = 0; i < total; i++) {
-            f3 a, b;
-            const float e = four_eval<ZERO>(sat, c_tab.four[i], sum, wsum, metric, a, b);
-            if (e < best) { best = e; bi = i; }
-        }
-    }
-    start = mk3(0, 0, 0);
-    end = mk3(0, 0, 0);
-    if (bi >= 0) four_eval<ZERO>(sat, c_tab.four[bi], sum, wsum, metric, start, end);
-}
-
 // The full search's best ordering code (0 when none), for training targets.
 __device__ uint32_t best_order_four(const Lane<float4> &sat, int n, f3 metric) {
     const float4 s = sat[n - 1];
@@ -493,34 +468,34 @@ __device__ uint32_t best_order_three(const Lane<float4> &sat, int n, f3 metric) 
     return bo;
 }
 
-template <bool ZERO = false>
-__device__ void cluster_fit_three(const Lane<float4> &sat, int n, f3 metric, f3 &start, f3 &end) {
-    const float4 s = sat[ZERO ? n : n - 1];
-    const f3 sum = xyz(s);
-    const float wsum = s.w;
-    float best = FLT_MAX;
-    int bi = -1;
-    if (ZERO) {  // the table's nest: last end t = 1..n, first end 0..t
-        int i = 0;
-        for (int t = 1; t <= n; t++) {
-            const float4 v1 = sat[t];
-            for (int c0 = 0; c0 <= t; c0++, i++) {
-                f3 a, b;
-                const float e = three_eval_v(sat[c0], v1, sum, wsum, metric, a, b);
-                if (e < best) { best = e; bi = i; }
-            }
-        }
+// The orderings of c_tab.four and c_tab.three as the scan reads them (ntg_scan.cuh), padded to whole rows of 64: lanes
+// read different entries, which constant memory would serve one by one.
+static __device__ ScanOrders<512> g_orders4;
+static __device__ ScanOrders<96> g_orders3;
+
+// The exact evaluation of an ordering from its entries in a block's table and the table's last: four_eval_v, or
+// three_eval_v with v1 unused, the two differing only in the sums they hand to cf_eval.
+__device__ __forceinline__ float fit_eval(bool four, float4 v0, float4 v1, float4 v2, float4 s, f3 metric, f3 &a, f3 &b) {
+    const f3 x0 = xyz(v0);
+    float a2, b2, ab;
+    P3 ax;
+    const float last = s.w - v2.w;
+    if (four) {
+        const float w0 = v0.w, w2 = v2.w - v1.w, w1 = v1.w - w0;
+        const P3 x1 = p3_sub(p3(xyz(v1)), p3(x0)), x2 = p3_sub(p3(xyz(v2)), p3(xyz(v1)));
+        a2 = w2 * (1.0f / 9.0f) + (w1 * (4.0f / 9.0f) + w0);
+        b2 = w1 * (1.0f / 9.0f) + (w2 * (4.0f / 9.0f) + last);
+        ab = (w1 + w2) * (2.0f / 9.0f);
+        ax = p3_add(p3(u3(x2) * (1.0f / 3.0f)), p3_add(p3(u3(x1) * (2.0f / 3.0f)), p3(x0)));
     } else {
-        const int total = c_tab.three_total[n - 1];
-        for (int i = 0; i < total; i++) {
-            f3 a, b;
-            const float e = three_eval<ZERO>(sat, c_tab.three[i], sum, wsum, metric, a, b);
-            if (e < best) { best = e; bi = i; }
-        }
+        const float w1 = v2.w - v0.w;
+        const P3 x1 = p3_sub(p3(xyz(v2)), p3(x0));
+        ab = w1 * 0.25f;
+        a2 = v0.w + ab;
+        b2 = last + ab;
+        ax = p3_add(p3(x0), p3(u3(x1) * 0.5f));
     }
-    start = mk3(0, 0, 0);
-    end = mk3(0, 0, 0);
-    if (bi >= 0) three_eval<ZERO>(sat, c_tab.three[bi], sum, wsum, metric, start, end);
+    return cf_eval(ax, p3(xyz(s)), a2, b2, ab, metric, a, b);
 }
 
 // refine_endpoints (src/nvtt/icbc.h:3329-3406), including the reference's use of the current
@@ -659,265 +634,454 @@ __device__ __forceinline__ Block1 single_colour(float4 c) {
     return o;
 }
 
-template <int LEVEL>  // 0: icbc Level1, 7: Level8, 8: Level9
-__global__ void __launch_bounds__(64) k_bc1(const EncJob *__restrict__ jobs, int njobs, long long nblocks,
-                                            const long long *__restrict__ list, const unsigned long long *__restrict__ count) {
+// icbc Level1 (Quality_Fastest): one thread per block.
+__global__ void __launch_bounds__(64) k_bc1_box(const EncJob *__restrict__ jobs, int njobs, long long nblocks) {
     extern __shared__ float4 smem[];
     const int T = blockDim.x;
     const int t = threadIdx.x;
-    long long gblk = (long long)blockIdx.x * T + t;
+    const long long gblk = (long long)blockIdx.x * T + t;
     if (gblk >= nblocks) return;
-    if (list) {  // a subset of the jobs' blocks (the learned path's fallbacks), *count long
-        if ((unsigned long long)gblk >= *count) return;
-        gblk = list[gblk];
-    }
     const EncJob &J = jobs[find_job(jobs, njobs, gblk)];
     const int blk = (int)(gblk - J.first_block);
-    // 17 float4 slots per thread: the texels (16) and one more. The weights are derived from the
-    // texels when read (AlphaW). The reduced colours overwrite the texels in place (reduce_colors
-    // only writes slots it has already read), the summed-area table overwrites the colours in place
-    // with a zero entry first (17 entries), and the texels are gathered again for the output stage
-    // once the cluster fits are done.
     Lane<float4> in{smem + t, T};
-    Lane<float4> col = in;
-    Lane<float4> sat = in;
     const AlphaW wi{smem + t, T, J.alpha_mode == 1, valid_texels(J, blk)};
     const f3 cw = mk3(J.cw[0], J.cw[1], J.cw[2]);
-    uint8_t *const out = J.out + 8 * (size_t)blk;
-
     gather_block(J, blk, in, wi);
-
     Block1 o{0, 0, 0};
     float err = FLT_MAX;
-
-    if (LEVEL == 0) {
-        // Level1: box fit of all 16 texels, inset, diagonal, then least squares
-        // (src/nvtt/icbc.h:3096-3151, 2984-3016)
-        f3 c0 = mk3(0, 0, 0), c1 = mk3(1, 1, 1);
-        for (int i = 0; i < 16; i++) {
-            f3 p = xyz(in[i]);
-            c0 = mk3(ic_max(c0.x, p.x), ic_max(c0.y, p.y), ic_max(c0.z, p.z));
-            c1 = mk3(ic_min(c1.x, p.x), ic_min(c1.y, p.y), ic_min(c1.z, p.z));
-        }
-        const float bias = (8.0f / 255.0f) / 16.0f;
-        f3 d = c0 - c1;
-        f3 inset = mk3(d.x / 16.0f, d.y / 16.0f, d.z / 16.0f) - mk3(bias, bias, bias);
-        c0 = sat3(c0 - inset);
-        c1 = sat3(c1 + inset);
-        f3 center = (c0 + c1) * 0.5f;
-        float cxz = 0.0f, cyz = 0.0f;
-        for (int i = 0; i < 16; i++) { f3 tt = xyz(in[i]) - center; cxz += tt.x * tt.z; cyz += tt.y * tt.z; }
-        float x0 = c0.x, y0 = c0.y, x1 = c1.x, y1 = c1.y;
-        if (cxz < 0) { float tt = x0; x0 = x1; x1 = tt; }
-        if (cyz < 0) { float tt = y0; y0 = y1; y1 = tt; }
-        c0 = mk3(x0, y0, c0.z); c1 = mk3(x1, y1, c1.z);
-        err = output_block4(in, wi, cw, c0, c1, o);
-        // optimize_end_points4 on the 16 input texels
-        float a2 = 0, b2 = 0, ab = 0;
-        f3 ax = mk3(0, 0, 0), bxs = mk3(0, 0, 0);
-        for (int i = 0; i < 16; i++) {
-            unsigned bits = o.idx >> (2 * i);
-            float beta = (float)(bits & 1);
-            if (bits & 2) beta = (1 + beta) / 3.0f;
-            float alpha = 1.0f - beta;
-            f3 p = xyz(in[i]);
-            a2 += alpha * alpha; b2 += beta * beta; ab += alpha * beta;
-            ax = ax + p * alpha; bxs = bxs + p * beta;
-        }
-        float den = a2 * b2 - ab * ab;
-        if (!(fabsf(den - 0.0f) < 0.0001f)) {
-            float f = 1.0f / den;
-            f3 na = sat3(((ax * b2) - (bxs * ab)) * f);
-            f3 nb = sat3(((bxs * a2) - (ax * ab)) * f);
-            Block1 t2;
-            float e2 = output_block4(in, wi, cw, na, nb, t2);
-            if (e2 < err) { err = e2; o = t2; }
-        }
-        store_block(out, o);
-        return;
+    // Level1: box fit of all 16 texels, inset, diagonal, then least squares
+    // (src/nvtt/icbc.h:3096-3151, 2984-3016)
+    f3 c0 = mk3(0, 0, 0), c1 = mk3(1, 1, 1);
+    for (int i = 0; i < 16; i++) {
+        f3 p = xyz(in[i]);
+        c0 = mk3(ic_max(c0.x, p.x), ic_max(c0.y, p.y), ic_max(c0.z, p.z));
+        c1 = mk3(ic_min(c1.x, p.x), ic_min(c1.y, p.y), ic_min(c1.z, p.z));
     }
-
-    bool any_black = false;
-    const int cnt = reduce_colors(in, wi, col, any_black);
-
-    if (cnt == 0) {
-        store_block(out, Block1{0, 0, 0});
-        return;
+    const float bias = (8.0f / 255.0f) / 16.0f;
+    f3 d = c0 - c1;
+    f3 inset = mk3(d.x / 16.0f, d.y / 16.0f, d.z / 16.0f) - mk3(bias, bias, bias);
+    c0 = sat3(c0 - inset);
+    c1 = sat3(c1 + inset);
+    f3 center = (c0 + c1) * 0.5f;
+    float cxz = 0.0f, cyz = 0.0f;
+    for (int i = 0; i < 16; i++) { f3 tt = xyz(in[i]) - center; cxz += tt.x * tt.z; cyz += tt.y * tt.z; }
+    float x0 = c0.x, y0 = c0.y, x1 = c1.x, y1 = c1.y;
+    if (cxz < 0) { float tt = x0; x0 = x1; x1 = tt; }
+    if (cyz < 0) { float tt = y0; y0 = y1; y1 = tt; }
+    c0 = mk3(x0, y0, c0.z); c1 = mk3(x1, y1, c1.z);
+    err = output_block4(in, wi, cw, c0, c1, o);
+    // optimize_end_points4 on the 16 input texels
+    float a2 = 0, b2 = 0, ab = 0;
+    f3 ax = mk3(0, 0, 0), bxs = mk3(0, 0, 0);
+    for (int i = 0; i < 16; i++) {
+        unsigned bits = o.idx >> (2 * i);
+        float beta = (float)(bits & 1);
+        if (bits & 2) beta = (1 + beta) / 3.0f;
+        float alpha = 1.0f - beta;
+        f3 p = xyz(in[i]);
+        a2 += alpha * alpha; b2 += beta * beta; ab += alpha * beta;
+        ax = ax + p * alpha; bxs = bxs + p * beta;
     }
-    if (cnt == 1) {
-        store_block(out, single_colour(col[0]));
-        return;
+    float den = a2 * b2 - ab * ab;
+    if (!(fabsf(den - 0.0f) < 0.0001f)) {
+        float f = 1.0f / den;
+        f3 na = sat3(((ax * b2) - (bxs * ab)) * f);
+        f3 nb = sat3(((bxs * a2) - (ax * ab)) * f);
+        Block1 t2;
+        float e2 = output_block4(in, wi, cw, na, nb, t2);
+        if (e2 < err) { err = e2; o = t2; }
     }
+    store_block(J.out + 8 * (size_t)blk, o);
+}
+
+// ---------------------------------------------------------------------------------------------
+// The cluster fits, two blocks per warp. Lanes 0-15 hold the texels of one block and lanes 16-31 those of the next
+// (a texel each, in registers) through gathering, reducing, sorting and the output stage; sums whose order the
+// reference fixes are taken by one lane per accumulator from shared memory. The two searches then run one block
+// after the other with all 32 lanes on its orderings (ntg_scan.cuh).
+//
+// Bound by the FMA pipe: 19 rows of 64 orderings at about 112 instructions a row, half of them packed (two cycles
+// each). One thread per block, every ordering evaluated exactly (165 instructions each), needed 117,000 blocks to
+// fill the GPU; here a 64x64 chain's 341 blocks spread over the SMs. One float level, before and after: 64x64 75
+// and 24 us (8 lanes per block before), 256x256 75 and 34, 1024x1024 416 and 316, 2048x2048 1,317 and 1,228,
+// 1024x1024 after toSrgb 503 and 360 (texels gathered once instead of three times), 512x512 at Level9 627 and 200.
+
+constexpr unsigned kAll = 0xffffffffu;
+
+// One half's scratch in shared memory.
+struct HalfScratch {
+    float stage[16 * 8];  // terms per texel or colour
+    float pad[8];         // the two halves' stages lie on different banks
+    float4 table[2][18];  // the ZERO summed-area tables (17 entries) of the two fits
+    ScanBlock block[2];   // and their scans' constants
+    float ends[12];       // the fits' end points
+};
+struct WarpScratch {
+    ScanScratch scan;
+    HalfScratch half[2];
+};
+
+struct Half {
+    int hl;         // lane in the half: texel or colour index
+    int shift;      // first lane of the half
+    HalfScratch *s;
+    __device__ __forceinline__ float get(float v, int src) const { return __shfl_sync(kAll, v, src, 16); }
+    __device__ __forceinline__ unsigned ballot(bool p) const { return (__ballot_sync(kAll, p) >> shift) & 0xffffu; }
+    // Sum over i < n, in order, of the terms stage[8 i + c]; lane c of the half returns it.
+    __device__ __forceinline__ float ordered(int n) const {
+        float acc = 0.0f;
+        const float *p = s->stage + (hl & 7);
+#pragma unroll
+        for (int i = 0; i < 16; i++)
+            if (i < n) acc += p[8 * i];
+        return acc;
+    }
+};
+
+// reduce_colors (src/nvtt/icbc.h:1638-1683): the texels in order, each matched against the colours so far, which the
+// half's lanes hold one each. Returns the colour count.
+__device__ __forceinline__ int half_reduce(const Half &H, float4 texel, float4 &q) {
+    const float thr = 1.0f / 256;
+    int cnt = 0;
+    q = make_float4(0, 0, 0, 0);
+    // when no two texels match, the colours are the texels of positive weight (noise: most blocks)
+    bool match = false;
+#pragma unroll
+    for (int r = 1; r <= 8; r++) {
+        const int o = (H.hl + r) & 15;
+        const f3 c = mk3(H.get(texel.x, o), H.get(texel.y, o), H.get(texel.z, o));
+        match = match || (fabsf(texel.x - c.x) < thr && fabsf(texel.y - c.y) < thr && fabsf(texel.z - c.z) < thr);
+    }
+    if (!__any_sync(kAll, match || !(texel.w > 0))) {
+        q = texel;
+        return 16;
+    }
+#pragma unroll 1
+    for (int i = 0; i < 16; i++) {
+        const f3 c = mk3(H.get(texel.x, i), H.get(texel.y, i), H.get(texel.z, i));
+        const float wt = H.get(texel.w, i);
+        const unsigned m = H.ballot(H.hl < cnt && fabsf(q.x - c.x) < thr && fabsf(q.y - c.y) < thr && fabsf(q.z - c.z) < thr);
+        if (wt > 0) {
+            if (m == 0) {
+                if (H.hl == cnt) q = make_float4(c.x, c.y, c.z, wt);
+                cnt++;
+            } else if (H.hl == __ffs(m) - 1) {
+                const float den = q.w + wt;
+                const f3 s = (xyz(q) * q.w) + (c * wt);
+                q = make_float4(s.x / den, s.y / den, s.z / den, q.w + wt);
+            }
+        }
+    }
+    return cnt;
+}
+
+// compute_sat (src/nvtt/icbc.h:1812-1882) of the colours that lanes 0..n-1 of the half hold, into the half's table `which`
+// (a ZERO one: entry k holds the sum of the first k colours in principal-axis order, the entries above n that of
+// all), and the scan's constants.
+__device__ __noinline__ void half_sat(Half H, float4 q, int n, f3 metric, int which) {
+    float *const st = H.s->stage;
+    const int hl = H.hl;
+    // computeCentroid / computeCovariance (src/nvtt/icbc.h:1700-1741)
+    __syncwarp();
+    *reinterpret_cast<float4 *>(st + 8 * hl) = make_float4(q.x * q.w, q.y * q.w, q.z * q.w, q.w);
+    __syncwarp();
+    const float cs = H.ordered(n);
+    const float total = H.get(cs, 3);
+    const f3 c = mk3(H.get(cs, 0), H.get(cs, 1), H.get(cs, 2)) * (1.0f / total);
+    const f3 a = xyz(q) - c, b = a * q.w;
+    __syncwarp();
+    *reinterpret_cast<float4 *>(st + 8 * hl) = make_float4(a.x * b.x, a.x * b.y, a.x * b.z, a.y * b.y);
+    *reinterpret_cast<float2 *>(st + 8 * hl + 4) = make_float2(a.y * b.z, a.z * b.z);
+    __syncwarp();
+    const float ms = H.ordered(n);
+    const float m0 = H.get(ms, 0), m1 = H.get(ms, 1), m2 = H.get(ms, 2), m3 = H.get(ms, 3), m4 = H.get(ms, 4), m5 = H.get(ms, 5);
+    // firstEigenVector_PowerMethod (src/nvtt/icbc.h:1760-1790)
+    f3 v = mk3(0, 0, 0);
+    if (!(m0 == 0 && m3 == 0 && m5 == 0)) {
+        const f3 r0 = mk3(m0, m1, m2), r1 = mk3(m1, m3, m4), r2 = mk3(m2, m4, m5);
+        const float l0 = dot(r0, r0), l1 = dot(r1, r1), l2 = dot(r2, r2);
+        v = (l0 > l1 && l0 > l2) ? r0 : (l1 > l2 ? r1 : r2);
+#pragma unroll 1
+        for (int it = 0; it < 8; it++) {
+            const float x = v.x * m0 + v.y * m1 + v.z * m2;
+            const float y = v.x * m1 + v.y * m3 + v.z * m4;
+            const float z = v.x * m2 + v.y * m4 + v.z * m5;
+            const float norm = ic_max(ic_max(x, y), z);
+            v = mk3(x, y, z) * (1.0f / norm);
+        }
+    }
+    __syncwarp();
+    // positions along the axis in a stable insertion sort's order: the rank, unless a projection is NaN
+    const float d = dot(xyz(q), v);
+    int rank = 0;
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+        const float e = H.get(d, j);
+        rank += j < n && (e < d || (e == d && j < hl));
+    }
+    const bool odd = H.ballot(hl < n && d != d) != 0;
+    if (__any_sync(kAll, odd)) {
+        float *const key = st;
+        int *const ord = reinterpret_cast<int *>(st + 16), *const pos = reinterpret_cast<int *>(st + 32);
+        __syncwarp();
+        key[hl] = d;
+        __syncwarp();
+        if (hl == 0) {
+            for (int i = 0; i < n; i++) ord[i] = i;
+            for (int i = 1; i < n; i++)
+                for (int j = i; j > 0 && key[j] < key[j - 1]; j--) {
+                    const float t = key[j]; key[j] = key[j - 1]; key[j - 1] = t;
+                    const int o = ord[j]; ord[j] = ord[j - 1]; ord[j - 1] = o;
+                }
+            for (int i = 0; i < n; i++) pos[ord[i]] = i;
+        }
+        __syncwarp();
+        if (odd && hl < n) rank = pos[hl];
+        __syncwarp();
+    }
+    if (hl < n) *reinterpret_cast<float4 *>(st + 4 * rank) = make_float4(q.x * q.w, q.y * q.w, q.z * q.w, q.w);
+    __syncwarp();
+    float acc = 0.0f;
+    if (hl < 4) {
+        float *const t = reinterpret_cast<float *>(H.s->table[which]) + hl;
+        t[0] = 0.0f;
+        acc = st[hl];
+        t[4] = acc;
+#pragma unroll
+        for (int i = 1; i < 16; i++)
+            { if (i < n) acc += st[4 * i + hl]; t[4 * (i + 1)] = acc; }
+    }
+    // the scan's constants
+    float big = hl < n ? max3_abs(q.x, q.y, q.z) : 0.0f;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(kAll, big, o));
+    const bool whole = H.ballot(hl < n && q.w != floorf(q.w)) == 0;
+    const f3 sum = mk3(H.get(acc, 0), H.get(acc, 1), H.get(acc, 2));
+    const float wsum = H.get(acc, 3);
+    if (hl == 0) scan_begin(H.s->block[which], n, sum, wsum, big, m0 + m3 + m5, whole, metric, 46.0f, 47.0f);
+    __syncwarp();
+}
+
+// Both cluster fits (cluster_fit_four, cluster_fit_three) of the warp's block b by all lanes: n4 and n3 colours (n3 = 0:
+// no three-colour fit); the end points to the half's `ends`. own3: the three-colour fit has its own table.
+__device__ __forceinline__ void warp_fit(WarpScratch &w, int b, int n4, int n3, bool own3, bool unit) {
+    const int lane = threadIdx.x & 31;
+    HalfScratch &h = w.half[b];
+    const float4 *const table3 = h.table[own3];
+    scan_centre(w.scan, h.block[0], h.table[0]);
+    const uint32_t bits4 = scan_bits(w.scan, h.block[0], g_orders4, (c_tab.four_total[n4 - 1] + 63) >> 6, 0, 3.0f, unit);
+    uint32_t bits3 = 0;
+    if (n3 > 0) {
+        if (own3) scan_centre(w.scan, h.block[1], table3);
+        bits3 = scan_bits(w.scan, h.block[own3], g_orders3, (c_tab.three_total[n3 - 1] + 63) >> 6, 16, 2.0f, unit);
+    }
+    __syncwarp();
+    uint16_t *const list = reinterpret_cast<uint16_t *>(w.scan.e);
+    int count = 0;
+    scan_list(list, count, bits4, 0x8000);
+    scan_list(list, count, bits3, 0);
+    __syncwarp();
+    const f3 metric = mk3(h.block[0].metric[0], h.block[0].metric[1], h.block[0].metric[2]);
+    FitBest best4, best3;
+#pragma unroll 1
+    for (int i = lane; i < count; i += 32) {
+        const int it = list[i], o = it & 0x7fff;
+        const bool four = (it & 0x8000) != 0;
+        const uint32_t ends = four ? scan_ends(g_orders4, o) : scan_ends(g_orders3, o), t = shared_address(four ? h.table[0] : table3);
+        f3 ea, eb;
+        const float e = fit_eval(four, load_shared(t + (ends & 1023)), load_shared(t + ((ends >> 10) & 1023)), load_shared(t + (ends >> 20)),
+                                 load_shared(t + 16 * 16), metric, ea, eb);
+        if (four) best4.take(e, o, ea, eb);
+        else best3.take(e, o, ea, eb);
+    }
+    best4.finish(h.ends);
+    best3.finish(h.ends + 6);
+    __syncwarp();
+}
+
+// Bit i of m to bit 2 i.
+__device__ __forceinline__ uint32_t spread_bits(uint32_t m) {
+    m = (m | (m << 8)) & 0x00ff00ffu;
+    m = (m | (m << 4)) & 0x0f0f0f0fu;
+    m = (m | (m << 2)) & 0x33333333u;
+    return (m | (m << 1)) & 0x55555555u;
+}
+
+// evaluate_mse over the input texels (src/nvtt/icbc.h:2733-2756): lane k's texel has index code k.
+__device__ __forceinline__ float half_mse(const Half &H, float4 texel, f3 cw, const Pal3 &pal, unsigned code) {
+    const f3 p = code == 0 ? pal.p[0] : (code == 1 ? pal.p[1] : (code == 2 ? pal.p[2] : pal.p[3]));
+    const f3 d = ((p - xyz(texel)) * cw) * 255.0f;
+    __syncwarp();
+    H.s->stage[H.hl] = texel.w * dot(d, d);
+    __syncwarp();
+    float err = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float4 t = reinterpret_cast<const float4 *>(H.s->stage)[i];
+        err += t.x; err += t.y; err += t.z; err += t.w;
+    }
+    return err;
+}
+
+// output_block4 / output_block3 (compute_indices4 / compute_indices3, src/nvtt/icbc.h:2803-2882).
+template <bool FOUR>
+__device__ __forceinline__ float half_output(const Half &H, float4 texel, f3 cw, f3 v0, f3 v1, Block1 &o) {
+    unsigned c0 = to565(v0), c1 = to565(v1);
+    if (FOUR ? c0 < c1 : c0 > c1) { const unsigned t = c0; c0 = c1; c1 = t; }
+    Pal3 pal;
+    palette_half(c0, c1, pal);
+    const f3 c = xyz(texel) * cw;
+    f3 t;
+    unsigned hi, lo;
+    if (FOUR) {
+        t = c - pal.p[0] * cw; const float d0 = dot(t, t);
+        t = c - pal.p[1] * cw; const float d1 = dot(t, t);
+        t = c - pal.p[2] * cw; const float d2 = dot(t, t);
+        t = c - pal.p[3] * cw; const float d3 = dot(t, t);
+        hi = ((d1 > d2) & (d0 > d2)) | ((d0 > d3) & (d1 > d3));
+        lo = (d0 > d3) & (d2 > d3);
+    } else {
+        t = pal.p[0] * cw - c; const float d0 = dot(t, t);
+        t = pal.p[1] * cw - c; const float d1 = dot(t, t);
+        t = pal.p[2] * cw - c; const float d2 = dot(t, t);
+        const float d3 = dot(c, c);
+        const unsigned i1 = d1 < d2, i2 = (d2 <= d0) & (d2 <= d1), i3 = (d3 <= d0) & (d3 <= d1) & (d3 <= d2);
+        hi = i2 | i3; lo = i1 | i3;
+    }
+    o.c0 = c0; o.c1 = c1;
+    o.idx = (spread_bits(H.ballot(hi)) << 1) | spread_bits(H.ballot(lo));
+    return half_mse(H, texel, cw, pal, (hi << 1) | lo);
+}
+
+// refine_endpoints (src/nvtt/icbc.h:3329-3406), including the reference's use of the current output's palette
+// (not the candidate's) for index selection (compute_indices, live branch, src/nvtt/icbc.h:2885-2941). `run`: this
+// half's block takes part.
+__device__ __forceinline__ float half_refine(const Half &H, float4 texel, f3 cw, float err, Block1 &o, bool run) {
+    const int8_t deltas[16][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {-1, 0, 0}, {0, -1, 0}, {0, 0, -1},
+                                  {1, 1, 0}, {1, 0, 1}, {0, 1, 1}, {-1, -1, 0}, {-1, 0, -1}, {0, -1, -1},
+                                  {-1, 1, 0}, {1, -1, 0}, {0, -1, 1}, {0, 1, -1}};
+    float best = err;
+    int last = 0;
+    const f3 c = xyz(texel) * cw;
+#pragma unroll 1
+    for (int i = 0; i < 256; i++) {
+        Block1 r = o;
+        const int8_t *d = deltas[i % 16];
+        unsigned e = ((i / 16) & 1) ? r.c0 : r.c1;
+        const unsigned er = ((e >> 11) + d[0]) & 31, eg = (((e >> 5) & 63) + d[1]) & 63, eb = ((e & 31) + d[2]) & 31;
+        e = (er << 11) | (eg << 5) | eb;
+        if ((i / 16) & 1) r.c0 = e; else r.c1 = e;
+        Pal3 pal;
+        palette_half(o.c0, o.c1, pal);
+        f3 t;
+        t = c - pal.p[0] * cw; const float d0 = dot(t, t);
+        t = c - pal.p[1] * cw; const float d1 = dot(t, t);
+        t = c - pal.p[2] * cw; const float d2 = dot(t, t);
+        t = c - pal.p[3] * cw; const float d3 = dot(t, t);
+        const unsigned i1 = (d1 <= d0) & (d1 < d2) & (d1 < d3);
+        const unsigned i2 = (d2 <= d0) & (d2 <= d1) & (d2 < d3);
+        const unsigned i3 = (d3 <= d0) & (d3 <= d1) & (d3 <= d2);
+        const unsigned hi = i2 | i3, lo = i1 | i3;
+        r.idx = (spread_bits(H.ballot(hi)) << 1) | spread_bits(H.ballot(lo));
+        Pal3 rp;
+        palette_half(r.c0, r.c1, rp);
+        const float x = half_mse(H, texel, cw, rp, (hi << 1) | lo);
+        if (run && x < best) { best = x; o = r; last = i; }
+        if (i - last > 32) run = false;
+        if (!__any_sync(kAll, run)) break;
+    }
+    return best;
+}
+
+// FloatColorCompressorTask gather (src/nvtt/BlockCompressor.cpp:116-166) of texel k of a block: colour after the
+// output transform, weight saturate(alpha) under AlphaMode_Transparency, 0 outside the image.
+__device__ __forceinline__ float4 gather_texel(const EncJob &J, int blk, int k) {
+    const int x = (blk % J.bw) * 4 + (k & 3), y = (blk / J.bw) * 4 + (k >> 2);
+    if (x >= J.w || y >= J.h) return make_float4(0, 0, 0, 0);
+    const size_t n = (size_t)J.w * J.h, s = (size_t)y * J.w + x;
+    float r, g, b, al;
+    if (J.bgra) {
+        // 8-bit source through the composed input/output transform table
+        const uint32_t p = J.bgra[s];
+        r = J.lut_f[(p >> 16) & 255]; g = J.lut_f[(p >> 8) & 255]; b = J.lut_f[p & 255];
+        al = (float)(p >> 24) / 255.0f;
+    } else {
+        r = J.rgba[s]; g = J.rgba[n + s]; b = J.rgba[2 * n + s]; al = J.rgba[3 * n + s];
+        if (J.out_xform == 1) { r = powf_5_11(r); g = powf_5_11(g); b = powf_5_11(b); }
+        else if (J.out_xform == 2) { r = to_srgb(r); g = to_srgb(g); b = to_srgb(b); }
+    }
+    return make_float4(r, g, b, J.alpha_mode == 1 ? ic_clamp(al, 0.0f, 1.0f) : 1.0f);
+}
+
+#ifndef NTG_BC1_MIN_CTAS
+#define NTG_BC1_MIN_CTAS 5
+#endif
+constexpr int kFitWarps = 4;  // warps per CTA, each on its own
+
+// icbc Level8 (LEVEL 7) and Level9 (LEVEL 8).
+template <int LEVEL>
+__global__ void __launch_bounds__(32 * kFitWarps, NTG_BC1_MIN_CTAS) k_bc1(const EncJob *__restrict__ jobs, int njobs, long long nblocks,
+                                                                         const long long *__restrict__ list,
+                                                                         const unsigned long long *__restrict__ count) {
+    __shared__ WarpScratch scratch[kFitWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    WarpScratch &w = scratch[warp];
+    const Half H{lane & 15, lane & 16, &w.half[lane >> 4]};
+    // `list`: a subset of the jobs' blocks (the learned path's fallbacks), *count long
+    const long long total = list ? min(nblocks, (long long)*count) : nblocks;
+    const long long first = 2 * ((long long)blockIdx.x * kFitWarps + warp);
+    if (first >= total) return;
+    long long gblk = first + (lane >> 4);
+    const bool live = gblk < total;  // the last warp's second half may have no block
+    if (!live) gblk = first;
+    if (list) gblk = list[gblk];
+    const EncJob &J = jobs[find_job(jobs, njobs, gblk)];
+    const int blk = (int)(gblk - J.first_block);
+    const f3 cw = mk3(J.cw[0], J.cw[1], J.cw[2]);
+    const f3 metric = cw * cw;
+    const bool unit = __all_sync(kAll, metric.x == 1.0f && metric.y == 1.0f && metric.z == 1.0f) != 0;
+    uint8_t *const out = J.out + 8 * (size_t)blk;
+
+    const float4 texel = gather_texel(J, blk, H.hl);
+    float4 q;
+    const int cnt = half_reduce(H, texel, q);
+    const bool black = H.ballot(texel.w > 0 && is_black(xyz(texel))) != 0;
+    if (live && H.hl == 0 && cnt <= 1) store_block(out, cnt == 0 ? Block1{0, 0, 0} : single_colour(q));
+    const bool fit = live && cnt > 1;
+    if (!__any_sync(kAll, fit)) return;
 
     // compress_dxt1_cluster_fit (src/nvtt/icbc.h:3292-3325); both fits first, then the output stage
     // (pure functions of the texels and the endpoints, so their order does not matter)
-    const f3 metric = cw * cw;
-    int sn = compute_sat_inplace(col, cnt);
-    f3 s0, s1, t0, t1;
-    cluster_fit_four<true>(sat, sn, metric, s0, s1);
-    bool run3 = true;
-    if (any_black) {
-        // the table has replaced the colours: reduce them again (the same colours), then
-        // skip_blacks in place, compacting the non-black ones to the front of `col`
-        gather_block(J, blk, in, wi);
-        bool again = false;
-        reduce_colors(in, wi, col, again);
-        int m = 0;
-        for (int i = 0; i < cnt; i++) {
-            float4 q = col[i];
-            if (is_black(xyz(q))) continue;
-            col[m++] = q;
-        }
-        if (m == 0) run3 = false;
-        else sn = compute_sat_inplace(col, m);
+    half_sat(H, q, cnt, metric, 0);
+    int n3 = fit ? cnt : 0;
+    if (__any_sync(kAll, fit && black)) {
+        // skip_blacks: the other colours, moved up to the first lanes
+        const unsigned keep = H.ballot(H.hl < cnt && !is_black(xyz(q)));
+        const int src = (int)__fns(keep, 0, H.hl + 1) & 15;
+        const float4 c = make_float4(H.get(q.x, src), H.get(q.y, src), H.get(q.z, src), H.get(q.w, src));
+        if (fit && black) n3 = __popc(keep);
+        half_sat(H, c, __popc(keep), metric, 1);
     }
-    if (run3) cluster_fit_three<true>(sat, sn, metric, t0, t1);
-    gather_block(J, blk, in, wi);
-    Block1 cf;
-    float cerr = output_block4(in, wi, cw, s0, s1, cf);
-    if (run3) {
-        Block1 c3;
-        float e3 = output_block3(in, wi, cw, true, t0, t1, c3);
-        if (e3 < cerr) { cerr = e3; cf = c3; }
+#pragma unroll 1
+    for (int b = 0; b < 2; b++) {
+        const int n4 = __shfl_sync(kAll, fit ? cnt : 0, 16 * b), bn3 = __shfl_sync(kAll, n3, 16 * b);
+        const bool own3 = __shfl_sync(kAll, (int)black, 16 * b) != 0;
+        if (n4 > 0) warp_fit(w, b, n4, bn3, own3, unit);
     }
+    const float *const ends = H.s->ends;
+    const f3 s0 = mk3(ends[0], ends[1], ends[2]), s1 = mk3(ends[3], ends[4], ends[5]);
+    const f3 t0 = mk3(ends[6], ends[7], ends[8]), t1 = mk3(ends[9], ends[10], ends[11]);
+    Block1 cf, c3;
+    float cerr = half_output<true>(H, texel, cw, s0, s1, cf);
+    const float e3 = half_output<false>(H, texel, cw, t0, t1, c3);
+    if (n3 > 0 && e3 < cerr) { cerr = e3; cf = c3; }
     // taken only when its error compares below FLT_MAX: a NaN error leaves the block as the
     // reference leaves it unwritten (this build writes zeros there)
-    if (cerr < err) { o = cf; err = cerr; }
-    if (LEVEL == 8) err = refine_endpoints(in, wi, cw, err, o);
-    store_block(out, o);
-}
-
-// The first strict minimum of a search split over the K lanes of a group, lane j having taken the
-// orderings i = j (mod K) with its own first strict minimum (e, i) (FLT_MAX, -1 when none): the
-// smallest error, and among equal errors the smallest ordering - the ordering the sequential search
-// keeps. Every lane of the group returns it.
-template <int K>
-__device__ __forceinline__ int group_first_min(unsigned gmask, float e, int i) {
-#pragma unroll
-    for (int off = K / 2; off > 0; off >>= 1) {
-        const float eo = __shfl_xor_sync(gmask, e, off, K);
-        const int io = __shfl_xor_sync(gmask, i, off, K);
-        if (eo < e || (eo == e && io < i)) { e = eo; i = io; }
-    }
-    return i;
-}
-
-// cluster_fit_four / cluster_fit_three over a ZERO table, lane j of K evaluating the orderings
-// j, j + K, ... of the icbc tables (listed in the sequential search's order); returns the group's best
-// ordering (-1 when none).
-template <int K>
-__device__ int split_fit_four(unsigned gmask, const Lane<float4> &sat, int n, f3 metric, int j) {
-    const float4 s = sat[n];
-    const f3 sum = xyz(s);
-    float best = FLT_MAX;
-    int bi = -1;
-    const int total = c_tab.four_total[n - 1];
-    for (int i = j; i < total; i += K) {
-        f3 a, b;
-        const float e = four_eval<true>(sat, c_tab.four[i], sum, s.w, metric, a, b);
-        if (e < best) { best = e; bi = i; }
-    }
-    return group_first_min<K>(gmask, best, bi);
-}
-template <int K>
-__device__ int split_fit_three(unsigned gmask, const Lane<float4> &sat, int n, f3 metric, int j) {
-    const float4 s = sat[n];
-    const f3 sum = xyz(s);
-    float best = FLT_MAX;
-    int bi = -1;
-    const int total = c_tab.three_total[n - 1];
-    for (int i = j; i < total; i += K) {
-        f3 a, b;
-        const float e = three_eval<true>(sat, c_tab.three[i], sum, s.w, metric, a, b);
-        if (e < best) { best = e; bi = i; }
-    }
-    return group_first_min<K>(gmask, best, bi);
-}
-
-// k_bc1 for launches too small to fill the GPU with one thread per block: a group of K lanes of one
-// warp encodes each block (64 / K blocks per 64-thread CTA). The group's first lane gathers, reduces
-// and builds the summed-area table, in 17 float4 slots of shared memory per block; the K lanes split
-// the orderings of each cluster fit; the first lane recomputes the winners' endpoints and runs the
-// output stage. The same operations on the same values as k_bc1, so the same blocks.
-template <int LEVEL, int K>
-__global__ void __launch_bounds__(64) k_bc1_split(const EncJob *__restrict__ jobs, int njobs, long long nblocks) {
-    extern __shared__ float4 smem[];
-    constexpr int G = 64 / K;  // blocks per CTA
-    const int t = threadIdx.x, g = t / K, j = t % K;
-    const long long gblk = (long long)blockIdx.x * G + g;
-    if (gblk >= nblocks) return;  // the whole group leaves together
-    const unsigned gmask = ((1u << K) - 1u) << ((t & 31) & ~(K - 1));
-    const EncJob &J = jobs[find_job(jobs, njobs, gblk)];
-    const int blk = (int)(gblk - J.first_block);
-    Lane<float4> in{smem + 17 * g, 1};  // one block's slots, consecutive: the lanes read different ones
-    Lane<float4> col = in;
-    Lane<float4> sat = in;
-    const AlphaW wi{smem + 17 * g, 1, J.alpha_mode == 1, valid_texels(J, blk)};
-    const f3 cw = mk3(J.cw[0], J.cw[1], J.cw[2]);
-    const f3 metric = cw * cw;
-    uint8_t *const out = J.out + 8 * (size_t)blk;
-
-    int cnt = 0, sn = 0, black = 0;
-    if (j == 0) {
-        gather_block(J, blk, in, wi);
-        bool any_black = false;
-        cnt = reduce_colors(in, wi, col, any_black);
-        black = any_black;
-        if (cnt == 0) store_block(out, Block1{0, 0, 0});
-        else if (cnt == 1) store_block(out, single_colour(col[0]));
-        else sn = compute_sat_inplace(col, cnt);
-    }
-    cnt = __shfl_sync(gmask, cnt, 0, K);
-    if (cnt <= 1) return;
-    sn = __shfl_sync(gmask, sn, 0, K);
-    black = __shfl_sync(gmask, black, 0, K);
-    __syncwarp(gmask);  // the table is written
-
-    f3 s0 = mk3(0, 0, 0), s1 = mk3(0, 0, 0), t0 = mk3(0, 0, 0), t1 = mk3(0, 0, 0);
-    const int b4 = split_fit_four<K>(gmask, sat, sn, metric, j);
-    int run3 = 1;
-    if (j == 0) {
-        if (b4 >= 0) four_eval<true>(sat, c_tab.four[b4], xyz(sat[sn]), sat[sn].w, metric, s0, s1);
-    }
-    __syncwarp(gmask);  // every lane is done with the table
-    if (black) {
-        if (j == 0) {
-            // the table has replaced the colours: reduce them again, then keep the non-black ones
-            gather_block(J, blk, in, wi);
-            bool again = false;
-            reduce_colors(in, wi, col, again);
-            int m = 0;
-            for (int i = 0; i < cnt; i++) {
-                float4 q = col[i];
-                if (is_black(xyz(q))) continue;
-                col[m++] = q;
-            }
-            if (m == 0) run3 = 0;
-            else sn = compute_sat_inplace(col, m);
-        }
-        run3 = __shfl_sync(gmask, run3, 0, K);
-        sn = __shfl_sync(gmask, sn, 0, K);
-        __syncwarp(gmask);
-    }
-    if (run3) {
-        const int b3 = split_fit_three<K>(gmask, sat, sn, metric, j);
-        if (j == 0 && b3 >= 0) three_eval<true>(sat, c_tab.three[b3], xyz(sat[sn]), sat[sn].w, metric, t0, t1);
-        __syncwarp(gmask);
-    }
-    if (j != 0) return;
-    gather_block(J, blk, in, wi);
     Block1 o{0, 0, 0};
     float err = FLT_MAX;
-    Block1 cf;
-    float cerr = output_block4(in, wi, cw, s0, s1, cf);
-    if (run3) {
-        Block1 c3;
-        const float e3 = output_block3(in, wi, cw, true, t0, t1, c3);
-        if (e3 < cerr) { cerr = e3; cf = c3; }
-    }
     if (cerr < err) { o = cf; err = cerr; }
-    if (LEVEL == 8) err = refine_endpoints(in, wi, cw, err, o);
-    store_block(out, o);
+    if (LEVEL == 8) err = half_refine(H, texel, cw, err, o, fit);
+    if (fit && H.hl == 0) store_block(out, o);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1414,40 +1578,20 @@ static size_t bc1_fit_smem(int T) { return (size_t)T * 17 * sizeof(float4); }
 // k_bc1_work: per thread the texels and 16 stored weights.
 static size_t bc1_work_smem(int T) { return (size_t)T * (16 * sizeof(float4) + 16 * sizeof(float)); }
 
-// Blocks the one-thread-per-block fit keeps in flight on a full GB300 (152 SMs x 12 CTAs of 64).
-constexpr long long kBc1InFlight = 152LL * 12 * 64;
-
-template <int LEVEL, int K>
-static void launch_bc1_split(const EncJob *d_jobs, int njobs, long long nblocks, cudaStream_t stream) {
-    constexpr int G = 64 / K;
-    k_bc1_split<LEVEL, K><<<(unsigned)((nblocks + G - 1) / G), 64, (size_t)G * 17 * sizeof(float4), stream>>>(
-        d_jobs, njobs, nblocks);
+template <int LEVEL>
+static int launch_bc1_fit(const EncJob *d_jobs, int njobs, long long nblocks, const long long *list, const unsigned long long *count,
+                          cudaStream_t stream) {
+    const long long per = 2 * kFitWarps;
+    k_bc1<LEVEL><<<(unsigned)((nblocks + per - 1) / per), 32 * kFitWarps, 0, stream>>>(d_jobs, njobs, nblocks, list, count);
+    return launch_status();
 }
 
 int launch_bc1(const EncJob *d_jobs, int njobs, long long nblocks, int quality, int threads, cudaStream_t stream) {
     if (nblocks == 0) return 0;
-    if (quality != 0 && nblocks * 4 <= 2 * kBc1InFlight) {
-        // too few blocks to keep the SMs busy one thread each (a single 512x512 chain has 21,847):
-        // 8 or 4 lanes per block, for up to two waves of threads
-        const bool eight = nblocks * 8 <= 2 * kBc1InFlight;
-        if (quality == 2) eight ? launch_bc1_split<8, 8>(d_jobs, njobs, nblocks, stream)
-                                : launch_bc1_split<8, 4>(d_jobs, njobs, nblocks, stream);
-        else eight ? launch_bc1_split<7, 8>(d_jobs, njobs, nblocks, stream)
-                   : launch_bc1_split<7, 4>(d_jobs, njobs, nblocks, stream);
-        return launch_status();
-    }
+    if (quality == 2) return launch_bc1_fit<8>(d_jobs, njobs, nblocks, nullptr, nullptr, stream);
+    if (quality != 0) return launch_bc1_fit<7>(d_jobs, njobs, nblocks, nullptr, nullptr, stream);
     const int T = threads == 32 ? 32 : 64;  // blocks per CTA (one thread per 4x4 block)
-    const size_t sm = bc1_fit_smem(T);
-    const unsigned grid = (unsigned)((nblocks + T - 1) / T);
-    static std::atomic<unsigned long long> configured{0};
-    if (first_use_on_device(configured)) {  // the per-thread arrays exceed the 48 KB default
-        cudaFuncSetAttribute(k_bc1<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        cudaFuncSetAttribute(k_bc1<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        cudaFuncSetAttribute(k_bc1<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    }
-    if (quality == 0) k_bc1<0><<<grid, T, sm, stream>>>(d_jobs, njobs, nblocks, nullptr, nullptr);
-    else if (quality == 2) k_bc1<8><<<grid, T, sm, stream>>>(d_jobs, njobs, nblocks, nullptr, nullptr);
-    else k_bc1<7><<<grid, T, sm, stream>>>(d_jobs, njobs, nblocks, nullptr, nullptr);
+    k_bc1_box<<<(unsigned)((nblocks + T - 1) / T), T, bc1_fit_smem(T), stream>>>(d_jobs, njobs, nblocks);
     return launch_status();
 }
 
@@ -1499,13 +1643,19 @@ int launch_bc1_work(const EncJob *d_jobs, int njobs, long long nblocks, unsigned
 int launch_bc1_list(const EncJob *d_jobs, int njobs, const long long *list, const unsigned long long *d_count,
                     long long max_count, cudaStream_t s) {
     if (max_count == 0) return 0;
-    const int T = 64;
-    static std::atomic<unsigned long long> configured{0};
-    allow_smem(k_bc1<7>, bc1_fit_smem(T), configured);
-    k_bc1<7><<<(unsigned)((max_count + T - 1) / T), T, bc1_fit_smem(T), s>>>(d_jobs, njobs, max_count, list, d_count);
-    return launch_status();
+    return launch_bc1_fit<7>(d_jobs, njobs, max_count, list, d_count, s);
 }
 
-NTG_DEFINE_TABLE_UPLOAD(upload_tables_bc1)
+int upload_tables_bc1(const HostTables &t) {
+    const std::unique_ptr<ScanOrders<512>> o4(new ScanOrders<512>);
+    ScanOrders<96> o3;
+    float unit8[256];
+    for (int v = 0; v < 256; v++) unit8[v] = (float)v / 255.0f;
+    scan_orders<3>(t.four, t.four_total[15], *o4);
+    scan_orders<2>(t.three, t.three_total[15], o3);
+    return cudaMemcpyToSymbol(c_tab, &t, sizeof t) == cudaSuccess && cudaMemcpyToSymbol(g_orders4, o4.get(), sizeof *o4) == cudaSuccess &&
+                   cudaMemcpyToSymbol(g_orders3, &o3, sizeof o3) == cudaSuccess && cudaMemcpyToSymbol(c_unit8, unit8, sizeof unit8) == cudaSuccess
+               ? 0 : 3;
+}
 
 }  // namespace ntg

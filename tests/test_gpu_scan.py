@@ -1,0 +1,54 @@
+"""The cluster fits' scan (ntg_scan.cuh) against the oracle, block for block, on the contents whose bounds
+are tightest: nearly flat blocks (every ordering a possible winner), end points on snapping ties, tiny and
+unequal weights, colours below the black threshold, values outside [0, 1], NaN and infinities; and on block
+counts that leave a warp's second half or a CTA's last warps without a block."""
+import numpy as np
+import pytest
+
+import ntg
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+def contents(kind, w, h, seed):
+    rng = np.random.default_rng(seed)
+    rgb = rng.random((3, h, w)).astype(np.float32)
+    a = rng.random((h, w)).astype(np.float32)
+    if kind == "flat":        # a few steps of 1 / 255 around a colour
+        rgb = (0.5 + rng.integers(-1, 2, (3, h, w)) / 255.0).astype(np.float32)
+    elif kind == "faint":     # just above the merging threshold
+        rgb = (rng.random((3, 1, 1)) + rng.random((3, h, w)) / 60.0).astype(np.float32)
+    elif kind == "grid":      # colours on the 5:6:5 grid and half way between its points
+        rgb = np.stack([rng.integers(0, 63, (h, w)) / 62.0, rng.integers(0, 127, (h, w)) / 126.0,
+                        rng.integers(0, 63, (h, w)) / 62.0]).astype(np.float32)
+    elif kind == "dark":
+        rgb *= 0.2
+    elif kind == "weights":   # alphas over five orders of magnitude
+        a = (10.0 ** -rng.uniform(0, 5, (h, w))).astype(np.float32)
+    elif kind == "wide":      # beyond what the scan's bound covers
+        rgb = (rgb * 6 - 3).astype(np.float32)
+    elif kind == "odd":
+        rgb[rng.random(rgb.shape) < 0.05] = np.nan
+        rgb[rng.random(rgb.shape) < 0.02] = np.inf
+    elif kind == "ramp":      # noise around a gradient, as smooth textures have it
+        rgb = (0.3 + 0.4 * (np.arange(w)[None, None, :] / w) + rng.uniform(-8, 8, (3, h, w)) / 255.0).astype(np.float32)
+    return np.concatenate([rgb.reshape(-1), a.reshape(-1)]).astype(np.float32)
+
+
+KINDS = ["noise", "flat", "faint", "grid", "dark", "weights", "wide", "odd", "ramp"]
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("fmt", [ntg.FORMAT_BC1])
+def test_fits_match_oracle(ctx, oracle, kind, fmt):
+    image = {ntg.FORMAT_BC1: oracle.bc1_image}[fmt]
+    for i, (w, h) in enumerate([(4, 4), (8, 4), (12, 4), (28, 4), (36, 4), (61, 35), (128, 96)]):
+        img = contents(kind, w, h, 100 * i + len(kind))
+        for quality, alpha, cw in [(1, 0, (1, 1, 1)), (1, 1, (1, 1, 1)), (2, 1, (0.6, 1.0, 0.4))]:
+            if quality == 2 and w > 61:
+                continue
+            got = ctx.encode(fmt, torch.from_numpy(img).cuda(), w, h, quality=quality, alpha_mode=alpha, cw=cw)
+            ref = image(img, w, h, alpha, quality, cw=cw, threads=8)
+            assert np.array_equal(got.cpu().numpy(), ref), (kind, w, h, quality, alpha)
