@@ -5,12 +5,14 @@
 // fit, output 6 the fit's log-error (used to decide when the pruned search falls back to the full
 // one), output 7 is unused. No counterpart in the reference.
 //
-// Every matrix product is one kernel, k_gemm: D[M x N] = A[M x K] * B[N x K]^T with both operands
-// K-major BF16, staged by the CTA's threads into shared memory in the canonical no-swizzle layout
+// Training runs in two kernels: k_mlp_train takes a tile of 128 rows forward and back through all layers
+// (weights in shared memory, accumulators in TMEM), and k_mlp_grads multiplies what it left in memory into the weight
+// gradients. Inference is k_mlp_infer. The unfused forward pass and ntg_gemm_bf16 use a plain product,
+// k_gemm: D[M x N] = A[M x K] * B[N x K]^T with both operands K-major BF16, staged by the CTA's threads into shared memory in the canonical no-swizzle layout
 // (8-row x 16-byte core matrices), multiplied by tcgen05.mma (kind::f16, M = 128) issued by one
 // thread into a TMEM accumulator, double-buffered with an mbarrier per stage that the MMA's
 // tcgen05.commit arrives on. The epilogue reads the accumulator back with tcgen05.ld (thread t owns
-// row t) and applies bias + GELU, GELU', or split-K atomics. Every wait is bounded (a poll count the
+// row t) and applies bias + GELU. Every wait is bounded (a poll count the
 // host sets per network, ntg_mlp_set_wait_limit): on timeout the kernel records an error, waits (with
 // the default limit) for the tensor-core work it has already issued, frees its TMEM and returns.
 #include <cuda_bf16.h>
@@ -34,23 +36,18 @@ constexpr int IN = 48, HID = 256, OUT = 8, OUTP = 16;  // OUTP: output rows padd
 constexpr int BM = 128, BK = 64;                       // CTA tile rows, K chunk
 constexpr uint32_t LBO = 128, SBO = 1024;              // K-direction and row-group core-matrix strides
 
-enum Epi { EPI_F32 = 0, EPI_GELU = 1, EPI_DGELU = 2, EPI_ATOMIC = 3 };
+enum Epi { EPI_F32 = 0, EPI_GELU = 1 };
 
 struct GemmArgs {
     const __nv_bfloat16 *A;  // [M x K], row stride lda (elements)
     const __nv_bfloat16 *B;  // [N x K], row stride ldb
     int lda, ldb, M, N, K;
-    int k_split;             // K per blockIdx.z (multiple of BK)
     int epi;
     const float *bias;       // [N] or null
     float *C;                // fp32 [M x N] (ldc), or null
     int ldc;
     __nv_bfloat16 *H;        // bf16 [M x N] (ldh), or null
     int ldh;
-    __nv_bfloat16 *HT;       // bf16 [N x M] (ldht), or null
-    int ldht;
-    const float *Z;          // pre-activation [M x N] (ldz) for EPI_DGELU
-    int ldz;
     int *status;             // set to a non-zero code when a wait gives up
     int polls;               // polls of each wait before it gives up
 };
@@ -115,6 +112,26 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// The same without the wait, into raw registers, and the wait that makes them valid (it names them, so that no use moves
+// above it): several loads in flight.
+__device__ __forceinline__ void tmem_ld16_start(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+        "[%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld16_finish(uint32_t (&r)[16], float (&v)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                   "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+
 // GELU in its tanh form (Hendrycks & Gimpel, "Gaussian Error Linear Units", 2016):
 // gelu(z) = z / 2 (1 + tanh(sqrt(2 / pi) (z + 0.044715 z^3))), with the hardware tanh
 // (tanh.approx.f32, about 2^-11 relative error, below the BF16 rounding of the activations), and its
@@ -162,8 +179,7 @@ __global__ void __launch_bounds__(128) k_gemm(GemmArgs g) {
     uint8_t *a_st[2] = {smem, smem + A_BYTES + B_BYTES};
     uint8_t *b_st[2] = {smem + A_BYTES, smem + 2 * A_BYTES + B_BYTES};
     const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-    const int kbeg = blockIdx.z * g.k_split, kend = min(g.K, kbeg + g.k_split);
-    const int chunks = (kend - kbeg + BK - 1) / BK;
+    const int chunks = (g.K + BK - 1) / BK;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (warp == 0) tmem_alloc(&tmem_base, TMEM_COLS);
@@ -186,9 +202,9 @@ __global__ void __launch_bounds__(128) k_gemm(GemmArgs g) {
             ok = __syncthreads_and(mbar_wait(&bars[s], ((c - 2) >> 1) & 1, g.polls)) != 0;
             if (!ok) break;
         }
-        const int k0 = kbeg + c * BK;
-        stage_tile(a_st[s], g.A, g.lda, m0, g.M, BM, k0, kend);
-        stage_tile(b_st[s], g.B, g.ldb, n0, g.N, BN, k0, kend);
+        const int k0 = c * BK;
+        stage_tile(a_st[s], g.A, g.lda, m0, g.M, BM, k0, g.K);
+        stage_tile(b_st[s], g.B, g.ldb, n0, g.N, BN, k0, g.K);
         fence_async_smem();
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -226,24 +242,9 @@ __global__ void __launch_bounds__(128) k_gemm(GemmArgs g) {
                 const int n = n0 + c0 + i;
                 if (n >= g.N) break;
                 float x = v[i];
-                if (g.epi == EPI_ATOMIC) {
-                    atomicAdd(g.C + (size_t)m * g.ldc + n, x);
-                    continue;
-                }
                 if (g.bias) x += g.bias[n];
-                float y = x;
-                if (g.epi == EPI_GELU) {
-                    if (g.C) g.C[(size_t)m * g.ldc + n] = x;
-                    y = gelu(x);
-                } else if (g.epi == EPI_DGELU) {
-                    y = x * gelu_grad(g.Z[(size_t)m * g.ldz + n]);
-                    if (g.C) g.C[(size_t)m * g.ldc + n] = y;
-                } else if (g.C) {
-                    g.C[(size_t)m * g.ldc + n] = x;
-                }
-                const __nv_bfloat16 hb = __float2bfloat16_rn(y);
-                if (g.H) g.H[(size_t)m * g.ldh + n] = hb;
-                if (g.HT) g.HT[(size_t)n * g.ldht + m] = hb;
+                if (g.C) g.C[(size_t)m * g.ldc + n] = x;
+                if (g.H) g.H[(size_t)m * g.ldh + n] = __float2bfloat16_rn(g.epi == EPI_GELU ? gelu(x) : x);
             }
         }
     }
@@ -255,101 +256,35 @@ __global__ void __launch_bounds__(128) k_gemm(GemmArgs g) {
 size_t gemm_smem(int bn) { return 2 * (size_t)(BM * BK * 2 + bn * BK * 2) + 1024; }
 
 template <int BN>
-int launch_gemm_t(const GemmArgs &g, int splits, cudaStream_t s) {
+int launch_gemm_t(const GemmArgs &g, cudaStream_t s) {
     static std::atomic<unsigned long long> configured{0};
     const size_t sm = gemm_smem(BN);
     if (first_use_on_device(configured)) cudaFuncSetAttribute(k_gemm<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    dim3 grid((g.M + BM - 1) / BM, (g.N + BN - 1) / BN, splits);
+    dim3 grid((g.M + BM - 1) / BM, (g.N + BN - 1) / BN);
     k_gemm<BN><<<grid, 128, sm, s>>>(g);
     return launch_status();
 }
 
 // Picks the N tile (16, 48, 64 or 256 columns) for the product's N.
-int launch_gemm(GemmArgs g, int splits, cudaStream_t s) {
+int launch_gemm(const GemmArgs &g, cudaStream_t s) {
     if (g.K % 8 || g.lda % 8 || g.ldb % 8) return NTG_ERROR_INVALID_INPUT;
-    splits = splits < 1 ? 1 : splits;
-    g.k_split = ((g.K + splits - 1) / splits + BK - 1) / BK * BK;
-    splits = (g.K + g.k_split - 1) / g.k_split;
-    if (g.N <= 16) return launch_gemm_t<16>(g, splits, s);
-    if (g.N <= 48) return launch_gemm_t<48>(g, splits, s);
-    if (g.N <= 64) return launch_gemm_t<64>(g, splits, s);
-    return launch_gemm_t<256>(g, splits, s);
+    if (g.N <= 16) return launch_gemm_t<16>(g, s);
+    if (g.N <= 48) return launch_gemm_t<48>(g, s);
+    if (g.N <= 64) return launch_gemm_t<64>(g, s);
+    return launch_gemm_t<256>(g, s);
 }
 
 // ---- elementwise kernels ----
 
-// fp32 [rows x cols] -> bf16 row-major and (optionally) bf16 transposed [cols x rows]
-__global__ void k_to_bf16(const float *__restrict__ x, int rows, int cols, __nv_bfloat16 *__restrict__ y,
-                          __nv_bfloat16 *__restrict__ yt) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)rows * cols;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int r = (int)(i / cols), c = (int)(i % cols);
-        const __nv_bfloat16 b = __float2bfloat16_rn(x[i]);
-        if (y) y[i] = b;
-        if (yt) yt[(size_t)c * rows + r] = b;
-    }
-}
-
-// Loss and output gradient: dY = 2 w (Y - T) / (B * OUT) for the weighted outputs, loss += w (Y - T)^2 / (B * OUT).
-__global__ void k_loss(const float *__restrict__ y, const float *__restrict__ t, int batch, const float *__restrict__ wout,
-                       float *__restrict__ dy, __nv_bfloat16 *__restrict__ dyb, __nv_bfloat16 *__restrict__ dyt,
-                       float *__restrict__ loss) {
-    float acc = 0.0f;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < batch * OUTP; i += gridDim.x * blockDim.x) {
-        const int r = i / OUTP, c = i % OUTP;
-        float g = 0.0f;
-        if (c < OUT) {
-            const float d = y[(size_t)r * OUTP + c] - t[(size_t)r * OUT + c];
-            const float w = wout[c] / (float)(batch * OUT);
-            acc += w * d * d;
-            g = 2.0f * w * d;
-        }
-        dy[i] = g;
-        const __nv_bfloat16 b = __float2bfloat16_rn(g);
-        dyb[i] = b;
-        dyt[(size_t)c * batch + r] = b;
-    }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, acc);
-}
-
-// Column sums of an fp32 [rows x cols] matrix into out[cols] (bias gradients).
-__global__ void k_colsum(const float *__restrict__ x, int rows, int cols, float *__restrict__ out) {
-    const int c = blockIdx.x;
-    float acc = 0.0f;
-    for (int r = threadIdx.x; r < rows; r += blockDim.x) acc += x[(size_t)r * cols + c];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    __shared__ float part[32];
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float s = 0.0f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += part[w];
-        out[c] = s;
-    }
+// fp32 -> bf16
+__global__ void k_to_bf16(const float *__restrict__ x, long long n, __nv_bfloat16 *__restrict__ y) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        y[i] = __float2bfloat16_rn(x[i]);
 }
 
 // Parameter layout (flat fp32): W1 [HID x IN], b1 [HID], W2 [HID x HID], b2 [HID], W3 [OUT x HID], b3 [OUT].
 constexpr size_t OFF_W1 = 0, OFF_B1 = OFF_W1 + (size_t)HID * IN, OFF_W2 = OFF_B1 + HID, OFF_B2 = OFF_W2 + (size_t)HID * HID,
                  OFF_W3 = OFF_B2 + HID, OFF_B3 = OFF_W3 + (size_t)OUT * HID, NPARAM = OFF_B3 + OUT;
-
-// Gathers the gradient pieces into the flat layout (dW3 arrives transposed, [HID x OUTP]).
-__global__ void k_gather_grads(const float *__restrict__ dw1, const float *__restrict__ db1, const float *__restrict__ dw2,
-                               const float *__restrict__ db2, const float *__restrict__ dw3t, const float *__restrict__ db3,
-                               float *__restrict__ g) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (int)NPARAM; i += gridDim.x * blockDim.x) {
-        float v;
-        if (i < (int)OFF_B1) v = dw1[i];
-        else if (i < (int)OFF_W2) v = db1[i - OFF_B1];
-        else if (i < (int)OFF_B2) v = dw2[i - OFF_W2];
-        else if (i < (int)OFF_W3) v = db2[i - OFF_B2];
-        else if (i < (int)OFF_B3) {
-            const int k = i - (int)OFF_W3, o = k / HID, j = k % HID;
-            v = dw3t[(size_t)j * OUTP + o];
-        } else v = db3[i - OFF_B3];
-        g[i] = v;
-    }
-}
 
 __global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
                        int n, float lr, float b1, float b2, float eps, float c1, float c2) {
@@ -404,14 +339,29 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-// Copies a bf16 row-major [rows x K] matrix from global memory into the canonical layout.
+// Copies a bf16 row-major [rows x K] matrix from global memory into the canonical layout; eight consecutive threads
+// write the eight rows of a core matrix (one 128-byte run: no bank conflicts), the next eight its neighbour along K.
 __device__ void load_operand(uint8_t *dst, const __nv_bfloat16 *src, int rows, int K) {
     const int chunks = K / 8;
     for (int p = threadIdx.x; p < rows * chunks; p += blockDim.x) {
-        const int r = p / chunks, kc = p % chunks;
+        const int g = p >> 3, kc = g % chunks, r = (g / chunks) * 8 + (p & 7);
         put8(dst, (uint32_t)chunks * LBO, r, kc, *reinterpret_cast<const uint4 *>(src + (size_t)r * K + kc * 8));
     }
 }
+
+// The same, asynchronously (cp.async, generic proxy): complete after async_wait<later groups> and a barrier.
+__device__ __forceinline__ void load_operand_async(uint8_t *dst, const __nv_bfloat16 *src, int rows, int K) {
+    const int chunks = K / 8;
+    for (int p = threadIdx.x; p < rows * chunks; p += blockDim.x) {
+        const int g = p >> 3, kc = g % chunks, r = (g / chunks) * 8 + (p & 7);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + (r >> 3) * (uint32_t)chunks * LBO + kc * LBO + (r & 7) * 16)),
+                     "l"(src + (size_t)r * K + kc * 8)
+                     : "memory");
+    }
+}
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LATER>
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LATER) : "memory"); }
 
 // Bias + GELU of this thread's quarter (64 columns from c_begin) of its row's accumulator, into its
 // row of the activation operand.
@@ -539,6 +489,369 @@ __global__ void __launch_bounds__(512, 1) k_mlp_infer(const __nv_bfloat16 *__res
     if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
+// ---- training: forward and backward of a 128-row tile in one kernel ----
+// The layers run as in k_mlp_infer, and back: Y -> dY -> dZ2 -> dZ1, with Z2 kept in TMEM (columns [256, 512)) for its
+// GELU', Z1 as FP32 in global memory (the TMEM columns of layer 1 are needed again), and the W2^T operand
+// loaded over W2 once layer 2 is done. What the weight gradients need goes to memory row-major in BF16, once;
+// bias gradients and the loss are summed in FP32 and added up with atomics. Bound by the four epilogues of 128 x 256
+// (tanh, conversions, shared-memory stores) on the batch's tiles, one CTA each, four warps a scheduler: 54 us at
+// batch 8192, and 18 for k_mlp_grads, where forward and backward as nine products, each writing its results element
+// by element and in two layouts, with their column sums and conversions took 840.
+struct TrainArgs {
+    const __nv_bfloat16 *w1, *w2, *w2t, *w3, *w3t;
+    const float *b1, *b2, *b3, *wout, *x, *t;
+    int batch;
+    float *z1;                                 // [batch x HID]
+    __nv_bfloat16 *h1, *h2, *dz1, *dz2, *dyb;  // [batch x HID], dyb [batch x OUTP]
+    float *g, *loss;
+    int *status;
+    int polls;
+    bool aligned;  // x lies on a 16-byte boundary
+};
+constexpr size_t T_DY = F_W1, T_W3T = T_DY + (size_t)BM * OUTP * 2, T_DB = T_W3T + (size_t)HID * OUTP * 2;  // over W1
+static_assert(T_DB + 2 * HID * 4 <= F_W2, "the operands that replace W1 fit its place");
+
+// Sums over the warp's 32 lanes of 16 values each: lane l gets the sum of value (l >> 1).
+__device__ __forceinline__ float warp_sum16(float (&v)[16]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int n = 8; n >= 1; n >>= 1) {  // lanes 2n apart exchange halves of what they still hold
+        const bool up = (lane & (2 * n)) != 0;
+#pragma unroll
+        for (int i = 0; i < n; i++) {
+            const float keep = up ? v[n + i] : v[i], send = up ? v[i] : v[n + i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * n);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// 16 values as BF16: into the activation operand (when act is given) and 32 bytes of a row in global memory.
+__device__ __forceinline__ void put_bf16(const float (&v)[16], uint8_t *act, int row, int c0, __nv_bfloat16 *dst, bool live) {
+    uint32_t p[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) p[i] = pack_bf16(v[2 * i], v[2 * i + 1]);
+    const uint4 lo = make_uint4(p[0], p[1], p[2], p[3]), hi = make_uint4(p[4], p[5], p[6], p[7]);
+    if (act) {
+        put8(act, SBO_HID, row, c0 / 8, lo);
+        put8(act, SBO_HID, row, c0 / 8 + 1, hi);
+    }
+    if (live) {
+        reinterpret_cast<uint4 *>(dst)[0] = lo;
+        reinterpret_cast<uint4 *>(dst)[1] = hi;
+    }
+}
+
+__global__ void __launch_bounds__(512, 1) k_mlp_train(TrainArgs g) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    uint8_t *const act = smem + F_ACT, *const dyop = smem + T_DY;
+    float *const sb = reinterpret_cast<float *>(smem + F_BIAS), *const db = reinterpret_cast<float *>(smem + T_DB);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = threadIdx.x & 127, quarter = threadIdx.x >> 7;
+    if (warp == 0) tmem_alloc(&tmem_base, 512);
+    if (threadIdx.x == 0) {
+        mbar_init(&bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int i = threadIdx.x; i < HID; i += blockDim.x) { sb[i] = g.b1[i]; sb[HID + i] = g.b2[i]; }
+    if (threadIdx.x < OUTP) sb[2 * HID + threadIdx.x] = g.b3[threadIdx.x];
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base, lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t a_act = smem_u32(act), a_w1 = smem_u32(smem + F_W1), a_w2 = smem_u32(smem + F_W2), a_w3 = smem_u32(smem + F_W3);
+    const uint32_t a_dy = smem_u32(dyop), a_w3t = smem_u32(smem + T_W3T);
+    constexpr uint32_t SBO_OUT = OUTP / 8 * 128;
+    uint32_t phase = 0;
+    bool ok = true;
+    // acc[128 x N] = A * B^T over `steps` 16-element steps of K; every thread returns once it is in TMEM
+    auto product = [&](uint32_t acc, uint32_t a, uint32_t a_sbo, uint32_t b, uint32_t b_sbo, int steps, uint32_t idesc) {
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");  // the epilogue's last load ahead
+        fence_async_smem();
+        tc_fence_before();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            tc_fence_after();
+            for (int j = 0; j < steps; j++) mma_bf16(acc, smem_desc(a + j * 2 * LBO, a_sbo), smem_desc(b + j * 2 * LBO, b_sbo), idesc, j > 0);
+            mma_commit(&bar);
+        }
+        ok = __syncthreads_and(mbar_wait(&bar, phase & 1, g.polls)) != 0;
+        // gave up: drain the MMAs (they write the accumulator) before TMEM is freed
+        if (!ok) __syncthreads_and(mbar_wait(&bar, phase & 1, kWaitPolls));
+        phase++;
+        tc_fence_after();
+        return ok;
+    };
+    const int tiles = (g.batch + BM - 1) / BM, c_begin = quarter * (HID / 4);
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int r = tile * BM + row;
+        const bool live = r < g.batch;
+        const size_t rh = (size_t)r * HID;
+        load_operand_async(smem + F_W1, g.w1, HID, IN);
+        async_commit();
+        load_operand_async(smem + F_W2, g.w2, HID, HID);
+        load_operand_async(smem + F_W3, g.w3, OUTP, HID);
+        async_commit();
+        if (quarter < 2) {
+#pragma unroll
+            for (int k = 0; k < IN / 16; k++) {
+                const int kc = quarter * (IN / 16) + k;
+                float4 a = make_float4(0, 0, 0, 0), b = a;
+                const float *const p = g.x + (size_t)r * IN + kc * 8;
+                if (live && g.aligned) {
+                    a = *reinterpret_cast<const float4 *>(p);
+                    b = *reinterpret_cast<const float4 *>(p + 4);
+                } else if (live) {
+                    a = make_float4(p[0], p[1], p[2], p[3]);
+                    b = make_float4(p[4], p[5], p[6], p[7]);
+                }
+                put8(act, SBO_IN, row, kc, make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w)));
+            }
+        }
+        async_wait<1>();
+        if (!product(tmem, a_act, SBO_IN, a_w1, SBO_IN, IN / 16, idesc_bf16(BM, HID))) break;
+        // Z1 -> H1; in each epilogue the next 16 columns are on their way while these are worked on
+        uint32_t raw[16];
+        tmem_ld16_start(lane_addr + c_begin, raw);
+#pragma unroll 1
+        for (int c0 = c_begin; c0 < c_begin + HID / 4; c0 += 16) {
+            float v[16];
+            tmem_ld16_finish(raw, v);
+            tmem_ld16_start(lane_addr + (c0 + 16 < c_begin + HID / 4 ? c0 + 16 : c0), raw);
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] += sb[c0 + i];
+            if (live)
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    reinterpret_cast<float4 *>(g.z1 + rh + c0)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] = gelu(v[i]);
+            put_bf16(v, act, row, c0, g.h1 + rh + c0, live);
+        }
+        // W1 is done with: its place takes W3^T and the bias sums (dY follows)
+        async_wait<0>();
+        load_operand_async(smem + T_W3T, g.w3t, HID, OUTP);
+        for (int i = threadIdx.x; i < 2 * HID; i += blockDim.x) db[i] = 0.0f;
+        if (!product(tmem + HID, a_act, SBO_HID, a_w2, SBO_HID, HID / 16, idesc_bf16(BM, HID))) break;
+        load_operand_async(smem + F_W2, g.w2t, HID, HID);  // beside the epilogue
+        async_commit();
+        // Z2 -> H2
+        tmem_ld16_start(lane_addr + HID + c_begin, raw);
+#pragma unroll 1
+        for (int c0 = c_begin; c0 < c_begin + HID / 4; c0 += 16) {
+            float v[16];
+            tmem_ld16_finish(raw, v);
+            tmem_ld16_start(lane_addr + HID + (c0 + 16 < c_begin + HID / 4 ? c0 + 16 : c0), raw);
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] = gelu(v[i] + sb[HID + c0 + i]);
+            put_bf16(v, act, row, c0, g.h2 + rh + c0, live);
+        }
+        if (!product(tmem, a_act, SBO_HID, a_w3, SBO_HID, HID / 16, idesc_bf16(BM, OUTP))) break;
+        // Y -> loss, dY = 2 w (Y - T) / (batch OUT)
+        if (quarter == 0) {
+            float v[16], part = 0.0f;
+            tmem_ld16(lane_addr, v);
+#pragma unroll
+            for (int c = 0; c < 16; c++) {
+                float d = 0.0f;
+                if (c < OUT && live) {
+                    const float e = v[c] + sb[2 * HID + c] - g.t[(size_t)r * OUT + c];
+                    const float w = g.wout[c] / (float)(g.batch * OUT);
+                    part += w * e * e;
+                    d = 2.0f * w * e;
+                }
+                v[c] = d;
+            }
+            const uint4 lo = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+            const uint4 zero = make_uint4(0, 0, 0, 0);
+            put8(dyop, SBO_OUT, row, 0, lo);
+            put8(dyop, SBO_OUT, row, 1, zero);
+            if (live) {
+                reinterpret_cast<uint4 *>(g.dyb + (size_t)r * OUTP)[0] = lo;
+                reinterpret_cast<uint4 *>(g.dyb + (size_t)r * OUTP)[1] = zero;
+            }
+            for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+            if (lane == 0) atomicAdd(g.loss, part);
+            const float s = warp_sum16(v);
+            if ((lane & 1) == 0 && (lane >> 1) < OUT) atomicAdd(g.g + OFF_B3 + (lane >> 1), s);
+        }
+        async_wait<0>();
+        if (!product(tmem, a_dy, SBO_OUT, a_w3t, SBO_OUT, 1, idesc_bf16(BM, HID))) break;
+        // dZ2 = (dY W3) gelu'(Z2)
+        uint32_t raw2[16];
+        tmem_ld16_start(lane_addr + c_begin, raw);
+        tmem_ld16_start(lane_addr + HID + c_begin, raw2);
+#pragma unroll 1
+        for (int c0 = c_begin; c0 < c_begin + HID / 4; c0 += 16) {
+            float v[16], z[16];
+            tmem_ld16_finish(raw, v);
+            tmem_ld16_finish(raw2, z);
+            const int next = c0 + 16 < c_begin + HID / 4 ? c0 + 16 : c0;
+            tmem_ld16_start(lane_addr + next, raw);
+            tmem_ld16_start(lane_addr + HID + next, raw2);
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] = live ? v[i] * gelu_grad(z[i] + sb[HID + c0 + i]) : 0.0f;
+            put_bf16(v, act, row, c0, g.dz2 + rh + c0, live);
+            const float s = warp_sum16(v);
+            if ((lane & 1) == 0) atomicAdd(&db[HID + c0 + (lane >> 1)], s);
+        }
+        if (!product(tmem, a_act, SBO_HID, a_w2, SBO_HID, HID / 16, idesc_bf16(BM, HID))) break;
+        // dZ1 = (dZ2 W2) gelu'(Z1)
+        float4 ahead[4];
+        auto fetch_z1 = [&](int c) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) ahead[i] = live ? reinterpret_cast<const float4 *>(g.z1 + rh + c)[i] : make_float4(0, 0, 0, 0);
+        };
+        fetch_z1(c_begin);
+        tmem_ld16_start(lane_addr + c_begin, raw);
+#pragma unroll 1
+        for (int c0 = c_begin; c0 < c_begin + HID / 4; c0 += 16) {
+            float v[16], z[16];
+            tmem_ld16_finish(raw, v);
+#pragma unroll
+            for (int i = 0; i < 4; i++) { z[4 * i] = ahead[i].x; z[4 * i + 1] = ahead[i].y; z[4 * i + 2] = ahead[i].z; z[4 * i + 3] = ahead[i].w; }
+            const int next = c0 + 16 < c_begin + HID / 4 ? c0 + 16 : c0;
+            tmem_ld16_start(lane_addr + next, raw);
+            fetch_z1(next);
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] = live ? v[i] * gelu_grad(z[i]) : 0.0f;
+            put_bf16(v, nullptr, row, c0, g.dz1 + rh + c0, live);
+            const float s = warp_sum16(v);
+            if ((lane & 1) == 0) atomicAdd(&db[c0 + (lane >> 1)], s);
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        __syncthreads();
+        if (threadIdx.x < HID) {
+            atomicAdd(g.g + OFF_B1 + threadIdx.x, db[threadIdx.x]);
+            atomicAdd(g.g + OFF_B2 + threadIdx.x, db[HID + threadIdx.x]);
+        }
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+    }
+    async_wait<0>();
+    if (!ok && threadIdx.x == 0) atomicExch(g.status, 1);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem, 512);
+}
+
+// ---- training: the weight gradients ----
+// dW2 = dZ2^T H1, dW1 = dZ1^T X, dW3 = dY^T H2: products over the batch, split into runs of GRAD_K rows (blockIdx.x);
+// blockIdx.y: dW2, dW1 and dW3^T, the upper and the lower 128 of their 256 rows. The operands lie row-major with the batch
+// outermost, so staging turns them: a thread reads two columns of eight batch rows and writes them as two 16-byte
+// runs along K. The sums go to the flat gradient with four-wide atomics.
+// Bound by the latency of the staging loads: 18 us at batch 8192 with 512 threads a CTA, 25 with 256.
+constexpr int GRAD_K = 256, GRAD_N = 256, GRAD_THREADS = 512;
+constexpr size_t GRAD_STAGE = (size_t)(BM + GRAD_N) * BK * 2;
+
+// Columns [c0, c0 + cols) of rows [k0, k0 + BK) (below `rows`) of a row-major matrix, as the K-major operand of `cols` rows.
+template <int cols, typename T>
+__device__ __forceinline__ void stage_turned(uint8_t *dst, const T *src, int ld, int c0, int k0, int rows) {
+#pragma unroll 4
+    for (int p = threadIdx.x; p < cols / 2 * (BK / 8); p += GRAD_THREADS) {
+        const int c = 2 * (p % (cols / 2)), kc = p / (cols / 2);
+        uint32_t v[8];  // columns c and c + 1 of eight rows
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int k = k0 + kc * 8 + i;
+            v[i] = 0;
+            if (k < rows) {
+                if constexpr (sizeof(T) == 2) {
+                    v[i] = *reinterpret_cast<const uint32_t *>(src + (size_t)k * ld + c0 + c);
+                } else {
+                    const float *const p = src + (size_t)k * ld + c0 + c;
+                    v[i] = pack_bf16(p[0], p[1]);
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int m = c + h;
+            const unsigned sel = h ? 0x7632u : 0x5410u;
+            *reinterpret_cast<uint4 *>(dst + (m >> 3) * SBO + kc * LBO + (m & 7) * 16) =
+                make_uint4(__byte_perm(v[0], v[1], sel), __byte_perm(v[2], v[3], sel), __byte_perm(v[4], v[5], sel), __byte_perm(v[6], v[7], sel));
+        }
+    }
+}
+
+__global__ void __launch_bounds__(GRAD_THREADS, 2) k_mlp_grads(TrainArgs g) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ uint64_t bars[2];
+    __shared__ uint32_t tmem_base;
+    const int job = blockIdx.y >> 1, m0 = (blockIdx.y & 1) * BM;
+    const int kbeg = blockIdx.x * GRAD_K, kend = min(g.batch, kbeg + GRAD_K), chunks = (kend - kbeg + BK - 1) / BK;
+    const int n = job == 0 ? HID : (job == 1 ? IN : OUTP);
+    const uint32_t idesc = job == 0 ? idesc_bf16(BM, HID) : (job == 1 ? idesc_bf16(BM, IN) : idesc_bf16(BM, OUTP));
+    const __nv_bfloat16 *const a = job == 0 ? g.dz2 : (job == 1 ? g.dz1 : g.h2);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 0) tmem_alloc(&tmem_base, GRAD_N);
+    if (threadIdx.x == 0) {
+        mbar_init(&bars[0], 1);
+        mbar_init(&bars[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base;
+    bool ok = true;
+    int committed = -1;
+    for (int c = 0; c < chunks; c++) {
+        const int s = c & 1;
+        if (c >= 2) {  // the MMAs of chunk c - 2 read this stage
+            ok = __syncthreads_and(mbar_wait(&bars[s], ((c - 2) >> 1) & 1, g.polls)) != 0;
+            if (!ok) break;
+        }
+        uint8_t *const as = smem + s * GRAD_STAGE, *const bs = as + (size_t)BM * BK * 2;
+        const int k0 = kbeg + c * BK;
+        stage_turned<BM>(as, a, HID, m0, k0, kend);
+        if (job == 0) stage_turned<HID>(bs, g.h1, HID, 0, k0, kend);
+        else if (job == 1) stage_turned<IN>(bs, g.x, IN, 0, k0, kend);
+        else stage_turned<OUTP>(bs, g.dyb, OUTP, 0, k0, kend);
+        fence_async_smem();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            tc_fence_after();
+            const uint32_t a0 = smem_u32(as), b0 = smem_u32(bs);
+#pragma unroll
+            for (int j = 0; j < BK / 16; j++)
+                mma_bf16(tmem, smem_desc(a0 + j * 2 * LBO), smem_desc(b0 + j * 2 * LBO), idesc, (c > 0 || j > 0) ? 1u : 0u);
+            mma_commit(&bars[s]);
+        }
+        committed = c;
+    }
+    if (ok) ok = __syncthreads_and(mbar_wait(&bars[committed & 1], (committed >> 1) & 1, g.polls)) != 0;
+    if (!ok) {
+        if (threadIdx.x == 0) atomicExch(g.status, 1);
+        // drain: the last commit's barrier completes once every MMA issued so far has finished
+        __syncthreads_and(mbar_wait(&bars[committed & 1], (committed >> 1) & 1, kWaitPolls));
+    }
+    tc_fence_after();
+    if (ok) {
+        const int m = m0 + (warp & 3) * 32 + lane;
+        const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        // the warps of each quarter of the CTA take every fourth run of 16 columns
+#pragma unroll 1
+        for (int c0 = 16 * (warp >> 2); c0 < n; c0 += 4 * GRAD_THREADS / 32) {
+            float v[16];
+            tmem_ld16(lane_addr + c0, v);
+            if (job == 2) {  // dW3^T: rows are W3's columns
+#pragma unroll
+                for (int i = 0; i < OUT; i++) atomicAdd(g.g + OFF_W3 + (size_t)i * HID + m, v[i]);
+            } else {
+                float4 *const o = reinterpret_cast<float4 *>(g.g + (job == 0 ? OFF_W2 + (size_t)m * HID : OFF_W1 + (size_t)m * IN) + c0);
+#pragma unroll
+                for (int i = 0; i < 4; i++) atomicAdd(o + i, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem, GRAD_N);
+}
+
 int grid_of(long long n) { return (int)std::min<long long>(152LL * 8, std::max<long long>(1, (n + 255) / 256)); }
 
 }  // namespace mlp
@@ -557,10 +870,8 @@ struct ntg_mlp {
     int *status = nullptr;
     int polls = kWaitPolls;  // polls of each tensor-core wait before it gives up
     // activations and gradients, batch `cap`
-    __nv_bfloat16 *xb = nullptr, *xt = nullptr, *h1 = nullptr, *h1t = nullptr, *h2 = nullptr, *h2t = nullptr;
-    __nv_bfloat16 *dyb = nullptr, *dyt = nullptr, *dz2b = nullptr, *dz2t = nullptr, *dz1b = nullptr, *dz1t = nullptr;
-    float *z1 = nullptr, *z2 = nullptr, *y = nullptr, *dy = nullptr, *dz2 = nullptr, *dz1 = nullptr;
-    float *dw1 = nullptr, *db1 = nullptr, *dw2 = nullptr, *db2 = nullptr, *dw3t = nullptr, *db3 = nullptr;
+    __nv_bfloat16 *xb = nullptr, *h1 = nullptr, *h2 = nullptr, *dyb = nullptr, *dz2 = nullptr, *dz1 = nullptr;
+    float *z1 = nullptr, *y = nullptr;
     std::vector<void *> owned, act;
 
     ~ntg_mlp() {
@@ -604,12 +915,9 @@ int ensure_batch(ntg_mlp *m, int batch) {
     m->act.clear();
     const size_t B = (size_t)batch;
     auto &L = m->act;
-    if (dalloc(L, &m->xb, B * IN) || dalloc(L, &m->xt, B * IN) || dalloc(L, &m->h1, B * HID) || dalloc(L, &m->h1t, B * HID) ||
-        dalloc(L, &m->h2, B * HID) || dalloc(L, &m->h2t, B * HID) || dalloc(L, &m->dyb, B * OUTP) ||
-        dalloc(L, &m->dyt, B * OUTP) || dalloc(L, &m->dz2b, B * HID) || dalloc(L, &m->dz2t, B * HID) ||
-        dalloc(L, &m->dz1b, B * HID) || dalloc(L, &m->dz1t, B * HID) || dalloc(L, &m->z1, B * HID) ||
-        dalloc(L, &m->z2, B * HID) || dalloc(L, &m->y, B * OUTP) || dalloc(L, &m->dy, B * OUTP) ||
-        dalloc(L, &m->dz2, B * HID) || dalloc(L, &m->dz1, B * HID))
+    m->cap = 0;
+    if (dalloc(L, &m->xb, B * IN) || dalloc(L, &m->h1, B * HID) || dalloc(L, &m->h2, B * HID) || dalloc(L, &m->dyb, B * OUTP) ||
+        dalloc(L, &m->dz2, B * HID) || dalloc(L, &m->dz1, B * HID) || dalloc(L, &m->z1, B * HID) || dalloc(L, &m->y, B * OUTP))
         return NTG_ERROR_CUDA;
     m->cap = batch;
     return NTG_OK;
@@ -624,62 +932,42 @@ GemmArgs gemm(const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *B, int ldb, 
     return g;
 }
 
-// Forward pass: X (bf16) -> Z1, H1, Z2, H2 -> Y [batch x OUTP]. `train` also writes the
-// transposed activations the weight gradients need.
-int forward(ntg_mlp *m, int batch, bool train, cudaStream_t s) {
+// The unfused forward pass: X -> H1 -> H2 -> Y [batch x OUTP], one product each.
+int forward(ntg_mlp *m, const float *d_x, int batch, cudaStream_t s) {
+    k_to_bf16<<<grid_of((long long)batch * IN), 256, 0, s>>>(d_x, (long long)batch * IN, m->xb);
+    MLP_LAUNCH(launch_status());
     GemmArgs g = gemm(m->xb, IN, m->w1, IN, batch, HID, IN, EPI_GELU, m->status, m->polls);
-    g.bias = m->p + OFF_B1; g.C = train ? m->z1 : nullptr; g.ldc = HID; g.H = m->h1; g.ldh = HID;
-    g.HT = train ? m->h1t : nullptr; g.ldht = batch;
-    MLP_LAUNCH(launch_gemm(g, 1, s));
+    g.bias = m->p + OFF_B1; g.H = m->h1; g.ldh = HID;
+    MLP_LAUNCH(launch_gemm(g, s));
     g = gemm(m->h1, HID, m->w2, HID, batch, HID, HID, EPI_GELU, m->status, m->polls);
-    g.bias = m->p + OFF_B2; g.C = train ? m->z2 : nullptr; g.ldc = HID; g.H = m->h2; g.ldh = HID;
-    g.HT = train ? m->h2t : nullptr; g.ldht = batch;
-    MLP_LAUNCH(launch_gemm(g, 1, s));
+    g.bias = m->p + OFF_B2; g.H = m->h2; g.ldh = HID;
+    MLP_LAUNCH(launch_gemm(g, s));
     g = gemm(m->h2, HID, m->w3, HID, batch, OUTP, HID, EPI_F32, m->status, m->polls);
     g.bias = m->b3p; g.C = m->y; g.ldc = OUTP;
-    MLP_LAUNCH(launch_gemm(g, 1, s));
+    MLP_LAUNCH(launch_gemm(g, s));
     return NTG_OK;
 }
 
-// Backward pass into the flat gradient vector m->g (needs forward(train = true) first).
-int backward(ntg_mlp *m, const float *d_t, int batch, cudaStream_t s) {
-    const int splits = std::max(1, batch / 256);
-    MLP_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(float), s));
-    k_loss<<<grid_of((long long)batch * OUTP), 256, 0, s>>>(m->y, d_t, batch, m->wout, m->dy, m->dyb, m->dyt, m->loss);
+// Forward and backward: the batch's loss into m->loss, its gradient into the flat vector m->g.
+int backprop(ntg_mlp *m, const float *d_x, const float *d_t, int batch, cudaStream_t s) {
+    static std::atomic<unsigned long long> configured{0};
+    if (first_use_on_device(configured)) {
+        cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F_BYTES);
+        cudaFuncSetAttribute(k_mlp_grads, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * GRAD_STAGE));
+    }
+    TrainArgs g;
+    g.w1 = m->w1; g.w2 = m->w2; g.w2t = m->w2t; g.w3 = m->w3; g.w3t = m->w3t;
+    g.b1 = m->p + OFF_B1; g.b2 = m->p + OFF_B2; g.b3 = m->b3p; g.wout = m->wout; g.x = d_x; g.t = d_t;
+    g.batch = batch;
+    g.aligned = reinterpret_cast<uintptr_t>(d_x) % 16 == 0;
+    g.z1 = m->z1; g.h1 = m->h1; g.h2 = m->h2; g.dz1 = m->dz1; g.dz2 = m->dz2; g.dyb = m->dyb;
+    g.g = m->g; g.loss = m->loss; g.status = m->status; g.polls = m->polls;
+    MLP_CUDA(cudaMemsetAsync(m->g, 0, (NPARAM + 1) * sizeof(float), s));
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
+    k_mlp_train<<<std::min((batch + BM - 1) / BM, std::max(1, sms)), 512, F_BYTES, s>>>(g);
     MLP_LAUNCH(launch_status());
-    MLP_CUDA(cudaMemsetAsync(m->dw3t, 0, sizeof(float) * HID * OUTP, s));
-    MLP_CUDA(cudaMemsetAsync(m->dw2, 0, sizeof(float) * HID * HID, s));
-    MLP_CUDA(cudaMemsetAsync(m->dw1, 0, sizeof(float) * HID * IN, s));
-    // dW3^T = H2^T dY
-    GemmArgs g = gemm(m->h2t, batch, m->dyt, batch, HID, OUTP, batch, EPI_ATOMIC, m->status, m->polls);
-    g.C = m->dw3t; g.ldc = OUTP;
-    MLP_LAUNCH(launch_gemm(g, splits, s));
-    k_colsum<<<OUTP, 256, 0, s>>>(m->dy, batch, OUTP, m->db3);
-    // dZ2 = (dY W3) * gelu'(Z2)
-    g = gemm(m->dyb, OUTP, m->w3t, OUTP, batch, HID, OUTP, EPI_DGELU, m->status, m->polls);
-    g.Z = m->z2; g.ldz = HID; g.C = m->dz2; g.ldc = HID; g.H = m->dz2b; g.ldh = HID; g.HT = m->dz2t; g.ldht = batch;
-    MLP_LAUNCH(launch_gemm(g, 1, s));
-    k_colsum<<<HID, 256, 0, s>>>(m->dz2, batch, HID, m->db2);
-    // dW2 = dZ2^T H1
-    g = gemm(m->dz2t, batch, m->h1t, batch, HID, HID, batch, EPI_ATOMIC, m->status, m->polls);
-    g.C = m->dw2; g.ldc = HID;
-    MLP_LAUNCH(launch_gemm(g, splits, s));
-    // dZ1 = (dZ2 W2) * gelu'(Z1)
-    g = gemm(m->dz2b, HID, m->w2t, HID, batch, HID, HID, EPI_DGELU, m->status, m->polls);
-    g.Z = m->z1; g.ldz = HID; g.C = m->dz1; g.ldc = HID; g.H = m->dz1b; g.ldh = HID; g.HT = m->dz1t; g.ldht = batch;
-    MLP_LAUNCH(launch_gemm(g, 1, s));
-    k_colsum<<<HID, 256, 0, s>>>(m->dz1, batch, HID, m->db1);
-    // dW1 = dZ1^T X
-    g = gemm(m->dz1t, batch, m->xt, batch, HID, IN, batch, EPI_ATOMIC, m->status, m->polls);
-    g.C = m->dw1; g.ldc = IN;
-    MLP_LAUNCH(launch_gemm(g, splits, s));
-    k_gather_grads<<<grid_of(NPARAM), 256, 0, s>>>(m->dw1, m->db1, m->dw2, m->db2, m->dw3t, m->db3, m->g);
-    MLP_LAUNCH(launch_status());
-    return NTG_OK;
-}
-
-int load_inputs(ntg_mlp *m, const float *d_x, int batch, cudaStream_t s) {
-    k_to_bf16<<<grid_of((long long)batch * IN), 256, 0, s>>>(d_x, batch, IN, m->xb, m->xt);
+    k_mlp_grads<<<dim3((batch + GRAD_K - 1) / GRAD_K, 6), GRAD_THREADS, 2 * GRAD_STAGE, s>>>(g);
     MLP_LAUNCH(launch_status());
     return NTG_OK;
 }
@@ -727,13 +1015,13 @@ int ntg_mlp_create(int device, unsigned long long seed, ntg_mlp **out) {
     std::unique_ptr<ntg_mlp> m(new ntg_mlp);
     m->device = device;
     auto &L = m->owned;
-    if (dalloc(L, &m->p, NPARAM) || dalloc(L, &m->g, NPARAM) || dalloc(L, &m->m, NPARAM) || dalloc(L, &m->v, NPARAM) ||
+    if (dalloc(L, &m->p, NPARAM) || dalloc(L, &m->g, NPARAM + 2) || dalloc(L, &m->m, NPARAM) || dalloc(L, &m->v, NPARAM) ||
         dalloc(L, &m->w1, (size_t)HID * IN) || dalloc(L, &m->w2, (size_t)HID * HID) || dalloc(L, &m->w2t, (size_t)HID * HID) ||
         dalloc(L, &m->w3, (size_t)OUTP * HID) || dalloc(L, &m->w3t, (size_t)HID * OUTP) || dalloc(L, &m->b3p, OUTP) ||
-        dalloc(L, &m->wout, OUT) || dalloc(L, &m->loss, 1) || dalloc(L, &m->status, 1) || dalloc(L, &m->dw1, (size_t)HID * IN) ||
-        dalloc(L, &m->db1, HID) || dalloc(L, &m->dw2, (size_t)HID * HID) || dalloc(L, &m->db2, HID) ||
-        dalloc(L, &m->dw3t, (size_t)HID * OUTP) || dalloc(L, &m->db3, OUTP))
+        dalloc(L, &m->wout, OUT))
         return NTG_ERROR_CUDA;
+    m->loss = m->g + NPARAM;  // zeroed with the gradient, read together with the status
+    m->status = reinterpret_cast<int *>(m->g + NPARAM + 1);
     // uniform(-1/sqrt(fan_in), 1/sqrt(fan_in)) weights and biases, seeded
     std::vector<float> p(NPARAM);
     std::mt19937_64 rng(seed);
@@ -792,8 +1080,7 @@ int ntg_mlp_infer_unfused(ntg_mlp *m, const float *d_x, int batch, float *d_y, v
     if (!m || !d_x || !d_y || batch <= 0) return mlp_fail(NTG_ERROR_INVALID_INPUT, "bad arguments");
     cudaStream_t s = (cudaStream_t)stream;
     int r = ensure_batch(m, batch);
-    if (!r) r = load_inputs(m, d_x, batch, s);
-    if (!r) r = forward(m, batch, false, s);
+    if (!r) r = forward(m, d_x, batch, s);
     if (r) return r;
     MLP_CUDA(cudaMemcpyAsync(d_y, m->y, sizeof(float) * batch * OUTP, cudaMemcpyDeviceToDevice, s));
     return NTG_OK;
@@ -804,24 +1091,21 @@ int ntg_mlp_gradients(ntg_mlp *m, const float *d_x, const float *d_t, int batch,
     if (!m || !d_x || !d_t || batch <= 0) return mlp_fail(NTG_ERROR_INVALID_INPUT, "bad arguments");
     cudaStream_t s = (cudaStream_t)stream;
     int r = ensure_batch(m, batch);
-    if (!r) r = load_inputs(m, d_x, batch, s);
-    if (!r) r = forward(m, batch, true, s);
-    if (!r) r = backward(m, d_t, batch, s);
+    if (!r) r = backprop(m, d_x, d_t, batch, s);
     if (r) return r;
     if (d_grads) MLP_CUDA(cudaMemcpyAsync(d_grads, m->g, NPARAM * sizeof(float), cudaMemcpyDeviceToDevice, s));
-    if (h_loss) {
-        MLP_CUDA(cudaMemcpyAsync(h_loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, s));
-    }
-    return check_status(m, s);
+    struct { float loss; int status; } h;
+    MLP_CUDA(cudaMemcpyAsync(&h, m->loss, sizeof h, cudaMemcpyDeviceToHost, s));
+    MLP_CUDA(cudaStreamSynchronize(s));
+    if (h_loss) *h_loss = h.loss;
+    return h.status ? mlp_fail(NTG_ERROR_CUDA, "tensor-core wait timed out") : NTG_OK;
 }
 
 int ntg_mlp_train_step(ntg_mlp *m, const float *d_x, const float *d_t, int batch, float lr, float *d_loss, void *stream) {
     if (!m || !d_x || !d_t || batch <= 0) return mlp_fail(NTG_ERROR_INVALID_INPUT, "bad arguments");
     cudaStream_t s = (cudaStream_t)stream;
     int r = ensure_batch(m, batch);
-    if (!r) r = load_inputs(m, d_x, batch, s);
-    if (!r) r = forward(m, batch, true, s);
-    if (!r) r = backward(m, d_t, batch, s);
+    if (!r) r = backprop(m, d_x, d_t, batch, s);
     if (r) return r;
     m->step++;
     const float b1 = 0.9f, b2 = 0.999f;
@@ -854,7 +1138,7 @@ int ntg_gemm_bf16(const void *d_a, const void *d_b, int M, int N, int K, float *
     if (!d_a || !d_b || !d_c || M <= 0 || N <= 0 || K <= 0) return mlp_fail(NTG_ERROR_INVALID_INPUT, "bad arguments");
     GemmArgs g = gemm((const __nv_bfloat16 *)d_a, K, (const __nv_bfloat16 *)d_b, K, M, N, K, EPI_F32, nullptr);
     g.C = d_c; g.ldc = N;
-    MLP_LAUNCH(launch_gemm(g, 1, (cudaStream_t)stream));
+    MLP_LAUNCH(launch_gemm(g, (cudaStream_t)stream));
     return NTG_OK;
 }
 
