@@ -321,16 +321,18 @@ const size_t NONE = (size_t)-1;
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
-ChainPlan plan_chain(int w, int h, const ntg_chain_options &o, bool keep_level0_float) {
+// `levels_only`: the levels of a call that returns them, every FP32 level back to back (level 0 included) and
+// nothing else; otherwise the workspace of a chain that is encoded, whose level 0 stays in its input bytes.
+ChainPlan plan_chain(int w, int h, const ntg_chain_options &o, bool levels_only) {
     ChainPlan P;
     P.lv = chain_levels(w, h, o.max_levels);
     filter_defaults(o, P.width, P.p);
     P.fast_box = uses_fast_box(o, P.width);
-    const bool need_q = o.format != NTG_FORMAT_BC1;
+    const bool need_q = o.format != NTG_FORMAT_BC1 && !levels_only;
     size_t off = 0;
     for (size_t l = 0; l < P.lv.size(); l++) {
         const size_t n = (size_t)P.lv[l].w * P.lv[l].h;
-        if (l > 0 || P.fast_box || keep_level0_float) { P.f_off.push_back(off); off = align256(off + 16 * n); }
+        if (l > 0 || levels_only) { P.f_off.push_back(off); off = levels_only ? off + 16 * n : align256(off + 16 * n); }
         else P.f_off.push_back(NONE);
         if (l > 0 && need_q) { P.q_off.push_back(off); off = align256(off + 4 * n); }
         else P.q_off.push_back(NONE);
@@ -341,7 +343,7 @@ ChainPlan plan_chain(int w, int h, const ntg_chain_options &o, bool keep_level0_
 
 struct MipKey {
     int kernel, ws, weighted, u8;
-    // the BGRA8 tile kernel loads these once per launch: its jobs must share them
+    // the BGRA8 tile and box kernels load these once per launch: their jobs must share them
     const float *lut = nullptr, *steps = nullptr;
     std::vector<float> taps;
     bool operator<(const MipKey &o) const {
@@ -361,8 +363,7 @@ int plan_step(ntg_context *ctx, const ntg_chain_options &o, float width, const f
     J.W = S.w; J.H = S.h; J.w = D.w; J.h = D.h;
     J.wrap = o.wrap; J.dst = dst; J.q_out = q; J.xform = o.out_xform; J.steps = steps;
     if (fast_box) {
-        if (!src) return fail(NTG_ERROR_INVALID_INPUT, "box downsample needs an FP32 source level");
-        key = {MIP_FAST_BOX, 0, 0, 0};
+        key = {MIP_FAST_BOX, 0, 0, src == nullptr, src ? nullptr : lut};
         return NTG_OK;
     }
     const AxisTable *ax = ctx->axis(o.filter, width, p[0], p[1], S.w, D.w);
@@ -525,8 +526,12 @@ void group_launches(const std::vector<std::pair<MipKey, MipJob>> &items, const M
 }
 
 // First destination level of a chain that its tail launch computes (lv.size() = no tail).
+// A narrow filter's tail begins at sources four times larger (64x64 instead of 32x32): a tail level's time grows with its
+// taps, a launch's does not. Measured for chains from 64 to 512 texels wide: box and triangle 2 to 4 us faster from 64x64,
+// Kaiser (13 taps) 2 us slower.
 size_t tail_start(const ChainPlan &P, const MipTuning &tune) {
-    const long long limit = std::min<long long>(tune.tail_texels, tail_max_texels());
+    const bool narrow = P.fast_box || P.width <= 1.0f;
+    const long long limit = std::min<long long>(tune.tail_texels * (narrow ? 4 : 1), tail_max_texels());
     for (size_t l = 1; l < P.lv.size(); l++) {
         const Level &S = P.lv[l - 1];
         // the X pass plane (H x max(1, W/2)) must fit the tail's half-size buffer as well: a 1-wide
@@ -540,7 +545,7 @@ size_t tail_start(const ChainPlan &P, const MipTuning &tune) {
 // Mip job of destination level l of a chain.
 int chain_step(ntg_context *ctx, const ChainPlan &P, size_t l, const uint32_t *d_bgra, const ntg_chain_options &o,
                const XformTables *xt, uint8_t *ws, MipJob &J, MipKey &key) {
-    const float *src = P.f_off[l - 1] != NONE ? (const float *)(ws + P.f_off[l - 1]) : nullptr;
+    const float *src = l > 1 ? (const float *)(ws + P.f_off[l - 1]) : nullptr;  // level 1 reads the input's bytes
     uint32_t *q = P.q_off[l] != NONE ? (uint32_t *)(ws + P.q_off[l]) : nullptr;
     return plan_step(ctx, o, P.width, P.p, P.fast_box, src, d_bgra, xt->d_in, P.lv[l - 1], P.lv[l],
                      (float *)(ws + P.f_off[l]), q, xt->d_steps, J, key);
@@ -606,9 +611,8 @@ int run_stages(const std::vector<std::vector<MipLaunch>> &stages, const MipJob *
     return NTG_OK;
 }
 
-// Builds the levels of a chain into the workspace. Level 0 comes straight from the BGRA8 input:
-// the fast box path materialises it as FP32, the polyphase path reads the bytes through the input
-// transform table.
+// Builds the levels of a chain into the workspace. Level 1 reads the BGRA8 input through the input transform
+// table; level 0 is materialised as FP32 only where the call returns it.
 int build_levels(ntg_context *ctx, const ChainPlan &P, const uint32_t *d_bgra, const ntg_chain_options &o,
                  const XformTables *xt, uint8_t *ws, cudaStream_t s) {
     if (P.f_off[0] != NONE) {
@@ -1014,25 +1018,14 @@ static int chain_common(ntg_context *ctx, const void *d_bgra, int w, int h, cons
     const ChainPlan P = plan_chain(w, h, *opt, d_levels != nullptr);
     const XformTables *xt = ctx->xform(opt->in_xform, opt->out_xform, opt->gamma);
     if (!xt) return fail(NTG_ERROR_CUDA, "table upload failed");
-    uint8_t *ws = nullptr;
-    NTG_TRY(ctx->workspace(std::max<size_t>(P.bytes, 256), s, &ws));
-    if (d_levels && P.f_off[0] != NONE && !P.fast_box) {
-        NTG_TRY(launched(launch_set_image((const uint32_t *)d_bgra, (size_t)w * h, xt->d_in, (float *)(ws + P.f_off[0]), s), "set image"));
-    }
+    uint8_t *ws = reinterpret_cast<uint8_t *>(d_levels);  // levels that the call returns are built where they belong
+    if (!d_levels) NTG_TRY(ctx->workspace(std::max<size_t>(P.bytes, 256), s, &ws));
     // The mip levels, then one encoder launch over every level. (Encoding level 0 beside the mip
     // launches, on a lower-priority stream, measured slower: the encoder's CTAs hold nearly all of an
     // SM's registers for ~0.4 ms each, so every mip launch first waits for SMs to drain.)
     if (ctx->profile) NTG_CUDA(cudaEventRecord(ctx->ev[0], s));
     NTG_TRY(build_levels(ctx, P, (const uint32_t *)d_bgra, *opt, xt, ws, s));
     if (ctx->profile) NTG_CUDA(cudaEventRecord(ctx->ev[1], s));
-    if (d_levels) {
-        size_t off = 0;
-        for (size_t l = 0; l < P.lv.size(); l++) {
-            const size_t n = 4 * (size_t)P.lv[l].w * P.lv[l].h;
-            NTG_CUDA(cudaMemcpyAsync(d_levels + off, ws + P.f_off[l], n * sizeof(float), cudaMemcpyDeviceToDevice, s));
-            off += n;
-        }
-    }
     if (d_blocks) {
         std::vector<EncJob> jobs;
         long long nblocks = 0;
@@ -1336,7 +1329,6 @@ struct ntg_batch {
     uint8_t *d_ws = nullptr;
     MipJob *d_mip = nullptr;
     EncJob *d_enc = nullptr;
-    std::vector<int> set_images;          // textures whose level 0 is materialised (box path)
     std::vector<std::vector<MipLaunch>> stages;
     struct Enc {
         int format, quality, first, njobs;
@@ -1423,13 +1415,11 @@ int batch_plan(ntg_batch *b) {
     const size_t n = b->tex.size();
     std::vector<MipJob> all;
     b->stages.clear();
-    b->set_images.clear();
     size_t max_levels = 0;
     std::vector<size_t> tails(n);
     for (size_t t = 0; t < n; t++) {
         max_levels = std::max(max_levels, b->plans[t].lv.size());
         tails[t] = tail_start(b->plans[t], b->tune);
-        if (b->plans[t].f_off[0] != NONE) b->set_images.push_back((int)t);
     }
     for (size_t l = 1; l < max_levels; l++) {
         std::vector<std::pair<MipKey, MipJob>> items;
@@ -1442,26 +1432,31 @@ int batch_plan(ntg_batch *b) {
         }
         std::vector<MipLaunch> stage;
         if (!items.empty()) group_launches(items, b->tune, all, stage);
-        for (int weighted = 0; weighted < 2; weighted++) {  // tails starting at this level
-            MipLaunch m;
-            std::memset(&m, 0, sizeof m);
-            m.kernel = MIP_TAIL;
-            m.weighted = weighted;
-            m.first_job = (int)all.size();
-            long long chains = 0;
-            for (size_t t = 0; t < n; t++) {
-                if (tails[t] != l || (b->opts[t].weighted != 0) != (weighted != 0)) continue;
-                NTG_TRY(chain_tail(ctx, b->plans[t], l, (const uint32_t *)b->io()[t].d_bgra, b->opts[t], b->xts[t],
-                                   b->d_ws + b->base[t], chains++, all));
-            }
-            if (chains) {
-                m.njobs = (int)all.size() - m.first_job;
-                m.units = chains;
-                stage.push_back(m);
-            }
-        }
         if (!stage.empty()) b->stages.push_back(stage);
     }
+    // every texture's tail in one launch, once the level before it is there for all: a tail is one CTA's work, and
+    // launched at the depth where each texture's begins they ran one after the other (five launches in a row for
+    // textures of 64 to 1024)
+    std::vector<MipLaunch> last;
+    for (int weighted = 0; weighted < 2; weighted++) {
+        MipLaunch m;
+        std::memset(&m, 0, sizeof m);
+        m.kernel = MIP_TAIL;
+        m.weighted = weighted;
+        m.first_job = (int)all.size();
+        long long chains = 0;
+        for (size_t t = 0; t < n; t++) {
+            if (tails[t] >= b->plans[t].lv.size() || (b->opts[t].weighted != 0) != (weighted != 0)) continue;
+            NTG_TRY(chain_tail(ctx, b->plans[t], tails[t], (const uint32_t *)b->io()[t].d_bgra, b->opts[t], b->xts[t],
+                               b->d_ws + b->base[t], chains++, all));
+        }
+        if (chains) {
+            m.njobs = (int)all.size() - m.first_job;
+            m.units = chains;
+            last.push_back(m);
+        }
+    }
+    if (!last.empty()) b->stages.push_back(last);
     std::map<std::pair<int, int>, std::vector<size_t>> groups;
     for (size_t t = 0; t < n; t++) groups[{b->opts[t].format, b->opts[t].quality}].push_back(t);
     std::vector<EncJob> ejobs;
@@ -1488,7 +1483,7 @@ int batch_plan(ntg_batch *b) {
     }
     NTG_CUDA(cudaMalloc((void **)&de, ejobs.size() * sizeof(EncJob)));
     NTG_CUDA(cudaMemcpy(de, ejobs.data(), ejobs.size() * sizeof(EncJob), cudaMemcpyHostToDevice));
-    b->launches = (int)b->set_images.size() + (int)b->encodes.size();
+    b->launches = (int)b->encodes.size();
     for (const auto &e : b->encodes)
         if (learned_group(b, e)) b->launches += 3;  // features, network, pruned fit, full-fit list
     for (const auto &st : b->stages) b->launches += (int)st.size();
@@ -1496,11 +1491,6 @@ int batch_plan(ntg_batch *b) {
 }
 
 int batch_mips(ntg_batch *b, cudaStream_t s) {
-    for (int t : b->set_images) {
-        const ChainPlan &P = b->plans[t];
-        NTG_TRY(launched(launch_set_image((const uint32_t *)b->io()[t].d_bgra, (size_t)P.lv[0].w * P.lv[0].h, b->xts[t]->d_in,
-                                          (float *)(b->d_ws + b->base[t] + P.f_off[0]), s), "set image"));
-    }
     return run_stages(b->stages, b->dmip(), s);
 }
 

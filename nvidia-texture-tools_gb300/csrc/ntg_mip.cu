@@ -28,17 +28,29 @@ __device__ unsigned int g_mip_status = 0;
 // transform. The input is 8-bit, so toLinear / toLinearFromSrgb of RGB collapse into a 256-entry
 // table built on the host; alpha is v / 255.
 
+// VEC: four texels a step (the planes and the input on 16-byte boundaries, a multiple of four texels).
+template <bool VEC>
 __global__ void k_set_image(const uint32_t *__restrict__ bgra, size_t n, const float *__restrict__ lut,
                             float *__restrict__ out) {
-    __shared__ float s_lut[256];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) s_lut[i] = lut[i];
+    __shared__ float s_lut[512];
+    for (int i = threadIdx.x; i < 512; i += blockDim.x) s_lut[i] = __ldg(lut + i);
     __syncthreads();
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        uint32_t p = bgra[i];
-        out[i] = s_lut[(p >> 16) & 255];
-        out[n + i] = s_lut[(p >> 8) & 255];
-        out[2 * n + i] = s_lut[p & 255];
-        out[3 * n + i] = (float)(p >> 24) / 255.0f;
+    const size_t steps = VEC ? n / 4 : n;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < steps; i += (size_t)gridDim.x * blockDim.x) {
+        if constexpr (VEC) {
+            const uint4 p = __ldg(reinterpret_cast<const uint4 *>(bgra) + i);
+            float4 *const o = reinterpret_cast<float4 *>(out) + i;
+            o[0] = make_float4(s_lut[(p.x >> 16) & 255], s_lut[(p.y >> 16) & 255], s_lut[(p.z >> 16) & 255], s_lut[(p.w >> 16) & 255]);
+            o[steps] = make_float4(s_lut[(p.x >> 8) & 255], s_lut[(p.y >> 8) & 255], s_lut[(p.z >> 8) & 255], s_lut[(p.w >> 8) & 255]);
+            o[2 * steps] = make_float4(s_lut[p.x & 255], s_lut[p.y & 255], s_lut[p.z & 255], s_lut[p.w & 255]);
+            o[3 * steps] = make_float4(s_lut[256 + (p.x >> 24)], s_lut[256 + (p.y >> 24)], s_lut[256 + (p.z >> 24)], s_lut[256 + (p.w >> 24)]);
+        } else {
+            const uint32_t p = __ldg(bgra + i);
+            out[i] = s_lut[(p >> 16) & 255];
+            out[n + i] = s_lut[(p >> 8) & 255];
+            out[2 * n + i] = s_lut[p & 255];
+            out[3 * n + i] = s_lut[256 + (p >> 24)];
+        }
     }
 }
 
@@ -150,70 +162,90 @@ __device__ __forceinline__ void load_steps(const MipJob *__restrict__ jobs, floa
 // ---------------------------------------------------------------------------------------------
 // FloatImage::fastDownSample (src/nvimage/FloatImage.cpp:559-737): 2x2 box for even sizes,
 // pair average for 1-D images and the three-tap polyphase box for odd sizes. One thread per
-// destination texel, all four channels.
+// destination texel, all four channels. U8: the source is the BGRA8 input through the input transform table (level 1 of
+// every chain): read as FP32 it had to be written first, 16 bytes a texel, by a launch of its own.
+template <bool U8>
 __global__ void k_fast_down(const MipJob *__restrict__ jobs, int njobs, long long units) {
     __shared__ float s_steps[256];
+    __shared__ float s_lut[U8 ? 512 : 1];
     load_steps(jobs, s_steps);
+    if (U8)  // the launch's jobs share the table
+        for (int i = threadIdx.x; i < 512; i += blockDim.x) s_lut[i] = __ldg(jobs[0].lut + i);
     __syncthreads();
     for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < units;
          u += (long long)gridDim.x * blockDim.x) {
         const MipJob &L = jobs[find_mip_job(jobs, njobs, u)];
         const int W = L.W, H = L.H;
-        const float *src0 = L.src;
         const unsigned w = W / 2 > 1 ? (unsigned)W / 2 : 1u, h = H / 2 > 1 ? (unsigned)H / 2 : 1u;
         const size_t sn = (size_t)W * H, dn = (size_t)w * h;
         const unsigned t = (unsigned)(u - L.first_unit);  // levels hold < 2^32 texels: 32-bit division
         const unsigned x = t % w, y = t / w;
-        float v[4];
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const float *src = src0 + c * sn;
-            float f;
-            if (W == 1 || H == 1) {
-                const unsigned n = w * h, i = (unsigned)t;
-                const float *s = src + 2 * (size_t)i;
-                if (((unsigned)W * (unsigned)H) & 1) {
-                    const float scale = 1.0f / (2 * n + 1);
-                    const float w0 = (float)(n - i), w1 = (float)(n - 0), w2 = (float)(1 + i);
-                    f = scale * (w0 * s[0] + w1 * s[1] + w2 * s[2]);
-                } else {
-                    f = 0.5f * (s[0] + s[1]);
-                }
-            } else if ((W & 1) == 0 && (H & 1) == 0) {
-                const float *s = src + (size_t)(2 * y) * W + 2 * x;
-                f = 0.25f * (s[0] + s[1] + s[W] + s[W + 1]);
-            } else if ((W & 1) && (H & 1)) {
-                const float scale = 1.0f / (float)((unsigned)W * (unsigned)H);
-                const float v0 = (float)(h - y), v1 = (float)(h - 0), v2 = (float)(1 + y);
-                const float w0 = (float)(w - x), w1 = (float)(w - 0), w2 = (float)(1 + x);
-                const float *s = src + (size_t)(2 * y) * W + 2 * x;
-                float acc = 0.0f;
-                acc += v0 * (w0 * s[0] + w1 * s[1] + w2 * s[2]);
-                acc += v1 * (w0 * s[W] + w1 * s[W + 1] + w2 * s[W + 2]);
-                acc += v2 * (w0 * s[2 * W] + w1 * s[2 * W + 1] + w2 * s[2 * W + 2]);
-                f = acc * scale;
-            } else if (W & 1) {
-                const float scale = 1.0f / (float)(2 * (unsigned)W);
-                const float w0 = (float)(w - x), w1 = (float)(w - 0), w2 = (float)(1 + x);
-                const float *s = src + (size_t)(2 * y) * W + 2 * x;
-                float acc = 0.0f;
-                acc += w0 * (s[0] + s[W]);
-                acc += w1 * (s[1] + s[W + 1]);
-                acc += w2 * (s[2] + s[W + 2]);
-                f = acc * scale;
+        auto texel = [&](size_t i, float (&v)[4]) {
+            if (U8) {
+                const uint32_t p = __ldg(L.bgra8 + i);
+                v[0] = s_lut[(p >> 16) & 255]; v[1] = s_lut[(p >> 8) & 255]; v[2] = s_lut[p & 255]; v[3] = s_lut[256 + (p >> 24)];
             } else {
-                const float scale = 1.0f / (float)(2 * (unsigned)H);
-                const float v0 = (float)(h - y), v1 = (float)(h - 0), v2 = (float)(1 + y);
-                const float *s = src + (size_t)(2 * y) * W + 2 * x;
-                float acc = 0.0f;
-                acc += v0 * (s[0] + s[1]);
-                acc += v1 * (s[W] + s[W + 1]);
-                acc += v2 * (s[2 * W] + s[2 * W + 1]);
-                f = acc * scale;
+#pragma unroll
+                for (int c = 0; c < 4; c++) v[c] = __ldg(L.src + c * sn + i);
             }
-            v[c] = f;
-            L.dst[c * dn + t] = f;
+        };
+        float v[4];
+        if (W == 1 || H == 1) {
+            const unsigned n = w * h, i = (unsigned)t;
+            float a[4], b[4];
+            texel(2 * (size_t)i, a);
+            texel(2 * (size_t)i + 1, b);
+            if (((unsigned)W * (unsigned)H) & 1) {
+                const float scale = 1.0f / (2 * n + 1);
+                const float w0 = (float)(n - i), w1 = (float)(n - 0), w2 = (float)(1 + i);
+                float d[4];
+                texel(2 * (size_t)i + 2, d);
+#pragma unroll
+                for (int c = 0; c < 4; c++) v[c] = scale * (w0 * a[c] + w1 * b[c] + w2 * d[c]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; c++) v[c] = 0.5f * (a[c] + b[c]);
+            }
+        } else {
+            // the window's texels: 2 or 3 per axis
+            const bool ox = W & 1, oy = H & 1;
+            const size_t s = (size_t)(2 * y) * W + 2 * x;
+            float q[3][3][4];
+#pragma unroll
+            for (int j = 0; j < 3; j++)
+#pragma unroll
+                for (int i = 0; i < 3; i++)
+                    if ((j < 2 || oy) && (i < 2 || ox)) texel(s + (size_t)j * W + i, q[j][i]);
+            const float v0 = (float)(h - y), v1 = (float)(h - 0), v2 = (float)(1 + y);
+            const float w0 = (float)(w - x), w1 = (float)(w - 0), w2 = (float)(1 + x);
+            const float both = 1.0f / (float)((unsigned)W * (unsigned)H), wide = 1.0f / (float)(2 * (unsigned)W), tall = 1.0f / (float)(2 * (unsigned)H);
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                if (!ox && !oy) {
+                    v[c] = 0.25f * (q[0][0][c] + q[0][1][c] + q[1][0][c] + q[1][1][c]);
+                } else if (ox && oy) {
+                    float acc = 0.0f;
+                    acc += v0 * (w0 * q[0][0][c] + w1 * q[0][1][c] + w2 * q[0][2][c]);
+                    acc += v1 * (w0 * q[1][0][c] + w1 * q[1][1][c] + w2 * q[1][2][c]);
+                    acc += v2 * (w0 * q[2][0][c] + w1 * q[2][1][c] + w2 * q[2][2][c]);
+                    v[c] = acc * both;
+                } else if (ox) {
+                    float acc = 0.0f;
+                    acc += w0 * (q[0][0][c] + q[1][0][c]);
+                    acc += w1 * (q[0][1][c] + q[1][1][c]);
+                    acc += w2 * (q[0][2][c] + q[1][2][c]);
+                    v[c] = acc * wide;
+                } else {
+                    float acc = 0.0f;
+                    acc += v0 * (q[0][0][c] + q[0][1][c]);
+                    acc += v1 * (q[1][0][c] + q[1][1][c]);
+                    acc += v2 * (q[2][0][c] + q[2][1][c]);
+                    v[c] = acc * tall;
+                }
+            }
         }
+#pragma unroll
+        for (int c = 0; c < 4; c++) L.dst[c * dn + t] = v[c];
         if (L.q_out) L.q_out[t] = quantize_bgra(v[0], v[1], v[2], v[3], L.xform, s_steps);
     }
 }
@@ -251,16 +283,6 @@ __device__ __forceinline__ bool in_box(int lo, int hi, int b0, int bn, int n, in
 }
 __device__ __forceinline__ int box_remap(int x, int b0, int n, int wrap) { return wrap_index(b0 + x, n, wrap) - b0; }
 
-template <bool SRC_U8>
-__device__ __forceinline__ float4 load_texel(const MipJob &L, size_t s, size_t sn) {
-    if (SRC_U8) {
-        const uint32_t p = __ldg(L.bgra8 + s);
-        return make_float4(__ldg(L.lut + ((p >> 16) & 255)), __ldg(L.lut + ((p >> 8) & 255)), __ldg(L.lut + (p & 255)),
-                           (float)(p >> 24) / 255.0f);
-    }
-    return make_float4(__ldg(L.src + s), __ldg(L.src + sn + s), __ldg(L.src + 2 * sn + s), __ldg(L.src + 3 * sn + s));
-}
-
 // One tap: sum += k * v for every channel (the weighted form weighs RGB by k * (alpha + 1/256)).
 template <bool WEIGHTED>
 __device__ __forceinline__ void tap(float4 &sum, float &norm, float k, const float4 v) {
@@ -291,7 +313,7 @@ __device__ __forceinline__ void store_texel(const MipJob &L, size_t o, size_t dn
 constexpr int PTW = 32;    // general kernel: output tile width (one warp lane per output column)
 constexpr int PTH = 16;    // general kernel: output tile height
 constexpr int PMAXW = 32;  // widest window handled
-constexpr int PTHREADS = 256;
+constexpr int PTHREADS = 512;
 constexpr int PWARPS = PTHREADS / 32;
 
 // General kernel, any scale and window (odd sizes, 1-wide axes). One CTA per PTW x PTH output
@@ -302,6 +324,7 @@ __global__ void __launch_bounds__(PTHREADS) k_poly(const MipJob *__restrict__ jo
     extern __shared__ float4 sm4[];
     __shared__ float s_kx[PTW * PMAXW], s_ky[PTH * PMAXW], s_steps[256];
     __shared__ int s_lx[PTW], s_ly[PTH];
+    __shared__ float s_lut[SRC_U8 ? 512 : 1];
     load_steps(jobs, s_steps);
     const MipJob &L = jobs[find_mip_job(jobs, njobs, blockIdx.x)];
     const int lu = (int)(blockIdx.x - L.first_unit);
@@ -316,6 +339,8 @@ __global__ void __launch_bounds__(PTHREADS) k_poly(const MipJob *__restrict__ jo
     int *s_col = reinterpret_cast<int *>(s_tmp + ry * PTW);  // rx
     int *s_row = s_col + rx;                                  // ry
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (SRC_U8)
+        for (int i = tid; i < 512; i += PTHREADS) s_lut[i] = __ldg(L.lut + i);
     for (int i = tid; i < tw * wsx; i += PTHREADS) s_kx[i] = L.kx[(size_t)ox0 * wsx + i];
     for (int i = tid; i < th * wsy; i += PTHREADS) s_ky[i] = L.ky[(size_t)oy0 * wsy + i];
     if (tid < tw) s_lx[tid] = L.lx[ox0 + tid] - xlo;
@@ -327,7 +352,16 @@ __global__ void __launch_bounds__(PTHREADS) k_poly(const MipJob *__restrict__ jo
     const size_t sn = (size_t)L.W * L.H;
     for (int r = warp; r < ry; r += PWARPS) {
         const size_t rowoff = (size_t)s_row[r] * L.W;
-        for (int x = lane; x < rx; x += 32) s_in[r * rx + x] = load_texel<SRC_U8>(L, rowoff + s_col[x], sn);
+#pragma unroll 3
+        for (int x = lane; x < rx; x += 32) {
+            const size_t s = rowoff + s_col[x];
+            if (SRC_U8) {
+                const uint32_t p = __ldg(L.bgra8 + s);
+                s_in[r * rx + x] = make_float4(s_lut[(p >> 16) & 255], s_lut[(p >> 8) & 255], s_lut[p & 255], s_lut[256 + (p >> 24)]);
+            } else {
+                s_in[r * rx + x] = make_float4(__ldg(L.src + s), __ldg(L.src + sn + s), __ldg(L.src + 2 * sn + s), __ldg(L.src + 3 * sn + s));
+            }
+        }
     }
     __syncthreads();
 
@@ -338,6 +372,7 @@ __global__ void __launch_bounds__(PTHREADS) k_poly(const MipJob *__restrict__ jo
             const float4 *row = s_in + r * rx + off;
             float4 sum = make_float4(0, 0, 0, 0);
             float norm = 0;
+#pragma unroll 4
             for (int j = 0; j < wsx; j++) tap<WEIGHTED>(sum, norm, k[j], row[j]);
             s_tmp[r * PTW + lane] = finish<WEIGHTED>(sum, norm);
         }
@@ -351,6 +386,7 @@ __global__ void __launch_bounds__(PTHREADS) k_poly(const MipJob *__restrict__ jo
             const float4 *col = s_tmp + s_ly[y] * PTW + lane;
             float4 sum = make_float4(0, 0, 0, 0);
             float norm = 0;
+#pragma unroll 4
             for (int j = 0; j < wsy; j++) tap<WEIGHTED>(sum, norm, k[j], col[j * PTW]);
             store_texel(L, (size_t)(oy0 + y) * L.w + ox0 + lane, dn, finish<WEIGHTED>(sum, norm), s_steps);
         }
@@ -990,58 +1026,80 @@ __global__ void __launch_bounds__(1024, 1) k_tile2x_f32(const MipJob *__restrict
 
 // Chain tails: once a texture's level is small (at most TAIL_MAX texels), one CTA finishes every
 // remaining level in shared memory, one level after the other, instead of one latency-bound
-// launch per tiny level. Levels are planar FP32 in shared memory; each polyphase step runs the
+// launch per tiny level. Levels are float4 texels in shared memory; each polyphase step runs the
 // X pass over every source row into a plane, then the Y pass (applyKernelX / applyKernelY order),
 // box steps use the fastDownSample formulas; every level is also written out. The jobs of a tail
 // are consecutive in the list: the first carries the number of levels in tiles_x, and all carry
 // the chain's index in first_unit.
+// Bound by latency (one CTA, a serial sum per output). The wrapped source position of every tap of every level is
+// therefore tabled beside its weight before the first level, so that a tap is three shared-memory loads whose
+// addresses depend on nothing and the sum's chain is its additions alone; with the wrap evaluated per tap, planes
+// loaded one by one and the tables laid out by one thread, five levels from 32x32 took 33 us (Kaiser) and 27 (triangle) from cold caches, and take 19 and 18.
 constexpr int TAIL_MAX = 4096;
-constexpr int TAIL_TAB = 12288;  // words of shared memory for the levels' weights and window starts
+constexpr int TAIL_TAB = 8192;  // taps of all levels in shared memory (weight and position)
+constexpr int TAIL_LEVELS = 16;
 
-__device__ __forceinline__ float fast_box_texel(const float *src, int W, int H, unsigned w, unsigned h, unsigned t) {
-    const unsigned x = t % w, y = t / w;
+// FloatImage::fastDownSample of one channel; texels STR floats apart.
+template <int STR>
+__device__ __forceinline__ float fast_box_texel(const float *src, int W, int H, unsigned w, unsigned h, unsigned x, unsigned y) {
     if (W == 1 || H == 1) {
-        const unsigned n = w * h, i = t;
-        const float *s = src + 2 * (size_t)i;
+        const unsigned n = w * h, i = y * w + x;
+        const float *s = src + 2 * STR * (size_t)i;
         if (((unsigned)W * (unsigned)H) & 1) {
             const float scale = 1.0f / (2 * n + 1);
             const float w0 = (float)(n - i), w1 = (float)(n - 0), w2 = (float)(1 + i);
-            return scale * (w0 * s[0] + w1 * s[1] + w2 * s[2]);
+            return scale * (w0 * s[0] + w1 * s[STR] + w2 * s[2 * STR]);
         }
-        return 0.5f * (s[0] + s[1]);
+        return 0.5f * (s[0] + s[STR]);
     }
-    const float *s = src + (size_t)(2 * y) * W + 2 * x;
-    if ((W & 1) == 0 && (H & 1) == 0) return 0.25f * (s[0] + s[1] + s[W] + s[W + 1]);
+    const float *s = src + STR * ((size_t)(2 * y) * W + 2 * x);
+    const int R = STR * W;
+    if ((W & 1) == 0 && (H & 1) == 0) return 0.25f * (s[0] + s[STR] + s[R] + s[R + STR]);
     if ((W & 1) && (H & 1)) {
         const float scale = 1.0f / (float)((unsigned)W * (unsigned)H);
         const float v0 = (float)(h - y), v1 = (float)(h - 0), v2 = (float)(1 + y);
         const float w0 = (float)(w - x), w1 = (float)(w - 0), w2 = (float)(1 + x);
         float acc = 0.0f;
-        acc += v0 * (w0 * s[0] + w1 * s[1] + w2 * s[2]);
-        acc += v1 * (w0 * s[W] + w1 * s[W + 1] + w2 * s[W + 2]);
-        acc += v2 * (w0 * s[2 * W] + w1 * s[2 * W + 1] + w2 * s[2 * W + 2]);
+        acc += v0 * (w0 * s[0] + w1 * s[STR] + w2 * s[2 * STR]);
+        acc += v1 * (w0 * s[R] + w1 * s[R + STR] + w2 * s[R + 2 * STR]);
+        acc += v2 * (w0 * s[2 * R] + w1 * s[2 * R + STR] + w2 * s[2 * R + 2 * STR]);
         return acc * scale;
     }
     if (W & 1) {
         const float scale = 1.0f / (float)(2 * (unsigned)W);
         const float w0 = (float)(w - x), w1 = (float)(w - 0), w2 = (float)(1 + x);
         float acc = 0.0f;
-        acc += w0 * (s[0] + s[W]);
-        acc += w1 * (s[1] + s[W + 1]);
-        acc += w2 * (s[2] + s[W + 2]);
+        acc += w0 * (s[0] + s[R]);
+        acc += w1 * (s[STR] + s[R + STR]);
+        acc += w2 * (s[2 * STR] + s[R + 2 * STR]);
         return acc * scale;
     }
     const float scale = 1.0f / (float)(2 * (unsigned)H);
     const float v0 = (float)(h - y), v1 = (float)(h - 0), v2 = (float)(1 + y);
     float acc = 0.0f;
-    acc += v0 * (s[0] + s[1]);
-    acc += v1 * (s[W] + s[W + 1]);
-    acc += v2 * (s[2 * W] + s[2 * W + 1]);
+    acc += v0 * (s[0] + s[STR]);
+    acc += v1 * (s[R] + s[R + STR]);
+    acc += v2 * (s[2 * R] + s[2 * R + STR]);
     return acc * scale;
 }
 
 size_t tail_smem_bytes() {
-    return (size_t)4 * (TAIL_MAX + TAIL_MAX / 2 + TAIL_MAX / 2) * sizeof(float) + TAIL_TAB * sizeof(float);
+    return (size_t)(TAIL_MAX + TAIL_MAX / 2 + TAIL_MAX / 2) * sizeof(float4) + TAIL_TAB * (sizeof(float) + sizeof(int));
+}
+
+// The taps of one output: `k` and `at` are the tabled weights and positions, or (at null) the level's weights and its
+// window start `left`, wrapped here.
+template <bool WEIGHTED>
+__device__ __forceinline__ float4 tail_taps(const float4 *src, int stride, const float *k, const int *at, int ws, int left, int n, int wrap) {
+    float4 sum = make_float4(0, 0, 0, 0);
+    float norm = 0;
+    if (at) {
+#pragma unroll 4
+        for (int j = 0; j < ws; j++) tap<WEIGHTED>(sum, norm, k[j], src[at[j] * stride]);
+    } else {
+        for (int j = 0; j < ws; j++) tap<WEIGHTED>(sum, norm, __ldg(k + j), src[wrap_index(left + j, n, wrap) * stride]);
+    }
+    return finish<WEIGHTED>(sum, norm);
 }
 
 template <bool WEIGHTED>
@@ -1049,21 +1107,22 @@ __global__ void __launch_bounds__(1024) k_mip_tail(const MipJob *__restrict__ jo
     extern __shared__ float4 sm4[];
     __shared__ float s_steps[256];
     __shared__ uint8_t s_buckets[kSrgbBuckets];
-    __shared__ int s_off[16][4];  // per level: offsets of kx, ky, lx, ly in s_tab, or -1 (read from global)
-    float *const lv0 = reinterpret_cast<float *>(sm4);  // levels alternate between two buffers: 4 planes of TAIL_MAX
-    float *const s_t = lv0 + 4 * TAIL_MAX;              // X pass, 4 planes of up to TAIL_MAX / 2
-    float *const lv1 = s_t + 2 * TAIL_MAX;              // 4 planes of up to TAIL_MAX / 2
-    float *const s_tab = lv1 + 2 * TAIL_MAX;            // every level's weights and window starts
+    __shared__ MipJob s_jobs[TAIL_LEVELS];
+    __shared__ int s_first;
+    float4 *const lv0 = sm4;                 // levels alternate between two buffers: TAIL_MAX texels
+    float4 *const s_t = lv0 + TAIL_MAX;      // X pass, up to TAIL_MAX / 2
+    float4 *const lv1 = s_t + TAIL_MAX / 2;  // up to TAIL_MAX / 2
+    float *const s_k = reinterpret_cast<float *>(lv1 + TAIL_MAX / 2);
+    int *const s_at = reinterpret_cast<int *>(s_k + TAIL_TAB);
     const int tid = threadIdx.x, nt = blockDim.x;
-    int j0 = 0, hi = njobs - 1;  // first job of chain blockIdx.x
-    while (j0 < hi) {
-        const int mid = (j0 + hi) >> 1;
-        if (jobs[mid].first_unit < (long long)blockIdx.x) j0 = mid + 1;
-        else hi = mid;
-    }
+    if (tid == 0) s_first = njobs - 1;
+    __syncthreads();
+    for (int i = tid; i < njobs; i += nt)  // first job of chain blockIdx.x
+        if (jobs[i].first_unit == (long long)blockIdx.x) { atomicMin(&s_first, i); break; }
+    __syncthreads();
+    const int j0 = s_first;
     // the chain's job records, copied to shared memory once (every thread reads them every level)
-    __shared__ MipJob s_jobs[16];
-    const int count = min(jobs[j0].tiles_x, 16);
+    const int count = min(jobs[j0].tiles_x, TAIL_LEVELS);
     {
         static_assert(sizeof(MipJob) % 8 == 0, "job records copy as 8-byte words");
         const unsigned long long *src = reinterpret_cast<const unsigned long long *>(jobs + j0);
@@ -1073,19 +1132,6 @@ __global__ void __launch_bounds__(1024) k_mip_tail(const MipJob *__restrict__ jo
     }
     __syncthreads();
     const bool quant = s_jobs[0].q_out != nullptr, srgb = quant && s_jobs[0].xform == 2;
-    if (tid == 0) {  // table layout: each level's tables where they fit, in level order
-        int off = 0;
-        for (int k = 0; k < count; k++) {
-            const MipJob &L = s_jobs[k];
-            const int need = L.kx ? L.w * L.wsx + L.h * L.wsy + L.w + L.h : 0;
-            const bool fit = L.kx && off + need <= TAIL_TAB;
-            s_off[k][0] = fit ? off : -1;
-            s_off[k][1] = fit ? off + L.w * L.wsx : -1;
-            s_off[k][2] = fit ? off + L.w * L.wsx + L.h * L.wsy : -1;
-            s_off[k][3] = fit ? off + L.w * L.wsx + L.h * L.wsy + L.w : -1;
-            if (fit) off += need;
-        }
-    }
     if (quant)
         for (int i = tid; i < 256; i += nt) s_steps[i] = __ldg(s_jobs[0].steps + i);
     if (srgb)
@@ -1094,79 +1140,61 @@ __global__ void __launch_bounds__(1024) k_mip_tail(const MipJob *__restrict__ jo
     {  // stage the chain's source level
         const MipJob &L = s_jobs[0];
         const int n = L.W * L.H;
-        float *s_a = lv0;
         for (int i = tid; i < n; i += nt) {
             if (L.src) {
-#pragma unroll
-                for (int c = 0; c < 4; c++) s_a[c * n + i] = __ldg(L.src + (size_t)c * n + i);
+                lv0[i] = make_float4(__ldg(L.src + i), __ldg(L.src + (size_t)n + i), __ldg(L.src + 2 * (size_t)n + i), __ldg(L.src + 3 * (size_t)n + i));
             } else {
                 const uint32_t q = __ldg(L.bgra8 + i);
-                s_a[i] = __ldg(L.lut + ((q >> 16) & 255));
-                s_a[n + i] = __ldg(L.lut + ((q >> 8) & 255));
-                s_a[2 * n + i] = __ldg(L.lut + (q & 255));
-                s_a[3 * n + i] = __ldg(L.lut + 256 + (q >> 24));
+                lv0[i] = make_float4(__ldg(L.lut + ((q >> 16) & 255)), __ldg(L.lut + ((q >> 8) & 255)), __ldg(L.lut + (q & 255)),
+                                     __ldg(L.lut + 256 + (q >> 24)));
             }
         }
     }
-    __syncthreads();
-    for (int k = 0; k < count; k++) {  // all levels' tables at once: one round of global latency
+    // every level's taps, X then Y, in level order as far as they fit
+    for (int k = 0, off = 0; k < count; k++) {
         const MipJob &L = s_jobs[k];
-        if (s_off[k][0] < 0) continue;
-        for (int i = tid; i < L.w * L.wsx; i += nt) s_tab[s_off[k][0] + i] = __ldg(L.kx + i);
-        for (int i = tid; i < L.h * L.wsy; i += nt) s_tab[s_off[k][1] + i] = __ldg(L.ky + i);
-        for (int i = tid; i < L.w; i += nt) reinterpret_cast<int *>(s_tab)[s_off[k][2] + i] = __ldg(L.lx + i);
-        for (int i = tid; i < L.h; i += nt) reinterpret_cast<int *>(s_tab)[s_off[k][3] + i] = __ldg(L.ly + i);
+        if (!L.kx) break;
+        const int nx = L.w * L.wsx, ny = L.h * L.wsy;
+        if (off + nx + ny > TAIL_TAB) continue;
+        for (int i = tid; i < nx + ny; i += nt) {
+            const bool y = i >= nx;
+            const int e = y ? i - nx : i, ws = y ? L.wsy : L.wsx, o = (int)((unsigned)e / (unsigned)ws);
+            s_k[off + i] = __ldg((y ? L.ky : L.kx) + e);
+            s_at[off + i] = wrap_index(__ldg((y ? L.ly : L.lx) + o) + e - o * ws, y ? L.H : L.W, L.wrap);
+        }
+        off += nx + ny;
     }
     __syncthreads();
-    for (int k = 0; k < count; k++) {
+    for (int k = 0, off = 0; k < count; k++) {
         const MipJob &L = s_jobs[k];
-        const float *src = (k & 1) ? lv1 : lv0;
-        float *dstb = (k & 1) ? lv0 : lv1;
+        const float4 *src = (k & 1) ? lv1 : lv0;
+        float4 *dstb = (k & 1) ? lv0 : lv1;
         const int W = L.W, H = L.H, w = L.w, h = L.h, wrap = L.wrap;
-        const int sn = W * H, tn = H * w, dn = w * h;
-        const int wsx = L.wsx, wsy = L.wsy;
-        const bool staged = s_off[k][0] >= 0;
-        const float *kxs = staged ? s_tab + s_off[k][0] : L.kx;
-        const float *kys = staged ? s_tab + s_off[k][1] : L.ky;
-        const int *lxs = staged ? reinterpret_cast<const int *>(s_tab) + s_off[k][2] : L.lx;
-        const int *lys = staged ? reinterpret_cast<const int *>(s_tab) + s_off[k][3] : L.ly;
+        const int tn = H * w, dn = w * h, wsx = L.wsx, wsy = L.wsy;
+        const int nx = w * wsx, ny = h * wsy;
+        const bool staged = L.kx && off + nx + ny <= TAIL_TAB;
+        const float *const kx = staged ? s_k + off : L.kx, *const ky = staged ? kx + nx : L.ky;
+        const int *const ax = staged ? s_at + off : nullptr, *const ay = staged ? ax + nx : nullptr;
+        if (staged) off += nx + ny;
+        const float inv = 1.0f / (float)w;  // i / w for i below 2^13 and w below 2^12: exact with the half added
         if (L.kx) {
             for (int i = tid; i < tn; i += nt) {  // X taps of every source row
-                const int y = i / w, x = i - y * w;
-                const float *kx = kxs + x * wsx;
-                const int lx = lxs[x];
-                const bool inside = lx >= 0 && lx + wsx <= W;
-                const float *row = src + y * W;
-                float4 sum = make_float4(0, 0, 0, 0);
-                float norm = 0;
-                for (int j = 0; j < wsx; j++) {
-                    const int s = inside ? lx + j : wrap_index(lx + j, W, wrap);
-                    tap<WEIGHTED>(sum, norm, kx[j], make_float4(row[s], row[sn + s], row[2 * sn + s], row[3 * sn + s]));
-                }
-                sum = finish<WEIGHTED>(sum, norm);
-                s_t[i] = sum.x; s_t[tn + i] = sum.y; s_t[2 * tn + i] = sum.z; s_t[3 * tn + i] = sum.w;
+                const int y = (int)(((float)i + 0.5f) * inv), x = i - y * w;
+                s_t[i] = tail_taps<WEIGHTED>(src + y * W, 1, kx + x * wsx, ax ? ax + x * wsx : nullptr, wsx, ax ? 0 : __ldg(L.lx + x), W, wrap);
             }
             __syncthreads();
         }
         for (int o = tid; o < dn; o += nt) {  // Y taps (or the box step), then out to the level
+            const int y = (int)(((float)o + 0.5f) * inv), x = o - y * w;
             float4 v;
             if (L.kx) {
-                const int y = o / w, x = o - y * w;
-                const float *ky = kys + y * wsy;
-                const int ly = lys[y];
-                const bool inside = ly >= 0 && ly + wsy <= H;
-                float4 sum = make_float4(0, 0, 0, 0);
-                float norm = 0;
-                for (int j = 0; j < wsy; j++) {
-                    const int s = (inside ? ly + j : wrap_index(ly + j, H, wrap)) * w + x;
-                    tap<WEIGHTED>(sum, norm, ky[j], make_float4(s_t[s], s_t[tn + s], s_t[2 * tn + s], s_t[3 * tn + s]));
-                }
-                v = finish<WEIGHTED>(sum, norm);
+                v = tail_taps<WEIGHTED>(s_t + x, w, ky + y * wsy, ay ? ay + y * wsy : nullptr, wsy, ay ? 0 : __ldg(L.ly + y), H, wrap);
             } else {
-                v = make_float4(fast_box_texel(src, W, H, w, h, o), fast_box_texel(src + sn, W, H, w, h, o),
-                                fast_box_texel(src + 2 * sn, W, H, w, h, o), fast_box_texel(src + 3 * sn, W, H, w, h, o));
+                const float *const f = reinterpret_cast<const float *>(src);
+                v = make_float4(fast_box_texel<4>(f, W, H, w, h, x, y), fast_box_texel<4>(f + 1, W, H, w, h, x, y),
+                                fast_box_texel<4>(f + 2, W, H, w, h, x, y), fast_box_texel<4>(f + 3, W, H, w, h, x, y));
             }
-            dstb[o] = v.x; dstb[dn + o] = v.y; dstb[2 * dn + o] = v.z; dstb[3 * dn + o] = v.w;
+            dstb[o] = v;
             L.dst[o] = v.x;
             L.dst[dn + o] = v.y;
             L.dst[2 * dn + o] = v.z;
@@ -1248,7 +1276,10 @@ int launch_srgb_fix(const float *host_chunk, uint32_t first, uint32_t count, int
 
 int launch_set_image(const uint32_t *bgra, size_t n, const float *lut, float *out, cudaStream_t s) {
     if (n == 0) return 0;
-    k_set_image<<<grid_for(n, 256), 256, 0, s>>>(bgra, n, lut, out);
+    if (n % 4 == 0 && reinterpret_cast<uintptr_t>(bgra) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0)
+        k_set_image<true><<<grid_for(n / 4, 256), 256, 0, s>>>(bgra, n, lut, out);
+    else
+        k_set_image<false><<<grid_for(n, 256), 256, 0, s>>>(bgra, n, lut, out);
     return launch_status();
 }
 
@@ -1431,7 +1462,8 @@ int launch_mip(const MipLaunch &m, const MipJob *d_jobs, cudaStream_t s) {
     switch (m.kernel) {
         case MIP_FAST_BOX: {
             const long long cap = 152LL * 64, g = (m.units + 255) / 256;
-            k_fast_down<<<(unsigned)(g < cap ? g : cap), 256, 0, s>>>(jobs, m.njobs, m.units);
+            if (m.u8) k_fast_down<true><<<(unsigned)(g < cap ? g : cap), 256, 0, s>>>(jobs, m.njobs, m.units);
+            else k_fast_down<false><<<(unsigned)(g < cap ? g : cap), 256, 0, s>>>(jobs, m.njobs, m.units);
             return launch_status();
         }
         case MIP_POLY:
