@@ -706,38 +706,6 @@ __global__ void __launch_bounds__(64) k_bc1_box(const EncJob *__restrict__ jobs,
 // and 24 us (8 lanes per block before), 256x256 75 and 34, 1024x1024 416 and 316, 2048x2048 1,317 and 1,228,
 // 1024x1024 after toSrgb 503 and 360 (texels gathered once instead of three times), 512x512 at Level9 627 and 200.
 
-constexpr unsigned kAll = 0xffffffffu;
-
-// One half's scratch in shared memory.
-struct HalfScratch {
-    float stage[16 * 8];  // terms per texel or colour
-    float pad[8];         // the two halves' stages lie on different banks
-    float4 table[2][18];  // the ZERO summed-area tables (17 entries) of the two fits
-    ScanBlock block[2];   // and their scans' constants
-    float ends[12];       // the fits' end points
-};
-struct WarpScratch {
-    ScanScratch scan;
-    HalfScratch half[2];
-};
-
-struct Half {
-    int hl;         // lane in the half: texel or colour index
-    int shift;      // first lane of the half
-    HalfScratch *s;
-    __device__ __forceinline__ float get(float v, int src) const { return __shfl_sync(kAll, v, src, 16); }
-    __device__ __forceinline__ unsigned ballot(bool p) const { return (__ballot_sync(kAll, p) >> shift) & 0xffffu; }
-    // Sum over i < n, in order, of the terms stage[8 i + c]; lane c of the half returns it.
-    __device__ __forceinline__ float ordered(int n) const {
-        float acc = 0.0f;
-        const float *p = s->stage + (hl & 7);
-#pragma unroll
-        for (int i = 0; i < 16; i++)
-            if (i < n) acc += p[8 * i];
-        return acc;
-    }
-};
-
 // reduce_colors (src/nvtt/icbc.h:1638-1683): the texels in order, each matched against the colours so far, which the
 // half's lanes hold one each. Returns the colour count.
 __device__ __forceinline__ int half_reduce(const Half &H, float4 texel, float4 &q) {
@@ -811,34 +779,8 @@ __device__ __noinline__ void half_sat(Half H, float4 q, int n, f3 metric, int wh
         }
     }
     __syncwarp();
-    // positions along the axis in a stable insertion sort's order: the rank, unless a projection is NaN
     const float d = dot(xyz(q), v);
-    int rank = 0;
-#pragma unroll
-    for (int j = 0; j < 16; j++) {
-        const float e = H.get(d, j);
-        rank += j < n && (e < d || (e == d && j < hl));
-    }
-    const bool odd = H.ballot(hl < n && d != d) != 0;
-    if (__any_sync(kAll, odd)) {
-        float *const key = st;
-        int *const ord = reinterpret_cast<int *>(st + 16), *const pos = reinterpret_cast<int *>(st + 32);
-        __syncwarp();
-        key[hl] = d;
-        __syncwarp();
-        if (hl == 0) {
-            for (int i = 0; i < n; i++) ord[i] = i;
-            for (int i = 1; i < n; i++)
-                for (int j = i; j > 0 && key[j] < key[j - 1]; j--) {
-                    const float t = key[j]; key[j] = key[j - 1]; key[j - 1] = t;
-                    const int o = ord[j]; ord[j] = ord[j - 1]; ord[j - 1] = o;
-                }
-            for (int i = 0; i < n; i++) pos[ord[i]] = i;
-        }
-        __syncwarp();
-        if (odd && hl < n) rank = pos[hl];
-        __syncwarp();
-    }
+    const int rank = half_rank(H, d, n);
     if (hl < n) *reinterpret_cast<float4 *>(st + 4 * rank) = make_float4(q.x * q.w, q.y * q.w, q.z * q.w, q.w);
     __syncwarp();
     float acc = 0.0f;
@@ -858,7 +800,7 @@ __device__ __noinline__ void half_sat(Half H, float4 q, int n, f3 metric, int wh
     const bool whole = H.ballot(hl < n && q.w != floorf(q.w)) == 0;
     const f3 sum = mk3(H.get(acc, 0), H.get(acc, 1), H.get(acc, 2));
     const float wsum = H.get(acc, 3);
-    if (hl == 0) scan_begin(H.s->block[which], n, sum, wsum, big, m0 + m3 + m5, whole, metric, 46.0f, 47.0f);
+    if (hl == 0) scan_begin(H.s->block[which], n, sum, wsum, big, m0 + m3 + m5, whole, metric, 46.0f, 47.0f, whole ? 0.0f : 67.0f);
     __syncwarp();
 }
 
@@ -897,14 +839,6 @@ __device__ __forceinline__ void warp_fit(WarpScratch &w, int b, int n4, int n3, 
     best4.finish(h.ends);
     best3.finish(h.ends + 6);
     __syncwarp();
-}
-
-// Bit i of m to bit 2 i.
-__device__ __forceinline__ uint32_t spread_bits(uint32_t m) {
-    m = (m | (m << 8)) & 0x00ff00ffu;
-    m = (m | (m << 4)) & 0x0f0f0f0fu;
-    m = (m | (m << 2)) & 0x33333333u;
-    return (m | (m << 1)) & 0x55555555u;
 }
 
 // evaluate_mse over the input texels (src/nvtt/icbc.h:2733-2756): lane k's texel has index code k.
@@ -1016,7 +950,6 @@ __device__ __forceinline__ float4 gather_texel(const EncJob &J, int blk, int k) 
 #ifndef NTG_BC1_MIN_CTAS
 #define NTG_BC1_MIN_CTAS 5
 #endif
-constexpr int kFitWarps = 4;  // warps per CTA, each on its own
 
 // icbc Level8 (LEVEL 7) and Level9 (LEVEL 8).
 template <int LEVEL>

@@ -13,9 +13,12 @@
 // shared memory as [element][thread] because the cluster-split loops index them by running
 // counts. Blocks with 16 distinct colours (the common case) all run the same 969-split schedule,
 // so those warps do not diverge in the search. Built with --fmad=false.
+#include <memory>
+
 #include "ntg.h"
 #include "ntg_device.cuh"
 #include "ntg_internal.h"
+#include "ntg_scan.cuh"
 
 namespace ntg {
 
@@ -792,6 +795,322 @@ __global__ void __launch_bounds__(128) k_bc4(const EncJob *__restrict__ jobs, in
 }
 
 // ---------------------------------------------------------------------------------------------
+// The squish fits of launches too small to fill the GPU one thread per block, two blocks per warp: a texel per lane
+// through the colour set, the sort, the alpha block and the indices, and all 32 lanes on one block's splits in turn
+// (ntg_scan.cuh). The same blocks as k_bc3<1> and k_bc1a. Bound by the FMA pipe in the scan (half of its time at 65,536
+// blocks) and by the exact evaluations: squish's point-by-point sums have a wide error bound, so about 90 splits of a
+// block with fractional weights, 16 with whole ones, may win.
+
+// Compress4's and Compress3's splits as cumulative ends, the one with every point in the last cluster first.
+static __device__ ScanOrders<512> g_splits4;
+static __device__ ScanOrders<96> g_splits3;
+
+// load_block's texel k.
+__device__ __forceinline__ uint32_t load_texel(const EncJob &J, int blk, int k) {
+    const int x = 4 * (blk % J.bw), y = 4 * (blk / J.bw);
+    const unsigned bw = min(J.w - x, 4), bh = min(J.h - y, 4);
+    const size_t n = (size_t)J.w * J.h, idx = (size_t)(y + (unsigned)(k >> 2) % bh) * J.w + x + (unsigned)(k & 3) % bw;
+    if (!J.bgra)
+        return quant_u8(J.rgba[idx + 2 * n]) | (quant_u8(J.rgba[idx + n]) << 8) | (quant_u8(J.rgba[idx]) << 16) |
+               (quant_u8(J.rgba[idx + 3 * n]) << 24);
+    const uint32_t p = J.bgra[idx];
+    if (!J.lut8) return p;
+    return (uint32_t)J.lut8[p & 255] | ((uint32_t)J.lut8[(p >> 8) & 255] << 8) | ((uint32_t)J.lut8[(p >> 16) & 255] << 16) |
+           ((uint32_t)J.lut8[256 + (p >> 24)] << 24);
+}
+
+// dxt5a_quick of the half's 16 values, one per lane.
+__device__ __forceinline__ AlphaBlk half_dxt5a_quick(const Half &H, int a) {
+    const unsigned mine = 0xffffu << H.shift;
+    const int hi = __reduce_max_sync(mine, a), lo = __reduce_min_sync(mine, a);
+    int a0 = (uint8_t)(hi - (hi - lo) / 34), a1 = (uint8_t)(lo + (hi - lo) / 34);
+    int k;
+    auto indices = [&]() {  // quick_alpha_indices: this lane's index, and the half's error
+        int pal[8];
+        alpha_palette(a0, a1, pal);
+        unsigned besterr = 256 * 256;
+        k = 8;
+#pragma unroll
+        for (int p = 0; p < 8; p++) {
+            const int d = pal[p] - a;
+            const unsigned e = (unsigned)(d * d);
+            if (e < besterr) { besterr = e; k = p; }
+        }
+        return __reduce_add_sync(mine, besterr);
+    };
+    unsigned best = indices();
+    int b0 = a0, b1 = a1, bk = k;
+    bool run = true;
+#pragma unroll 1
+    for (int it = 0; it < 8 && __any_sync(kAll, run); it++) {
+        // quick_alpha_refit: the sums in texel order
+        const float alpha = k < 2 ? 1.0f - k : (8.0f - k) / 7.0f, beta = 1 - alpha;
+        __syncwarp();
+        *reinterpret_cast<float4 *>(H.s->stage + 8 * H.hl) = make_float4(alpha * alpha, beta * beta, alpha * beta, alpha * a);
+        H.s->stage[8 * H.hl + 4] = beta * a;
+        __syncwarp();
+        const float sum = H.ordered(16);
+        const float a2 = H.get(sum, 0), b2 = H.get(sum, 1), ab = H.get(sum, 2), ax = H.get(sum, 3), bx = H.get(sum, 4);
+        const float f = 1.0f / (a2 * b2 - ab * ab);
+        const float fa = (ax * b2 - bx * ab) * f, fb = (bx * a2 - ax * ab) * f;
+        const unsigned v0 = (unsigned)ic_min(ic_max(fa, 0.0f), 255.0f), v1 = (unsigned)ic_min(ic_max(fb, 0.0f), 255.0f);
+        a0 = (int)max(v0, v1);
+        a1 = (int)min(v0, v1);
+        const unsigned e = indices();
+        if (e >= best) run = false;
+        if (run) {
+            run = !(a0 == b0 && a1 == b1);
+            best = e;
+            b0 = a0; b1 = a1; bk = k;
+        }
+    }
+    AlphaBlk b{b0, b1, 0};
+    const unsigned i0 = H.ballot(bk & 1), i1 = H.ballot(bk & 2), i2 = H.ballot(bk & 4);
+    uint64_t idx = 0;
+#pragma unroll
+    for (int i = 0; i < 16; i++) idx |= (uint64_t)(((i0 >> i) & 1) | (((i1 >> i) & 1) << 1) | (((i2 >> i) & 1) << 2)) << (3 * i);
+    b.idx = idx;
+    return b;
+}
+
+// The running sums of a block's clusters, as the searches accumulate them from each cluster's first point: entry (i, l) is the
+// sum of the l points from sorted point i on, l = 1..16 - i.
+__device__ __forceinline__ uint32_t run_at(uint32_t table, int i, int l) { return table + 16 * (uint32_t)((i * (33 - i) >> 1) + l - 1); }
+__device__ __forceinline__ float4 run_sum(uint32_t table, int i, int l) {
+    return l > 0 ? load_shared(run_at(table, i, l)) : make_float4(0, 0, 0, 0);
+}
+
+// A split's error as squish_search4 (four) or squish_search3 computes it; b0, b1, b2 are its cluster sizes.
+__device__ __forceinline__ float split_eval(bool four, uint32_t runs, int b0, int b1, int b2, f3 xsum, float wsum, f3 msq, f3 &a, f3 &b) {
+    const float4 s0 = run_sum(runs, 0, b0), s1 = run_sum(runs, b0, b1);
+    const f3 x0 = mk3(s0.x, s0.y, s0.z), x1 = mk3(s1.x, s1.y, s1.z);
+    const float w0 = s0.w, w1 = s1.w;
+    float a2, b2s, ab;
+    f3 ax;
+    if (four) {
+        const float4 s2 = run_sum(runs, b0 + b1, b2);
+        const f3 x2 = mk3(s2.x, s2.y, s2.z);
+        const float w2 = s2.w, wr = wsum - w0 - w1, w3 = wr - w2;
+        a2 = (w0 + w1 * (4.0f / 9.0f)) + w2 * (1.0f / 9.0f);
+        b2s = w3 + w2 * (4.0f / 9.0f) + w1 * (1.0f / 9.0f);
+        ab = (w1 + w2) * (2.0f / 9.0f);
+        ax = (x0 + (x1 * (2.0f / 3.0f))) + (x2 * (1.0f / 3.0f));
+    } else {
+        const float w2 = wsum - w0 - w1;
+        a2 = w0 + w1 * 0.25f;
+        b2s = w2 + w1 * 0.25f;
+        ab = w1 * 0.25f;
+        ax = x0 + x1 * 0.5f;
+    }
+    const float f = 1.0f / (a2 * b2s - ab * ab);
+    const f3 bx = xsum - ax;
+    a = snap565((ax * b2s) - (bx * ab), f);
+    b = snap565((bx * a2) - (ax * ab), f);
+    const f3 t = (((a * b) * ab) - (a * ax)) - (b * bx);
+    const f3 e1 = (((a * a) * a2) + ((b * b) * b2s)) + (t * 2.0f);
+    return dot(e1, msq);
+}
+
+// The splits of the warp's block b by all lanes: winners (key: cluster sizes, 5 bits each), their errors and end points
+// to the half's scratch. FOUR, THREE: which searches run.
+__device__ __forceinline__ void warp_splits(WarpScratch &w, int b, bool four, bool three, bool unit) {
+    const int lane = threadIdx.x & 31;
+    HalfScratch &h = w.half[b];
+    const ScanBlock &blk = h.block[0];
+    const int n = blk.n;
+    const float4 sum = h.sum;
+    scan_centre(w.scan, blk, h.table[0], true);
+    uint32_t bits4 = 0, bits3 = 0;
+    if (four) bits4 = scan_bits(w.scan, blk, g_splits4, n ? (c_tab.four_total[n - 1] + 64) >> 6 : 1, 0, 3.0f, unit);
+    if (three) bits3 = scan_bits(w.scan, blk, g_splits3, n ? (c_tab.three_total[n - 1] + 64) >> 6 : 1, 16, 2.0f, unit);
+    __syncwarp();
+    uint16_t *const list = reinterpret_cast<uint16_t *>(w.scan.e);
+    int count = 0;
+    scan_list(list, count, bits4, 0x8000);
+    scan_list(list, count, bits3, 0);
+    // the running sums go behind the list, a lane per first point
+    constexpr int kRuns = 2304;
+    static_assert(kRuns >= 2 * 1120 && kRuns + 136 * 16 <= (int)sizeof w.scan.e, "list and running sums share the errors' place");
+    const uint32_t runs = shared_address(w.scan.e) + kRuns;
+    if (lane < n) {
+        const uint32_t wp = shared_address(h.table[1]);
+        float4 acc = make_float4(0, 0, 0, 0);
+        for (int l = 1; l <= n - lane; l++) {
+            const float4 q = load_shared(wp + 16 * (lane + l - 1));
+            acc = make_float4(acc.x + q.x, acc.y + q.y, acc.z + q.z, acc.w + q.w);
+            const uint32_t at = run_at(runs, lane, l);
+            store_shared(at, acc.x, acc.y);
+            store_shared(at + 8, acc.z, acc.w);
+        }
+    }
+    __syncwarp();
+    const f3 msq = mk3(blk.metric[0], blk.metric[1], blk.metric[2]);
+    FitBest best4, best3;
+#pragma unroll 1
+    for (int i = lane; i < count; i += 32) {
+        const int it = list[i], o = it & 0x7fff;
+        const bool is4 = (it & 0x8000) != 0;
+        const uint32_t ends = is4 ? scan_ends(g_splits4, o) : scan_ends(g_splits3, o);
+        // ends above the count are the count's: such an ordering repeats an earlier one
+        const int c0 = min((int)(ends & 1023) >> 4, n), c2 = min((int)(ends >> 24), n), c1 = is4 ? min((int)((ends >> 10) & 1023) >> 4, n) : c2;
+        f3 ea, eb;
+        const float e = split_eval(is4, runs, c0, c1 - c0, c2 - c1, mk3(sum.x, sum.y, sum.z), sum.w, msq, ea, eb);
+        const int key = (c0 << 10) | ((c1 - c0) << 5) | (c2 - c1);
+        if (is4) best4.take(e, key, ea, eb);
+        else best3.take(e, key, ea, eb);
+    }
+    const int o4 = best4.finish(h.ends), o3 = best3.finish(h.ends + 6);
+    const uint32_t e4 = __reduce_min_sync(kAll, best4.key), e3 = __reduce_min_sync(kAll, best3.key);
+    if (lane == 0) { h.order[0] = o4; h.order[1] = o3; h.error[0] = e4; h.error[1] = e3; }
+    __syncwarp();
+}
+
+// DXT1: k_bc1a's blocks, else k_bc3<1>'s.
+template <bool DXT1>
+__global__ void __launch_bounds__(32 * kFitWarps, 5) k_squish(const EncJob *__restrict__ jobs, int njobs, long long nblocks) {
+    __shared__ WarpScratch scratch[kFitWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, hl = lane & 15;
+    WarpScratch &w = scratch[warp];
+    const Half H{hl, lane & 16, &w.half[lane >> 4]};
+    const long long first = 2 * ((long long)blockIdx.x * kFitWarps + warp);
+    if (first >= nblocks) return;
+    const bool live = first + (lane >> 4) < nblocks;  // the last warp's second half may have no block
+    const long long gblk = live ? first + (lane >> 4) : first;
+    const EncJob &J = jobs[find_job(jobs, njobs, gblk)];
+    const int blk = (int)(gblk - J.first_block);
+    uint8_t *const dst = J.out + (DXT1 ? 8 : 16) * (size_t)blk;
+    const f3 metric = mk3(J.cw[0], J.cw[1], J.cw[2]), msq = metric * metric;
+    const bool unit = __all_sync(kAll, msq.x == 1.0f && msq.y == 1.0f && msq.z == 1.0f) != 0;
+    const uint32_t px = load_texel(J, blk, hl), rgb = px & 0xFFFFFF;
+    if (!DXT1) {
+        const AlphaBlk ab = half_dxt5a_quick(H, (int)(px >> 24));
+        if (live && hl == 0) pack_alpha(ab, dst);
+    }
+    const bool clear = DXT1 && (px >> 24) == 0;
+    const unsigned transparent = H.ballot(clear);
+    const uint32_t rgb0 = __shfl_sync(kAll, rgb, 0, 16);
+    const bool single = H.ballot(rgb == rgb0) == 0xffffu;
+    if (single && live && hl == 0)
+        *reinterpret_cast<uint2 *>(dst + (DXT1 ? 0 : 8)) =
+            DXT1 ? dxt1a_single_color((rgb0 >> 16) & 255, (rgb0 >> 8) & 255, rgb0 & 255, spread_bits(transparent) * 3)
+                 : dxt1_single_color((rgb0 >> 16) & 255, (rgb0 >> 8) & 255, rgb0 & 255);
+    const bool fit = live && !single;
+    if (!__any_sync(kAll, fit)) return;
+
+    // the minimal set in texel slots (squish_points): a texel's slot is the first with its RGB; the weights of a slot,
+    // multiples of 1 / 256, add up exactly in any order
+    const uint32_t half_bit = (uint32_t)(lane & 16) << 20;
+    const unsigned same = (__match_any_sync(kAll, clear ? 0x80000000u | half_bit | (uint32_t)hl : half_bit | rgb) >> H.shift) & 0xffffu;
+    const int slot = __ffs(same) - 1;
+    const bool point = slot == hl && !clear;
+    const int own = J.alpha_mode == 1 ? (int)(px >> 24) + 1 : 256;
+    int all = 0;
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+        const int v = __shfl_sync(kAll, own, j, 16);
+        if ((same >> j) & 1) all += v;
+    }
+    const float W = (float)(point ? all : own) * (1.0f / 256.0f);
+    const f3 X = mk3((float)((px >> 16) & 255) / 255.0f, (float)((px >> 8) & 255) / 255.0f, (float)(px & 255) / 255.0f);
+    const unsigned points = H.ballot(point);
+    const int n = __popc(points);
+    float *const st = H.s->stage;
+    const f3 p = X * W;
+    __syncwarp();
+    *reinterpret_cast<float4 *>(st + 8 * hl) = make_float4(p.x, p.y, p.z, W);
+    __syncwarp();
+    const float cs = H.ordered_of(points);
+    const f3 cen = mk3(H.get(cs, 0), H.get(cs, 1), H.get(cs, 2)) * (1.0f / H.get(cs, 3));
+    const f3 a = (X - cen) * metric, b = a * W;
+    __syncwarp();
+    *reinterpret_cast<float4 *>(st + 8 * hl) = make_float4(a.x * b.x, a.x * b.y, a.x * b.z, a.y * b.y);
+    *reinterpret_cast<float2 *>(st + 8 * hl + 4) = make_float2(a.y * b.z, a.z * b.z);
+    __syncwarp();
+    const float ms = H.ordered_of(points);
+    const float m0 = H.get(ms, 0), m1 = H.get(ms, 1), m2 = H.get(ms, 2), m3 = H.get(ms, 3), m4 = H.get(ms, 4), m5 = H.get(ms, 5);
+    const f3 r0 = mk3(m0, m1, m2), r1 = mk3(m1, m3, m4), r2 = mk3(m2, m4, m5);
+    const float l0 = dot(r0, r0), l1 = dot(r1, r1), l2 = dot(r2, r2);
+    f3 v = (l0 > l1 && l0 > l2) ? r0 : (l1 > l2 ? r1 : r2);
+#pragma unroll 1
+    for (int it = 0; it < 8; it++) {
+        const float x = v.x * m0 + v.y * m1 + v.z * m2;
+        const float y = v.x * m1 + v.y * m3 + v.z * m4;
+        const float z = v.x * m2 + v.y * m4 + v.z * m5;
+        const float norm = sq_max(sq_max(x, y), z);
+        const float iv = 1.0f / norm;
+        if (norm == 0.0f) { v = mk3(0, 0, 0); break; }
+        v = mk3(x * iv, y * iv, z * iv);
+    }
+    __syncwarp();
+    // sorted along the axis, slots without a point last
+    const int rank = half_rank(H, point ? dot(X, v) : __int_as_float(0x7f800000), 16);
+    H.s->table[1][rank] = make_float4(p.x, p.y, p.z, W);
+    __syncwarp();
+    // the sums in sorted order (xsum, wsum), then the table of centred prefix sums for the scan
+    const float *const q = reinterpret_cast<const float *>(H.s->table[1]) + (hl & 3);
+    float acc = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; i++)
+        if (i < n) acc += q[4 * i];
+    const f3 sum = mk3(H.get(acc, 0), H.get(acc, 1), H.get(acc, 2));
+    const float wsum = H.get(acc, 3);
+    const bool whole = H.ballot(point && W != floorf(W)) == 0;
+    float big = point ? max3_abs(X.x, X.y, X.z) : 0.0f;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(kAll, big, o));
+    // the scatter without the metric, for the bound (a zero weight: the most there can be)
+    const float scatter = (msq.x > 0 ? m0 / msq.x : wsum) + (msq.y > 0 ? m3 / msq.y : wsum) + (msq.z > 0 ? m5 / msq.z : wsum);
+    if (hl == 0) {
+        scan_begin(H.s->block[0], n, sum, wsum, big, scatter, whole, msq, whole ? 101.0f : 156.0f, whole ? 90.0f : 153.0f, whole ? 0.0f : 8.0f);
+        H.s->sum = make_float4(sum.x, sum.y, sum.z, wsum);
+    }
+    __syncwarp();
+    if (hl < 4) {
+        const float mu = hl < 3 ? H.s->block[0].mu[hl] : 0.0f;
+        const float *const qw = reinterpret_cast<const float *>(H.s->table[1]) + 3;
+        float *const t = reinterpret_cast<float *>(H.s->table[0]) + hl;
+        float c = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            t[4 * i] = c;
+            if (i < n) c += __fmaf_rn(-qw[4 * i], mu, q[4 * i]);
+        }
+        t[64] = c;
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int i = 0; i < 2; i++) {
+        const bool run = __shfl_sync(kAll, (int)fit, 16 * i) != 0, four = !DXT1 || __shfl_sync(kAll, transparent, 16 * i) == 0;
+        if (run) warp_splits(w, i, four, DXT1, unit);
+    }
+    // the blocks: WriteColourBlock4 / 3 over the texels' positions in the sorted set
+    const int pos = __shfl_sync(kAll, rank, slot, 16);
+    const float *const ends = H.s->ends;
+    auto colour = [&](bool four) {
+        const int key = fit ? H.s->order[four ? 0 : 1] : -1;
+        const int b0 = key >> 10, b1 = b0 + ((key >> 5) & 31), b2 = b1 + (key & 31);
+        const unsigned code = clear ? 3u : (pos < b0 ? 0u : (pos < b1 ? 2u : (four && pos < b2 ? 3u : 1u)));
+        uint32_t idx = (spread_bits(H.ballot(code & 2)) << 1) | spread_bits(H.ballot(code & 1));
+        const float *const e = ends + (four ? 0 : 6);
+        int ea = squish_565(mk3(e[0], e[1], e[2])), eb = squish_565(mk3(e[3], e[4], e[5]));
+        if (four) {
+            if (ea < eb) { const int t = ea; ea = eb; eb = t; idx ^= 0x55555555u; }
+            else if (ea == eb) idx = 0;
+        } else if (ea > eb) {
+            const int t = ea; ea = eb; eb = t;
+            idx ^= (~idx >> 1) & 0x55555555u;
+        }
+        return key < 0 ? make_uint2(0, 0) : make_uint2((uint32_t)ea | ((uint32_t)eb << 16), idx);
+    };
+    uint2 out = colour(!DXT1);
+    if (DXT1) {  // a later mode replaces the block only with a strictly smaller error
+        const uint2 four = colour(true);
+        if (transparent == 0 && H.s->order[0] >= 0 && (H.s->order[1] < 0 || H.s->error[0] < H.s->error[1])) out = four;
+    }
+    if (fit && hl == 0) *reinterpret_cast<uint2 *>(dst + (DXT1 ? 0 : 8)) = out;
+}
+
+// ---------------------------------------------------------------------------------------------
 // Learned endpoint proposal for the BC3 colour block (no counterpart in the reference). The network
 // (the same MLP as BC1's, trained on BC3 blocks) reads the block's 16 texels as the encoder sees them
 // (after ColorBlock's quantiser, RGB / 255) in order of their projection on the squish principal axis
@@ -1112,8 +1431,22 @@ int launch_bc3_list(const EncJob *d_jobs, int njobs, const long long *list, cons
     return launch_status();
 }
 
+// Launches of at most this many blocks take k_squish. One thread per block keeps 97,280 in flight (152 SMs x 5 CTAs of
+// 128) and takes at least 178 us however few there are; measured with the alpha field (BC3), one level, one thread per
+// block against k_squish: 64x64 179 and 34 us, 256x256 178 and 41, 512x512 186 and 104, 700x700 (30,625 blocks) 236 and
+// 180, 1024x1024 (65,536) 382 and 365, 2048x2048 1,185 and 1,500; BC1a: 256x256 194 and 45, 1024x1024 392 and 337.
+constexpr long long kSquishWarpBlocks = 68096;
+
+template <bool DXT1>
+static int launch_squish(const EncJob *d_jobs, int njobs, long long nblocks, cudaStream_t stream) {
+    const long long per = 2 * kFitWarps;
+    k_squish<DXT1><<<(unsigned)((nblocks + per - 1) / per), 32 * kFitWarps, 0, stream>>>(d_jobs, njobs, nblocks);
+    return launch_status();
+}
+
 int launch_bc3(const EncJob *d_jobs, int njobs, long long nblocks, int quality, int threads, cudaStream_t stream) {
     if (nblocks == 0) return 0;
+    if ((quality == 1 || quality == 2) && nblocks <= kSquishWarpBlocks) return launch_squish<false>(d_jobs, njobs, nblocks, stream);
     const int T = threads == 32 || threads == 64 ? threads : 128;  // blocks per CTA
     const size_t sm = (size_t)T * 17 * sizeof(float4);
     const unsigned grid = (unsigned)((nblocks + T - 1) / T);
@@ -1137,6 +1470,7 @@ int launch_bc5(const EncJob *d_jobs, int njobs, long long nblocks, int quality, 
 int launch_bc1a(const EncJob *d_jobs, int njobs, long long nblocks, int quality, int threads, cudaStream_t stream) {
     if (nblocks == 0) return 0;
     if (quality == 0) return NTG_ERROR_UNSUPPORTED_FEATURE;  // see ntg_encode's check
+    if (nblocks <= kSquishWarpBlocks) return launch_squish<true>(d_jobs, njobs, nblocks, stream);
     const int T = threads == 32 || threads == 64 ? threads : 128;  // blocks per CTA
     const size_t sm = (size_t)T * 17 * sizeof(float4);
     k_bc1a<<<(unsigned)((nblocks + T - 1) / T), T, sm, stream>>>(d_jobs, njobs, nblocks);
@@ -1152,6 +1486,14 @@ int launch_bc4(const EncJob *d_jobs, int njobs, long long nblocks, int quality, 
     return launch_status();
 }
 
-NTG_DEFINE_TABLE_UPLOAD(upload_tables_bc3)
+int upload_tables_bc3(const HostTables &t) {
+    const std::unique_ptr<ScanOrders<512>> o4(new ScanOrders<512>);
+    ScanOrders<96> o3;
+    scan_orders<3, 512, true>(t.four, t.four_total[15], *o4);
+    scan_orders<2, 96, true>(t.three, t.three_total[15], o3);
+    return cudaMemcpyToSymbol(c_tab, &t, sizeof t) == cudaSuccess && cudaMemcpyToSymbol(g_splits4, o4.get(), sizeof *o4) == cudaSuccess &&
+                   cudaMemcpyToSymbol(g_splits3, &o3, sizeof o3) == cudaSuccess
+               ? 0 : 3;
+}
 
 }  // namespace ntg

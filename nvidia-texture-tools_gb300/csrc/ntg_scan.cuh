@@ -17,11 +17,11 @@
 // The error bound. u = 2^-24, M the largest |component|, T = sum w |x - mu|^2 (metric included). For an
 // ordering with a scanned error below 0, |fit|^2 <= 4 T, which bounds |d| and |m| by multiples of sqrt(T).
 //   - The reference's own roundings: sums of W-weighted terms of size at most 1 (end points are in [0, 1])
-//     and M: u W (13 + 46 M) per unit of metric weight with icbc's prefix sums; squish adds points one by
-//     one, up to 15 roundings a sum: u W (13 + 150 M).
+//     and M: u W (13 + 46 M) per unit of metric weight with icbc's prefix sums; squish adds a cluster's points one by
+//     one: u W (13 + 101 M) when the weights are whole (partial sums grow evenly), u W (13 + 156 M) when not.
 //   - The scan's: relative to T, 2,500 u T. With whole weights D is exact; with fractional ones it loses up to
-//     60 u W^2 to cancellation: the end points' bound grows by 200 u W^2 / D, and the error by 60 u W (|d| is at
-//     most 1 per channel).
+//     60 u W^2 to cancellation (8 u W^2 with weights that are multiples of 1 / 256, whose sums are exact): the end
+//     points' bound grows by three times that over D, and the error by as much over W (|d| is at most 1 per channel).
 //   - Snapping: both arithmetics reach the least-squares end points within eta = c u W^2 / D + 24 u. Where an end
 //     point lies closer than that to the middle between two grid points they may snap apart: such an
 //     ordering (about one of 120) always counts among the possible winners, and never as the lowest scanned one.
@@ -73,19 +73,20 @@ struct ScanBlock {
     float metric[3];
 };
 
-// `ref_m`: the reference's rounding bound per unit of M (46 icbc, 150 squish); `eta_m`: the same for the end
-// points (47 icbc, 153 squish); `whole`: the weights are whole numbers.
+// `ref_m`: the reference's rounding bound per unit of M (46 icbc, 101 or 156 squish); `eta_m`: the same for the end
+// points (47 icbc, 90 or 153 squish); `err_d`: the bound of D's rounding in u W^2; `whole`: the weights are whole
+// numbers.
 __device__ __forceinline__ void scan_begin(ScanBlock &s, int n, f3 sum, float wsum, float maxabs, float scatter, bool whole,
-                                           f3 metric, float ref_m, float eta_m) {
+                                           f3 metric, float ref_m, float eta_m, float err_d) {
     const float u = 5.9604645e-8f;
     s.mu[0] = sum.x / wsum; s.mu[1] = sum.y / wsum; s.mu[2] = sum.z / wsum;
     s.W = wsum;
     const float mx = fmaxf(fmaxf(metric.x, metric.y), metric.z), mn = fminf(fminf(metric.x, metric.y), metric.z);
     const bool fits = maxabs <= 2.0f && mn >= 0.0f && mx <= 4.0f && scatter <= 256.0f && wsum > 0.0f && wsum <= 16.5f;
-    const float per = wsum * (13.0f + ref_m * maxabs + (whole ? 0.0f : 60.0f));
+    const float per = wsum * (13.0f + ref_m * maxabs + err_d);
     s.slack = 2.0f * u * (per * (metric.x + metric.y + metric.z) + 2500.0f * scatter * mx);
     // an infinite bound makes every ordering a possible winner
-    s.eta = fits ? 63.0f * u * (eta_m * maxabs + 20.0f + 24.0f * sqrtf(scatter / wsum) + (whole ? 0.0f : 200.0f)) * wsum * wsum
+    s.eta = fits ? 63.0f * u * (eta_m * maxabs + 20.0f + 24.0f * sqrtf(scatter / wsum) + 3.0f * err_d) * wsum * wsum
                  : __int_as_float(0x7f800000);
     s.n = n;
     s.flat = n == 16 && whole && wsum == 16.0f;
@@ -102,11 +103,13 @@ struct ScanOrders {
     struct __align__(16) Sums { float nA[2], cD[2]; } s[PAIRS];
 };
 
-// Fills the pairs from an icbc table (bytes: cumulative ends), repeating the first ordering at the end. Host.
-template <int K, int PAIRS>
+// Fills the pairs from an icbc table (bytes: cumulative ends), repeating the first ordering at the end; EMPTY puts the
+// ordering with every end 0, which squish tries and icbc leaves out, first. Host.
+template <int K, int PAIRS, bool EMPTY = false>
 inline void scan_orders(const uint32_t *table, int total, ScanOrders<PAIRS> &out) {
     for (int i = 0; i < 2 * PAIRS; i++) {
-        const uint32_t o = table[i < total ? i : 0];
+        const int at = EMPTY ? i - 1 : i;
+        const uint32_t o = at < 0 ? 0 : table[at < total ? at : 0];
         const int c0 = o & 255, c1 = K == 3 ? (o >> 8) & 255 : 0, c2 = (o >> (K == 3 ? 16 : 8)) & 255;
         const int A = c0 + c1 + c2, U = K == 3 ? 5 * c0 + 3 * c1 + c2 : 3 * c0 + c2, D = 16 * U - A * A;
         const int p = 32 * (i / 64) + i % 32, h = (i / 32) & 1;
@@ -137,15 +140,14 @@ struct ScanScratch {
                            // possible winners' list
 };
 
-// Centres a block's table for scan_rows.
-__device__ __forceinline__ void scan_centre(ScanScratch &w, const ScanBlock &blk, const float4 *table) {
+// A block's table for scan_rows, centred here unless it is already.
+__device__ __forceinline__ void scan_centre(ScanScratch &w, const ScanBlock &blk, const float4 *table, bool centred = false) {
     const int lane = threadIdx.x & 31;
     __syncwarp();
     if (lane < 18) {
-        const float4 p = table[lane];
-        w.centred[lane] = lane == 17 ? make_float4(0, 0, 0, 0)
-                                     : make_float4(__fmaf_rn(-p.w, blk.mu[0], p.x), __fmaf_rn(-p.w, blk.mu[1], p.y),
-                                                   __fmaf_rn(-p.w, blk.mu[2], p.z), p.w);
+        float4 p = table[lane];
+        if (!centred) p = make_float4(__fmaf_rn(-p.w, blk.mu[0], p.x), __fmaf_rn(-p.w, blk.mu[1], p.y), __fmaf_rn(-p.w, blk.mu[2], p.z), p.w);
+        w.centred[lane] = lane == 17 ? make_float4(0, 0, 0, 0) : p;
     }
     __syncwarp();
 }
@@ -281,8 +283,8 @@ struct FitBest {
         const uint32_t k = float_order(e);
         if (e < FLT_MAX && (k < key || (k == key && o < order))) { key = k; order = o; a = ea; b = eb; }
     }
-    // The warp's best writes its end points to out[0..5]; zeros when there is none.
-    __device__ __forceinline__ void finish(float *out) const {
+    // The warp's best writes its end points to out[0..5]; zeros when there is none. Returns its ordering, -1 for none.
+    __device__ __forceinline__ int finish(float *out) const {
         const uint32_t least = __reduce_min_sync(0xffffffffu, key);
         const int first = __reduce_min_sync(0xffffffffu, key == least ? order : 0x7fffffff);
         if (least == 0xffffffffu) {
@@ -290,7 +292,96 @@ struct FitBest {
         } else if (key == least && order == first) {
             out[0] = a.x; out[1] = a.y; out[2] = a.z; out[3] = b.x; out[4] = b.y; out[5] = b.z;
         }
+        return least == 0xffffffffu ? -1 : first;
     }
 };
+
+// ---- two blocks per warp: lanes 0-15 one block's texels, lanes 16-31 the next one's ----
+
+constexpr unsigned kAll = 0xffffffffu;
+constexpr int kFitWarps = 4;  // warps per CTA, each on its own
+
+// One half's scratch in shared memory.
+struct HalfScratch {
+    float stage[16 * 8];  // terms per texel or colour
+    float pad[8];         // the two halves' stages lie on different banks
+    float4 table[2][18];  // the ZERO summed-area tables (17 entries) of the two fits; squish: the one table, the points
+    float4 sum;           // squish: the sum of the points
+    ScanBlock block[2];   // and their scans' constants
+    float ends[12];       // the fits' end points
+    int order[2];         // the fits' winners (-1: none) and
+    uint32_t error[2];    // their errors (float_order), where the caller wants them
+};
+struct WarpScratch {
+    ScanScratch scan;
+    HalfScratch half[2];
+};
+
+struct Half {
+    int hl;         // lane in the half: texel or colour index
+    int shift;      // first lane of the half
+    HalfScratch *s;
+    __device__ __forceinline__ float get(float v, int src) const { return __shfl_sync(kAll, v, src, 16); }
+    __device__ __forceinline__ unsigned ballot(bool p) const { return (__ballot_sync(kAll, p) >> shift) & 0xffffu; }
+    // Sum over i < n, in order, of the terms stage[8 i + c]; lane c of the half returns it.
+    __device__ __forceinline__ float ordered(int n) const {
+        float acc = 0.0f;
+        const float *p = s->stage + (hl & 7);
+#pragma unroll
+        for (int i = 0; i < 16; i++)
+            if (i < n) acc += p[8 * i];
+        return acc;
+    }
+    // The same over the set bits i of `mask`.
+    __device__ __forceinline__ float ordered_of(unsigned mask) const {
+        float acc = 0.0f;
+        const float *p = s->stage + (hl & 7);
+#pragma unroll
+        for (int i = 0; i < 16; i++)
+            if ((mask >> i) & 1) acc += p[8 * i];
+        return acc;
+    }
+};
+
+// A lane's position among its half's first n keys in a stable insertion sort's order: its rank, unless a key is NaN (which
+// the sort leaves where it meets it).
+__device__ __forceinline__ int half_rank(const Half &H, float d, int n) {
+    float *const st = H.s->stage;
+    int rank = 0;
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+        const float e = H.get(d, j);
+        rank += j < n && (e < d || (e == d && j < H.hl));
+    }
+    const bool odd = H.ballot(H.hl < n && d != d) != 0;
+    __syncwarp();
+    if (__any_sync(kAll, odd)) {
+        float *const key = st;
+        int *const ord = reinterpret_cast<int *>(st + 16), *const pos = reinterpret_cast<int *>(st + 32);
+        key[H.hl] = d;
+        __syncwarp();
+        if (H.hl == 0) {
+            for (int i = 0; i < n; i++) ord[i] = i;
+            for (int i = 1; i < n; i++)
+                for (int j = i; j > 0 && key[j] < key[j - 1]; j--) {
+                    const float t = key[j]; key[j] = key[j - 1]; key[j - 1] = t;
+                    const int o = ord[j]; ord[j] = ord[j - 1]; ord[j - 1] = o;
+                }
+            for (int i = 0; i < n; i++) pos[ord[i]] = i;
+        }
+        __syncwarp();
+        if (odd && H.hl < n) rank = pos[H.hl];
+        __syncwarp();
+    }
+    return rank;
+}
+
+// Bit i of m to bit 2 i.
+__device__ __forceinline__ uint32_t spread_bits(uint32_t m) {
+    m = (m | (m << 8)) & 0x00ff00ffu;
+    m = (m | (m << 4)) & 0x0f0f0f0fu;
+    m = (m | (m << 2)) & 0x33333333u;
+    return (m | (m << 1)) & 0x55555555u;
+}
 
 }  // namespace ntg

@@ -34,6 +34,8 @@ def contents(kind, w, h, seed):
         rgb[rng.random(rgb.shape) < 0.02] = np.inf
     elif kind == "ramp":      # noise around a gradient, as smooth textures have it
         rgb = (0.3 + 0.4 * (np.arange(w)[None, None, :] / w) + rng.uniform(-8, 8, (3, h, w)) / 255.0).astype(np.float32)
+    if kind != "weights":
+        a[rng.random((h, w)) < 0.1] = 0
     return np.concatenate([rgb.reshape(-1), a.reshape(-1)]).astype(np.float32)
 
 
@@ -41,9 +43,10 @@ KINDS = ["noise", "flat", "faint", "grid", "dark", "weights", "wide", "odd", "ra
 
 
 @pytest.mark.parametrize("kind", KINDS)
-@pytest.mark.parametrize("fmt", [ntg.FORMAT_BC1])
+@pytest.mark.parametrize("fmt", [ntg.FORMAT_BC1, ntg.FORMAT_BC1A, ntg.FORMAT_BC3])
 def test_fits_match_oracle(ctx, oracle, kind, fmt):
-    image = {ntg.FORMAT_BC1: oracle.bc1_image}[fmt]
+    image = {ntg.FORMAT_BC1: oracle.bc1_image, ntg.FORMAT_BC3: oracle.bc3_image,
+             ntg.FORMAT_BC1A: lambda i, w, h, alpha, q, **kw: oracle.bc1a_image(i, w, h, alpha, **kw)}[fmt]
     for i, (w, h) in enumerate([(4, 4), (8, 4), (12, 4), (28, 4), (36, 4), (61, 35), (128, 96)]):
         img = contents(kind, w, h, 100 * i + len(kind))
         for quality, alpha, cw in [(1, 0, (1, 1, 1)), (1, 1, (1, 1, 1)), (2, 1, (0.6, 1.0, 0.4))]:
