@@ -929,8 +929,8 @@ __device__ __forceinline__ void warp_splits(WarpScratch &w, int b, bool four, bo
     scan_list(list, count, bits4, 0x8000);
     scan_list(list, count, bits3, 0);
     // the running sums go behind the list, a lane per first point
-    constexpr int kRuns = 2304;
-    static_assert(kRuns >= 2 * 1120 && kRuns + 136 * 16 <= (int)sizeof w.scan.e, "list and running sums share the errors' place");
+    constexpr int kRuns = 2 * 64 * (16 + 3);  // the list may hold every ordering of all rows, the last ones' repeats too
+    static_assert(kRuns % 16 == 0 && kRuns + 136 * 16 <= (int)sizeof w.scan.e, "list and running sums share the errors' place");
     const uint32_t runs = shared_address(w.scan.e) + kRuns;
     if (lane < n) {
         const uint32_t wp = shared_address(h.table[1]);

@@ -55,3 +55,12 @@ def test_fits_match_oracle(ctx, oracle, kind, fmt):
             got = ctx.encode(fmt, torch.from_numpy(img).cuda(), w, h, quality=quality, alpha_mode=alpha, cw=cw)
             ref = image(img, w, h, alpha, quality, cw=cw, threads=8)
             assert np.array_equal(got.cpu().numpy(), ref), (kind, w, h, quality, alpha)
+
+
+def test_bc1a_every_split_a_candidate(ctx, oracle):
+    """Nearly flat blocks with unequal weights: every split of both fits, and the repeats that fill the tables' last rows,
+    are possible winners, as many as the list of them can hold."""
+    w, h = 4, 4 * 6083
+    img = contents("faint", w, h, 6088)
+    got = ctx.encode(ntg.FORMAT_BC1A, torch.from_numpy(img).cuda(), w, h, quality=1, alpha_mode=1)
+    assert np.array_equal(got.cpu().numpy(), oracle.bc1a_image(img, w, h, 1, threads=8))
