@@ -1089,7 +1089,8 @@ __global__ void __launch_bounds__(32 * kFitWarps, 5) k_squish(const EncJob *__re
     auto colour = [&](bool four) {
         const int key = fit ? H.s->order[four ? 0 : 1] : -1;
         const int b0 = key >> 10, b1 = b0 + ((key >> 5) & 31), b2 = b1 + (key & 31);
-        const unsigned code = clear ? 3u : (pos < b0 ? 0u : (pos < b1 ? 2u : (four && pos < b2 ? 3u : 1u)));
+        // an axis that is NaN (tiny weights) leaves points behind the first n places, which stay at index 0
+        const unsigned code = clear ? 3u : (pos < b0 || pos >= n ? 0u : (pos < b1 ? 2u : (four && pos < b2 ? 3u : 1u)));
         uint32_t idx = (spread_bits(H.ballot(code & 2)) << 1) | spread_bits(H.ballot(code & 1));
         const float *const e = ends + (four ? 0 : 6);
         int ea = squish_565(mk3(e[0], e[1], e[2])), eb = squish_565(mk3(e[3], e[4], e[5]));

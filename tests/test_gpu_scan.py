@@ -64,3 +64,16 @@ def test_bc1a_every_split_a_candidate(ctx, oracle):
     img = contents("faint", w, h, 6088)
     got = ctx.encode(ntg.FORMAT_BC1A, torch.from_numpy(img).cuda(), w, h, quality=1, alpha_mode=1)
     assert np.array_equal(got.cpu().numpy(), oracle.bc1a_image(img, w, h, 1, threads=8))
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("fmt", [ntg.FORMAT_BC1A, ntg.FORMAT_BC3])
+def test_squish_launch_sizes_agree(ctx, fmt, kind):
+    """The two kernels of the squish fits, which share the work by launch size (68,096 blocks), over the same blocks;
+    among them ("weights") single points of so tiny a weight that their axis is NaN."""
+    w, h = 4, 4 * 60000
+    img = torch.from_numpy(contents(kind, w, h, 3007)).cuda().reshape(4, h, w)
+    small = ctx.encode(fmt, img, w, h, quality=1, alpha_mode=1)
+    img = torch.cat([img, img[:, :4 * 8097]], 1).contiguous()
+    large = ctx.encode(fmt, img, w, 4 * 68097, quality=1, alpha_mode=1)
+    assert torch.equal(large[:small.numel()], small)
