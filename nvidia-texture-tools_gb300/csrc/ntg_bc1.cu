@@ -955,17 +955,18 @@ __device__ __forceinline__ float4 gather_texel(const EncJob &J, int blk, int k) 
 template <int LEVEL>
 __global__ void __launch_bounds__(32 * kFitWarps, NTG_BC1_MIN_CTAS) k_bc1(const EncJob *__restrict__ jobs, int njobs, long long nblocks,
                                                                          const long long *__restrict__ list,
-                                                                         const unsigned long long *__restrict__ count) {
+                                                                         const unsigned long long *__restrict__ count,
+                                                                         int per_warp) {
     __shared__ WarpScratch scratch[kFitWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     WarpScratch &w = scratch[warp];
     const Half H{lane & 15, lane & 16, &w.half[lane >> 4]};
     // `list`: a subset of the jobs' blocks (the learned path's fallbacks), *count long
     const long long total = list ? min(nblocks, (long long)*count) : nblocks;
-    const long long first = 2 * ((long long)blockIdx.x * kFitWarps + warp);
+    const long long first = per_warp * ((long long)blockIdx.x * kFitWarps + warp);
     if (first >= total) return;
     long long gblk = first + (lane >> 4);
-    const bool live = gblk < total;  // the last warp's second half may have no block
+    const bool live = (lane >> 4) < per_warp && gblk < total;  // a half without a block follows the other's
     if (!live) gblk = first;
     if (list) gblk = list[gblk];
     const EncJob &J = jobs[find_job(jobs, njobs, gblk)];
@@ -1514,8 +1515,8 @@ static size_t bc1_work_smem(int T) { return (size_t)T * (16 * sizeof(float4) + 1
 template <int LEVEL>
 static int launch_bc1_fit(const EncJob *d_jobs, int njobs, long long nblocks, const long long *list, const unsigned long long *count,
                           cudaStream_t stream) {
-    const long long per = 2 * kFitWarps;
-    k_bc1<LEVEL><<<(unsigned)((nblocks + per - 1) / per), 32 * kFitWarps, 0, stream>>>(d_jobs, njobs, nblocks, list, count);
+    const int per_warp = fit_blocks_per_warp(nblocks), per = per_warp * kFitWarps;
+    k_bc1<LEVEL><<<(unsigned)((nblocks + per - 1) / per), 32 * kFitWarps, 0, stream>>>(d_jobs, njobs, nblocks, list, count, per_warp);
     return launch_status();
 }
 

@@ -967,14 +967,15 @@ __device__ __forceinline__ void warp_splits(WarpScratch &w, int b, bool four, bo
 
 // DXT1: k_bc1a's blocks, else k_bc3<1>'s.
 template <bool DXT1>
-__global__ void __launch_bounds__(32 * kFitWarps, 5) k_squish(const EncJob *__restrict__ jobs, int njobs, long long nblocks) {
+__global__ void __launch_bounds__(32 * kFitWarps, 5) k_squish(const EncJob *__restrict__ jobs, int njobs, long long nblocks,
+                                                              int per_warp) {
     __shared__ WarpScratch scratch[kFitWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, hl = lane & 15;
     WarpScratch &w = scratch[warp];
     const Half H{hl, lane & 16, &w.half[lane >> 4]};
-    const long long first = 2 * ((long long)blockIdx.x * kFitWarps + warp);
+    const long long first = per_warp * ((long long)blockIdx.x * kFitWarps + warp);
     if (first >= nblocks) return;
-    const bool live = first + (lane >> 4) < nblocks;  // the last warp's second half may have no block
+    const bool live = (lane >> 4) < per_warp && first + (lane >> 4) < nblocks;  // a half without a block follows the other's
     const long long gblk = live ? first + (lane >> 4) : first;
     const EncJob &J = jobs[find_job(jobs, njobs, gblk)];
     const int blk = (int)(gblk - J.first_block);
@@ -1440,8 +1441,8 @@ constexpr long long kSquishWarpBlocks = 68096;
 
 template <bool DXT1>
 static int launch_squish(const EncJob *d_jobs, int njobs, long long nblocks, cudaStream_t stream) {
-    const long long per = 2 * kFitWarps;
-    k_squish<DXT1><<<(unsigned)((nblocks + per - 1) / per), 32 * kFitWarps, 0, stream>>>(d_jobs, njobs, nblocks);
+    const int per_warp = fit_blocks_per_warp(nblocks), per = per_warp * kFitWarps;
+    k_squish<DXT1><<<(unsigned)((nblocks + per - 1) / per), 32 * kFitWarps, 0, stream>>>(d_jobs, njobs, nblocks, per_warp);
     return launch_status();
 }
 

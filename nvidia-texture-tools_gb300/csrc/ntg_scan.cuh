@@ -301,6 +301,12 @@ struct FitBest {
 constexpr unsigned kAll = 0xffffffffu;
 constexpr int kFitWarps = 4;  // warps per CTA, each on its own
 
+// Blocks per warp of a launch: one where the GPU holds a warp for each (152 SMs x 5 CTAs x 4 warps), because what such a
+// launch takes is one warp's time through its blocks. One float level, two blocks per warp against one: BC1 32x32 28 and
+// 21 us, 128x128 27 and 23, 192x192 (2,304 blocks) 29 and 25, 256x256 (4,096) 35 and 39; BC3 64x64 38 and 29, 192x192 39
+// and 31, 256x256 41 and 44.
+constexpr int fit_blocks_per_warp(long long nblocks) { return nblocks <= 152 * 5 * kFitWarps ? 1 : 2; }
+
 // One half's scratch in shared memory.
 struct HalfScratch {
     float stage[16 * 8];  // terms per texel or colour

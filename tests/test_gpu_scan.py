@@ -77,3 +77,16 @@ def test_squish_launch_sizes_agree(ctx, fmt, kind):
     img = torch.cat([img, img[:, :4 * 8097]], 1).contiguous()
     large = ctx.encode(fmt, img, w, 4 * 68097, quality=1, alpha_mode=1)
     assert torch.equal(large[:small.numel()], small)
+
+
+@pytest.mark.parametrize("blocks", [3040, 3041, 6083])
+@pytest.mark.parametrize("fmt", [ntg.FORMAT_BC1, ntg.FORMAT_BC1A, ntg.FORMAT_BC3])
+def test_blocks_per_warp(ctx, oracle, fmt, blocks):
+    """Where launches go from one block per warp to two (3,040 blocks), and an odd count above it."""
+    image = {ntg.FORMAT_BC1: oracle.bc1_image, ntg.FORMAT_BC3: oracle.bc3_image,
+             ntg.FORMAT_BC1A: lambda i, w, h, alpha, q, **kw: oracle.bc1a_image(i, w, h, alpha, **kw)}[fmt]
+    w, h = 4, 4 * blocks
+    for kind in KINDS:
+        img = contents(kind, w, h, blocks + len(kind))
+        got = ctx.encode(fmt, torch.from_numpy(img).cuda(), w, h, quality=1, alpha_mode=1)
+        assert np.array_equal(got.cpu().numpy(), image(img, w, h, 1, 1, threads=8)), kind
