@@ -135,6 +135,43 @@ struct XformTables {
 
 }  // namespace
 
+// A second stream for work that runs beside a call's own, and the events that tie the two: the call's stream waits for it
+// before the call returns, so whatever is ordered after the call is ordered after both. Its priority is the highest, so
+// that the few CTAs of a small launch don't queue behind the thousands of an encoder.
+struct SideStream {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    int create() {
+        if (stream && fork && join) return NTG_OK;
+        int least = 0, greatest = 0;
+        NTG_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        if (!fork) NTG_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+        if (!join) NTG_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+        if (!stream) NTG_CUDA(cudaStreamCreateWithPriority(&stream, cudaStreamNonBlocking, greatest));
+        return NTG_OK;
+    }
+    // What `s` has been given so far precedes the side stream's next work.
+    int begin(cudaStream_t s) {
+        NTG_CUDA(cudaEventRecord(fork, s));
+        NTG_CUDA(cudaStreamWaitEvent(stream, fork, 0));
+        return NTG_OK;
+    }
+    // The side stream's work precedes what `s` is given next. Called also where the work between has failed.
+    int end(cudaStream_t s, int status) {
+        const cudaError_t a = cudaEventRecord(join, stream);
+        const cudaError_t b = a == cudaSuccess ? cudaStreamWaitEvent(s, join, 0) : a;
+        return status != NTG_OK ? status : b == cudaSuccess ? NTG_OK : cuda_fail(b, "join the side stream");
+    }
+    SideStream() = default;
+    SideStream(const SideStream &) = delete;
+    SideStream &operator=(const SideStream &) = delete;
+    ~SideStream() {
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
+        if (stream) cudaStreamDestroy(stream);
+    }
+};
+
 struct ntg_context {
     int device = 0;
     HostTables tables;
@@ -151,6 +188,7 @@ struct ntg_context {
     MipTuning tune;
     bool profile = false;       // record phase events in chain calls
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+    SideStream side;            // see Overlap
 
     ~ntg_context() {
         cudaSetDevice(device);
@@ -647,15 +685,20 @@ int launch_encode(int format, const EncJob *d_jobs, int njobs, long long nblocks
     return launched(r, "encoder launch");
 }
 
-// Encode jobs of a chain: level 0 from the input bytes (through the composed transform tables),
+// Encode jobs of a chain's levels from..to - 1: level 0 from the input bytes (through the composed transform tables),
 // the other levels from the workspace.
 void chain_jobs(const ChainPlan &P, const uint32_t *d_bgra, const ntg_chain_options &o, const XformTables *xt,
-                uint8_t *ws, uint8_t *d_blocks, std::vector<EncJob> &jobs, long long &nblocks) {
+                uint8_t *ws, uint8_t *d_blocks, std::vector<EncJob> &jobs, long long &nblocks, size_t from = 0,
+                size_t to = SIZE_MAX) {
     float cw[3];
     colour_weights(o, cw);
     size_t out_off = 0;
-    for (size_t l = 0; l < P.lv.size(); l++) {
+    for (size_t l = 0; l < std::min(to, P.lv.size()); l++) {
         const Level &L = P.lv[l];
+        if (l < from) {
+            out_off += (size_t)block_bytes(o.format) * blocks_of(L.w, L.h);
+            continue;
+        }
         EncJob j;
         std::memset(&j, 0, sizeof j);
         j.w = L.w; j.h = L.h; j.bw = (L.w + 3) / 4;
@@ -675,6 +718,46 @@ void chain_jobs(const ChainPlan &P, const uint32_t *d_bgra, const ntg_chain_opti
         nblocks += blocks_of(L.w, L.h);
         out_off += (size_t)block_bytes(o.format) * blocks_of(L.w, L.h);
     }
+}
+
+// Which levels of a chain are encoded beside the mip filters of the others.
+//   beside_tail: the levels before the tail, on the side stream, beside the tail (one CTA) and the encoding of its levels,
+//     which are about as long for small images;
+//   else: levels 0 and 1, as soon as level 1 is there, beside all the other levels' filters and their encoding, which go
+//     to the side stream. (Level 0 alone, from the start: the filters' large CTAs then wait for SMs that the encoder
+//     keeps full; 2048x2048 BC1 with Kaiser mips gained 14 us of 1,838 that way and 41 this way.)
+// Measured, BC1 unless stated, one after the other / beside the tail / beside the filters, us: 64x64 40 / 35 / 37, 256x256
+// 65 / 56 / 74, 384x384 106 / 98 / 98, 512x512 155 / 145 / 135, 1024x1024 473 / 461 / 451; BC3 256x256 101 / 80 / 92, 512x512
+// 177 / 157 / 148, 2048x2048 (k_bc3, whose CTAs hold their SM for 0.4 ms) 1,542 / 1,543 / 1,579; BC5 1024x1024 107 / 100 /
+// 109, 1500x1500 163 / 157 / 154, 2048x2048 235 / 227 / 195; Fastest BC1 1024x1024 73 / 66 / 74.
+struct Overlap {
+    size_t split = 0;  // levels of the first launch; 0: no overlap
+    bool beside_tail = false;
+};
+
+Overlap chain_overlap(const ChainPlan &P, const ntg_chain_options &o, size_t tail) {
+    const long long first = blocks_of(P.lv[0].w, P.lv[0].h);
+    bool deep;  // beside the filters
+    if (o.format == NTG_FORMAT_BC1)
+        deep = o.quality != NTG_QUALITY_FASTEST && first >= 12288;
+    else if ((o.format == NTG_FORMAT_BC3 || o.format == NTG_FORMAT_BC1A) && (o.quality == NTG_QUALITY_NORMAL || o.quality == NTG_QUALITY_PRODUCTION))
+        deep = first >= 12288 && first <= 52000;  // both launches in the warp kernel (k_squish)
+    else
+        deep = first >= 131072;
+    Overlap v;
+    if (first < 1024) return v;  // smaller ones gain nothing: tail and encoder are one CTA's and one warp's time either way
+    v.beside_tail = !deep;
+    v.split = deep ? std::min<size_t>(tail, 2) : tail;
+    if (v.split >= P.lv.size()) v.split = 0;
+    return v;
+}
+
+// True while `s` records a graph: a stream that joins the recording stays part of it until it ends, which may be after
+// another call wants the side stream.
+bool recording(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) { cudaGetLastError(); return true; }
+    return st != cudaStreamCaptureStatusNone;
 }
 
 // Surface::toLinear/toGamma return early for gamma == 1 (nv::equal, src/nvtt/Surface.cpp:1470-1488).
@@ -1020,9 +1103,30 @@ static int chain_common(ntg_context *ctx, const void *d_bgra, int w, int h, cons
     if (!xt) return fail(NTG_ERROR_CUDA, "table upload failed");
     uint8_t *ws = reinterpret_cast<uint8_t *>(d_levels);  // levels that the call returns are built where they belong
     if (!d_levels) NTG_TRY(ctx->workspace(std::max<size_t>(P.bytes, 256), s, &ws));
-    // The mip levels, then one encoder launch over every level. (Encoding level 0 beside the mip
-    // launches, on a lower-priority stream, measured slower: the encoder's CTAs hold nearly all of an
-    // SM's registers for ~0.4 ms each, so every mip launch first waits for SMs to drain.)
+    const size_t tail = tail_start(P, ctx->tune);
+    const Overlap ov = d_blocks && !ctx->profile && !recording(s) ? chain_overlap(P, *opt, tail) : Overlap();
+    if (ov.split) {
+        NTG_TRY(ctx->side.create());
+        std::vector<MipJob> all;
+        std::vector<std::vector<MipLaunch>> stages;
+        NTG_TRY(chain_stages(ctx, P, (const uint32_t *)d_bgra, *opt, xt, ws, all, stages));
+        NTG_TRY(upload_mip_jobs(ctx, all, s));
+        std::vector<EncJob> jobs;
+        long long early = 0, late = 0;
+        chain_jobs(P, (const uint32_t *)d_bgra, *opt, xt, ws, (uint8_t *)d_blocks, jobs, early, 0, ov.split);
+        chain_jobs(P, (const uint32_t *)d_bgra, *opt, xt, ws, (uint8_t *)d_blocks, jobs, late, ov.split);
+        NTG_TRY(upload_jobs(ctx, jobs, s));
+        const auto cut = stages.begin() + std::min(stages.size(), ov.split - 1);
+        const std::vector<std::vector<MipLaunch>> before(stages.begin(), cut), after(cut, stages.end());
+        NTG_TRY(run_stages(before, ctx->d_mipjobs, s));
+        NTG_TRY(ctx->side.begin(s));
+        const cudaStream_t filters = ov.beside_tail ? s : ctx->side.stream, encoder = ov.beside_tail ? ctx->side.stream : s;
+        int r = run_stages(after, ctx->d_mipjobs, filters);
+        if (r == NTG_OK) r = launch_encode(opt->format, ctx->d_jobs, (int)ov.split, early, opt->quality, encoder);
+        if (r == NTG_OK)
+            r = launch_encode(opt->format, ctx->d_jobs + ov.split, (int)(jobs.size() - ov.split), late, opt->quality, filters);
+        return ctx->side.end(s, r);
+    }
     if (ctx->profile) NTG_CUDA(cudaEventRecord(ctx->ev[0], s));
     NTG_TRY(build_levels(ctx, P, (const uint32_t *)d_bgra, *opt, xt, ws, s));
     if (ctx->profile) NTG_CUDA(cudaEventRecord(ctx->ev[1], s));

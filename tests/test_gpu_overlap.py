@@ -1,0 +1,77 @@
+"""Chains whose first levels are encoded beside the filters of the others, against the same calls with the phases timed,
+which run one after the other: at the sizes where the rule changes, odd extents, chains without a tail, and calls from
+several threads and streams on one context."""
+import threading
+
+import numpy as np
+import pytest
+
+import ntg
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+def image(w, h, seed):
+    rng = np.random.default_rng(seed)
+    img = rng.integers(0, 256, (h, w, 4), dtype=np.uint8)
+    img[: h // 2] = img[: h // 2] // 16 + 100  # half of it nearly flat
+    return torch.from_numpy(img).cuda()
+
+
+def serial(ctx, img, w, h, opt):
+    ctx.profile(True)
+    try:
+        return ctx.compress_chain(img, w, h, opt)
+    finally:
+        ctx.profile(False)
+
+
+SIZES = [(1, 1), (2, 5), (4, 4), (16, 16), (33, 64), (65, 65), (64, 1), (200, 120), (444, 440), (448, 439), (512, 512),
+         (513, 770), (1366, 769), (1500, 3)]
+
+
+@pytest.mark.parametrize("fmt", [ntg.FORMAT_BC1, ntg.FORMAT_BC1A, ntg.FORMAT_BC3, ntg.FORMAT_BC4, ntg.FORMAT_BC5])
+@pytest.mark.parametrize("filt", [ntg.FILTER_BOX, ntg.FILTER_KAISER])
+def test_chain(ctx, fmt, filt):
+    for i, (w, h) in enumerate(SIZES):
+        img = image(w, h, i)
+        for quality, x, levels in [(1, ntg.XFORM_SRGB, 0), (0, ntg.XFORM_NONE, 0), (1, ntg.XFORM_GAMMA, 2), (1, ntg.XFORM_NONE, 1)]:
+            if fmt == ntg.FORMAT_BC1A and quality == 0:
+                continue
+            opt = ntg.ChainOptions.make(format=fmt, quality=quality, filter=filt, alpha_mode=ntg.ALPHA_TRANSPARENCY, in_xform=x,
+                                        out_xform=x, max_levels=levels)
+            assert torch.equal(ctx.compress_chain(img, w, h, opt), serial(ctx, img, w, h, opt)), (w, h, quality, levels)
+
+
+@pytest.mark.parametrize("fmt,size", [(ntg.FORMAT_BC5, 1452), (ntg.FORMAT_BC3, 912), (ntg.FORMAT_BC3, 916), (ntg.FORMAT_BC1, 2048)])
+def test_large(ctx, fmt, size):
+    img = image(size, size, 9)
+    opt = ntg.ChainOptions.make(format=fmt, filter=ntg.FILTER_TRIANGLE)
+    assert torch.equal(ctx.compress_chain(img, size, size, opt), serial(ctx, img, size, size, opt))
+
+
+def test_streams_and_threads(ctx):
+    """Each thread's chains on its own stream and context, and the results read on that stream straight away."""
+    errors = []
+
+    def work(k):
+        own = ntg.Context(0)
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            for i in range(6):
+                w, h = [(64, 64), (512, 512), (700, 300)][(i + k) % 3]
+                opt = ntg.ChainOptions.make(format=[ntg.FORMAT_BC1, ntg.FORMAT_BC3][k % 2])
+                img = image(w, h, 10 * k + i)
+                got = own.compress_chain(img, w, h, opt).clone()
+                img.zero_()  # ordered after the call
+                stream.synchronize()
+                if not torch.equal(got, serial(own, image(w, h, 10 * k + i), w, h, opt)):
+                    errors.append((k, i))
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
