@@ -75,3 +75,18 @@ def test_streams_and_threads(ctx):
     for t in threads:
         t.join()
     assert not errors
+
+
+@pytest.mark.parametrize("filt", [ntg.FILTER_BOX, ntg.FILTER_KAISER])
+def test_levels(ctx, filt):
+    """Returned levels: level 0 is written beside the filters of the others."""
+    for w, h in [(1, 1), (2, 5), (65, 65), (513, 770), (1024, 1024)]:
+        img = image(w, h, w)
+        for levels in (0, 1, 2):
+            opt = ntg.ChainOptions.make(filter=filt, in_xform=ntg.XFORM_SRGB, max_levels=levels)
+            got = ctx.mip_chain(img, w, h, opt)
+            ctx.profile(True)
+            try:
+                assert torch.equal(got, ctx.mip_chain(img, w, h, opt)), (w, h, levels)
+            finally:
+                ctx.profile(False)
