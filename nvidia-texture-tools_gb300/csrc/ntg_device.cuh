@@ -13,6 +13,14 @@
 
 namespace ntg {
 
+// See launch_after: lets the next launch's CTAs in, and waits until the previous launch is complete and its writes are
+// visible. `njobs`, from which a kernel finds its job and through that its data, comes out of the wait, so that no load of
+// data is moved above it. (Passing the job list's pointer through instead lost its __restrict__, and the filters 10%.)
+__device__ __forceinline__ void after_previous(int &njobs, int order) {
+    if (order & 1) asm volatile("griddepcontrol.launch_dependents;");
+    if (order & 2) asm volatile("griddepcontrol.wait;" : "+r"(njobs) : : "memory");
+}
+
 // Min/max in the two comparison forms the reference uses; they differ on NaN.
 //   ic_*: icbc::max/min and nv::max/min   (src/nvtt/icbc.h:180-190, src/nvcore/Utils.h:159-187)
 //   sq_*: std::max/std::min as squish calls them (src/nvtt/squish/maths.h)

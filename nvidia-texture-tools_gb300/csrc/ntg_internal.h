@@ -25,6 +25,28 @@ inline int launch_status() {
     return e == cudaSuccess ? 0 : kLaunchErrorBase + (int)e;
 }
 
+// How a kernel of a sequence is launched. EARLY: it may begin while the kernel before it on the stream is running, so that
+// its CTAs are resident, past their launch latency, when that one ends; that one has LETS_IN. Such kernels' first statement
+// is after_previous (ntg_device.cuh), in every thread, so that nothing they read or write is earlier than in plain stream
+// order. (Letting others in where none follows early costs a few per cent.)
+enum LaunchOrder { PLAIN = 0, LETS_IN = 1, EARLY = 2 };
+
+template <typename... P, typename... A>
+inline int launch_after(int order, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &attr;
+    c.numAttrs = order & EARLY ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, (P)args...);
+    return launch_status();
+}
+
 // One texture level to encode. An encoder launch walks a list of jobs: thread-blocks of 4x4
 // texels are numbered across all jobs and a thread finds its job by binary search over the
 // running block counts (`first_block`), so one launch covers a whole mip chain or a batch of
@@ -123,7 +145,7 @@ struct MipLaunch {
 int launch_set_image(const uint32_t *bgra, size_t n, const float *lut, float *out, cudaStream_t s);
 int launch_quantize(const float *rgba, size_t n, int xform, const float *steps, uint32_t *out, cudaStream_t s);
 int launch_transform(float *rgba, size_t n, int kind, float p, cudaStream_t s);
-int launch_mip(const MipLaunch &m, const MipJob *d_jobs, cudaStream_t s);
+int launch_mip(const MipLaunch &m, const MipJob *d_jobs, cudaStream_t s, int order = PLAIN);
 // The sRGB curves' correction tables (ntg_device.cuh): one chunk of entries from the host's results,
 // and the tables' device addresses for the kernels of each translation unit that evaluates the curves.
 int launch_srgb_fix(const float *host_chunk, uint32_t first, uint32_t count, int which, uint8_t *fix, unsigned int *bad,

@@ -165,7 +165,8 @@ __device__ __forceinline__ void load_steps(const MipJob *__restrict__ jobs, floa
 // destination texel, all four channels. U8: the source is the BGRA8 input through the input transform table (level 1 of
 // every chain): read as FP32 it had to be written first, 16 bytes a texel, by a launch of its own.
 template <bool U8>
-__global__ void k_fast_down(const MipJob *__restrict__ jobs, int njobs, long long units) {
+__global__ void k_fast_down(const MipJob *__restrict__ jobs, int njobs, long long units, int order) {
+    after_previous(njobs, order);
     __shared__ float s_steps[256];
     __shared__ float s_lut[U8 ? 512 : 1];
     load_steps(jobs, s_steps);
@@ -320,7 +321,8 @@ constexpr int PWARPS = PTHREADS / 32;
 // tile: wrap maps for the tile's source rows and columns, the wrapped source window staged once as
 // float4, X taps for every window row into a (rows x PTW) plane, then the Y taps.
 template <bool WEIGHTED, bool SRC_U8>
-__global__ void __launch_bounds__(PTHREADS) k_poly(const MipJob *__restrict__ jobs, int njobs) {
+__global__ void __launch_bounds__(PTHREADS) k_poly(const MipJob *__restrict__ jobs, int njobs, int order) {
+    after_previous(njobs, order);
     extern __shared__ float4 sm4[];
     __shared__ float s_kx[PTW * PMAXW], s_ky[PTH * PMAXW], s_steps[256];
     __shared__ int s_lx[PTW], s_ly[PTH];
@@ -426,7 +428,8 @@ __device__ __forceinline__ void fetch_raw(const MipJob &L, size_t s, size_t sn, 
 }
 
 template <int WS, bool WEIGHTED, bool SRC_U8>
-__global__ void __launch_bounds__(512, 2) k_tile2x(const MipJob *__restrict__ jobs, int njobs) {
+__global__ void __launch_bounds__(512, 2) k_tile2x(const MipJob *__restrict__ jobs, int njobs, int order) {
+    after_previous(njobs, order);
     using P = Tile2x<WS>;
     constexpr int TW = P::TW, RW = P::RW, HALF = P::HALF, ROW = P::ROW;
     extern __shared__ float4 sm4[];
@@ -640,7 +643,8 @@ __device__ __forceinline__ void tile_u8_fetch(const TilePos &p, uint32_t *raw) {
 }
 
 template <int WS, bool WEIGHTED>
-__global__ void __launch_bounds__(1024, 1) k_tile2x_u8(const MipJob *__restrict__ jobs, int njobs, long long units) {
+__global__ void __launch_bounds__(1024, 1) k_tile2x_u8(const MipJob *__restrict__ jobs, int njobs, long long units, int order) {
+    after_previous(njobs, order);
     using P = TileU8<WS>;
     constexpr int TW = P::TW, TH = P::TH, D = P::D, NC = P::NC, QP = P::QP, ROWS = P::ROWS;
     extern __shared__ float4 sm4[];
@@ -856,7 +860,8 @@ __device__ __forceinline__ void tile_f32_fetch(const TileF32Pos &p, float *raw, 
 }
 
 template <int WS>
-__global__ void __launch_bounds__(1024, 1) k_tile2x_f32(const MipJob *__restrict__ jobs, int njobs, long long units) {
+__global__ void __launch_bounds__(1024, 1) k_tile2x_f32(const MipJob *__restrict__ jobs, int njobs, long long units, int order) {
+    after_previous(njobs, order);
     using P = TileF32<WS>;
     constexpr int TW = P::TW, D = P::D, NC = P::NC, NV = P::NV;
     extern __shared__ float4 sm4[];
@@ -1103,7 +1108,8 @@ __device__ __forceinline__ float4 tail_taps(const float4 *src, int stride, const
 }
 
 template <bool WEIGHTED>
-__global__ void __launch_bounds__(1024) k_mip_tail(const MipJob *__restrict__ jobs, int njobs) {
+__global__ void __launch_bounds__(1024) k_mip_tail(const MipJob *__restrict__ jobs, int njobs, int order) {
+    after_previous(njobs, order);
     extern __shared__ float4 sm4[];
     __shared__ float s_steps[256];
     __shared__ uint8_t s_buckets[kSrgbBuckets];
@@ -1296,33 +1302,31 @@ int launch_quantize(const float *rgba, size_t n, int xform, const float *steps, 
 }
 
 template <bool W, bool U8>
-static int launch_poly_t(const MipLaunch &m, const MipJob *jobs, cudaStream_t s) {
+static int launch_poly_t(const MipLaunch &m, const MipJob *jobs, cudaStream_t s, int order) {
     static std::atomic<unsigned long long> configured{0};
     if (first_use_on_device(configured))
         cudaFuncSetAttribute(k_poly<W, U8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    k_poly<W, U8><<<(unsigned)m.units, PTHREADS, m.smem, s>>>(jobs, m.njobs);
-    return launch_status();
+    return launch_after(order, k_poly<W, U8>, (unsigned)m.units, PTHREADS, m.smem, s, jobs, m.njobs, order);
 }
 
 template <int WS, bool W, bool U8>
-static int launch_tile2x_t(const MipLaunch &m, const MipJob *jobs, cudaStream_t s) {
+static int launch_tile2x_t(const MipLaunch &m, const MipJob *jobs, cudaStream_t s, int order) {
     static std::atomic<unsigned long long> configured{0};
     if (first_use_on_device(configured))
         cudaFuncSetAttribute(k_tile2x<WS, W, U8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    k_tile2x<WS, W, U8><<<(unsigned)m.units, m.threads, m.smem, s>>>(jobs, m.njobs);
-    return launch_status();
+    return launch_after(order, k_tile2x<WS, W, U8>, (unsigned)m.units, m.threads, m.smem, s, jobs, m.njobs, order);
 }
 
 template <int WS>
-static int launch_tile2x_ws(const MipLaunch &m, const MipJob *jobs, cudaStream_t s) {
-    if (m.weighted) return m.u8 ? launch_tile2x_t<WS, true, true>(m, jobs, s) : launch_tile2x_t<WS, true, false>(m, jobs, s);
-    return m.u8 ? launch_tile2x_t<WS, false, true>(m, jobs, s) : launch_tile2x_t<WS, false, false>(m, jobs, s);
+static int launch_tile2x_ws(const MipLaunch &m, const MipJob *jobs, cudaStream_t s, int order) {
+    if (m.weighted) return m.u8 ? launch_tile2x_t<WS, true, true>(m, jobs, s, order) : launch_tile2x_t<WS, true, false>(m, jobs, s, order);
+    return m.u8 ? launch_tile2x_t<WS, false, true>(m, jobs, s, order) : launch_tile2x_t<WS, false, false>(m, jobs, s, order);
 }
 
 bool poly2x_supported(int ws) { return ws == 3 || ws == 5 || ws == 13; }
 
 template <int WS, bool W>
-static int launch_tile2x_u8_t(const MipLaunch &m, const MipJob *jobs, cudaStream_t s) {
+static int launch_tile2x_u8_t(const MipLaunch &m, const MipJob *jobs, cudaStream_t s, int order) {
     static std::atomic<unsigned long long> configured{0};
     static int sms = 0;
     if (first_use_on_device(configured)) {
@@ -1332,17 +1336,16 @@ static int launch_tile2x_u8_t(const MipLaunch &m, const MipJob *jobs, cudaStream
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d);
     }
     const long long grid = std::min<long long>(m.units, sms > 0 ? sms : 152);
-    k_tile2x_u8<WS, W><<<(unsigned)grid, 1024, TileU8<WS>::smem(), s>>>(jobs, m.njobs, m.units);
-    return launch_status();
+    return launch_after(order, k_tile2x_u8<WS, W>, (unsigned)grid, 1024, TileU8<WS>::smem(), s, jobs, m.njobs, m.units, order);
 }
 
 template <int WS>
-static int launch_tile2x_u8_ws(const MipLaunch &m, const MipJob *jobs, cudaStream_t s) {
-    return m.weighted ? launch_tile2x_u8_t<WS, true>(m, jobs, s) : launch_tile2x_u8_t<WS, false>(m, jobs, s);
+static int launch_tile2x_u8_ws(const MipLaunch &m, const MipJob *jobs, cudaStream_t s, int order) {
+    return m.weighted ? launch_tile2x_u8_t<WS, true>(m, jobs, s, order) : launch_tile2x_u8_t<WS, false>(m, jobs, s, order);
 }
 
 template <int WS>
-static int launch_tile2x_f32_t(const MipLaunch &m, const MipJob *jobs, cudaStream_t s) {
+static int launch_tile2x_f32_t(const MipLaunch &m, const MipJob *jobs, cudaStream_t s, int order) {
     static std::atomic<unsigned long long> configured{0};
     static int sms = 0;
     if (first_use_on_device(configured)) {
@@ -1352,8 +1355,7 @@ static int launch_tile2x_f32_t(const MipLaunch &m, const MipJob *jobs, cudaStrea
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d);
     }
     const long long grid = std::min<long long>(m.units, sms > 0 ? sms : 152);
-    k_tile2x_f32<WS><<<(unsigned)grid, 1024, TileF32<WS>::smem(), s>>>(jobs, m.njobs, m.units);
-    return launch_status();
+    return launch_after(order, k_tile2x_f32<WS>, (unsigned)grid, 1024, TileF32<WS>::smem(), s, jobs, m.njobs, m.units, order);
 }
 
 int tile_f32_phase(int ws) {
@@ -1456,45 +1458,43 @@ size_t poly2x_smem_bytes(int ws, int tile_h) {
     return ws == 3 ? Tile2x<3>::smem(tile_h) : ws == 5 ? Tile2x<5>::smem(tile_h) : Tile2x<13>::smem(tile_h);
 }
 
-int launch_mip(const MipLaunch &m, const MipJob *d_jobs, cudaStream_t s) {
+int launch_mip(const MipLaunch &m, const MipJob *d_jobs, cudaStream_t s, int order) {
     if (m.units <= 0 || m.njobs <= 0) return 0;
     const MipJob *jobs = d_jobs + m.first_job;
     switch (m.kernel) {
         case MIP_FAST_BOX: {
             const long long cap = 152LL * 64, g = (m.units + 255) / 256;
-            if (m.u8) k_fast_down<true><<<(unsigned)(g < cap ? g : cap), 256, 0, s>>>(jobs, m.njobs, m.units);
-            else k_fast_down<false><<<(unsigned)(g < cap ? g : cap), 256, 0, s>>>(jobs, m.njobs, m.units);
-            return launch_status();
+            return launch_after(order, m.u8 ? k_fast_down<true> : k_fast_down<false>, (unsigned)(g < cap ? g : cap), 256, 0, s, jobs,
+                                    m.njobs, m.units, order);
         }
         case MIP_POLY:
             if (m.smem > 200 * 1024) return 2;  // Error_UnsupportedFeature
-            if (m.weighted) return m.u8 ? launch_poly_t<true, true>(m, jobs, s) : launch_poly_t<true, false>(m, jobs, s);
-            return m.u8 ? launch_poly_t<false, true>(m, jobs, s) : launch_poly_t<false, false>(m, jobs, s);
+            if (m.weighted) return m.u8 ? launch_poly_t<true, true>(m, jobs, s, order) : launch_poly_t<true, false>(m, jobs, s, order);
+            return m.u8 ? launch_poly_t<false, true>(m, jobs, s, order) : launch_poly_t<false, false>(m, jobs, s, order);
         case MIP_TAIL: {
             static std::atomic<unsigned long long> configured{0};
             if (first_use_on_device(configured)) {
                 cudaFuncSetAttribute(k_mip_tail<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tail_smem_bytes());
                 cudaFuncSetAttribute(k_mip_tail<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tail_smem_bytes());
             }
-            if (m.weighted) k_mip_tail<true><<<(unsigned)m.units, 1024, tail_smem_bytes(), s>>>(jobs, m.njobs);
-            else k_mip_tail<false><<<(unsigned)m.units, 1024, tail_smem_bytes(), s>>>(jobs, m.njobs);
-            return launch_status();
+            return launch_after(order, m.weighted ? k_mip_tail<true> : k_mip_tail<false>, (unsigned)m.units, 1024, tail_smem_bytes(), s,
+                                    jobs, m.njobs, order);
         }
         case MIP_TILE_U8:
-            if (m.ws == 3) return launch_tile2x_u8_ws<3>(m, jobs, s);
-            if (m.ws == 5) return launch_tile2x_u8_ws<5>(m, jobs, s);
-            if (m.ws == 13) return launch_tile2x_u8_ws<13>(m, jobs, s);
+            if (m.ws == 3) return launch_tile2x_u8_ws<3>(m, jobs, s, order);
+            if (m.ws == 5) return launch_tile2x_u8_ws<5>(m, jobs, s, order);
+            if (m.ws == 13) return launch_tile2x_u8_ws<13>(m, jobs, s, order);
             return 2;
         case MIP_TILE_F32:
-            if (m.ws == 3) return launch_tile2x_f32_t<3>(m, jobs, s);
-            if (m.ws == 5) return launch_tile2x_f32_t<5>(m, jobs, s);
-            if (m.ws == 13) return launch_tile2x_f32_t<13>(m, jobs, s);
+            if (m.ws == 3) return launch_tile2x_f32_t<3>(m, jobs, s, order);
+            if (m.ws == 5) return launch_tile2x_f32_t<5>(m, jobs, s, order);
+            if (m.ws == 13) return launch_tile2x_f32_t<13>(m, jobs, s, order);
             return 2;
         case MIP_POLY2X:
             if (m.threads < 64 || m.threads > 512 || m.threads % 32 || m.smem > 200 * 1024) return 1;
-            if (m.ws == 3) return launch_tile2x_ws<3>(m, jobs, s);
-            if (m.ws == 5) return launch_tile2x_ws<5>(m, jobs, s);
-            if (m.ws == 13) return launch_tile2x_ws<13>(m, jobs, s);
+            if (m.ws == 3) return launch_tile2x_ws<3>(m, jobs, s, order);
+            if (m.ws == 5) return launch_tile2x_ws<5>(m, jobs, s, order);
+            if (m.ws == 13) return launch_tile2x_ws<13>(m, jobs, s, order);
             return 2;
         default:
             return 1;
