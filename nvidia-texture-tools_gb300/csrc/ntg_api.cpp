@@ -698,8 +698,8 @@ int upload_jobs(ntg_context *ctx, const std::vector<EncJob> &jobs, cudaStream_t 
 }
 
 int launch_encode(int format, const EncJob *d_jobs, int njobs, long long nblocks, int quality, cudaStream_t s,
-                  int threads = 0) {
-    int r = format == NTG_FORMAT_BC1    ? launch_bc1(d_jobs, njobs, nblocks, quality, threads, s)
+                  bool transformed, int threads = 0) {
+    int r = format == NTG_FORMAT_BC1    ? launch_bc1(d_jobs, njobs, nblocks, quality, threads, transformed, s)
             : format == NTG_FORMAT_BC3  ? launch_bc3(d_jobs, njobs, nblocks, quality, threads, s)
             : format == NTG_FORMAT_BC1A ? launch_bc1a(d_jobs, njobs, nblocks, quality, threads, s)
             : format == NTG_FORMAT_BC4  ? launch_bc4(d_jobs, njobs, nblocks, quality, threads, s)
@@ -1106,7 +1106,7 @@ int ntg_encode(ntg_context *ctx, int format, const float *d_rgba, int w, int h, 
     j.first_block = 0;
     std::vector<EncJob> jobs(1, j);
     NTG_TRY(upload_jobs(ctx, jobs, s));
-    return launch_encode(format, ctx->d_jobs, 1, blocks_of(w, h), quality, s);
+    return launch_encode(format, ctx->d_jobs, 1, blocks_of(w, h), quality, s, j.out_xform != NTG_XFORM_NONE);
 }
 
 static int chain_common(ntg_context *ctx, const void *d_bgra, int w, int h, const ntg_chain_options *opt_in,
@@ -1145,9 +1145,10 @@ static int chain_common(ntg_context *ctx, const void *d_bgra, int w, int h, cons
         NTG_TRY(ctx->side.begin(s));
         const cudaStream_t filters = ov.beside_tail ? s : ctx->side.stream, encoder = ov.beside_tail ? ctx->side.stream : s;
         int r = run_stages(after, ctx->d_mipjobs, filters, ov.beside_tail, !before.empty());
-        if (r == NTG_OK) r = launch_encode(opt->format, ctx->d_jobs, (int)ov.split, early, opt->quality, encoder);
+        const bool xform = opt->out_xform != NTG_XFORM_NONE;  // of the float levels, all but level 0
+        if (r == NTG_OK) r = launch_encode(opt->format, ctx->d_jobs, (int)ov.split, early, opt->quality, encoder, xform && ov.split > 1);
         if (r == NTG_OK)
-            r = launch_encode(opt->format, ctx->d_jobs + ov.split, (int)(jobs.size() - ov.split), late, opt->quality, filters);
+            r = launch_encode(opt->format, ctx->d_jobs + ov.split, (int)(jobs.size() - ov.split), late, opt->quality, filters, xform);
         return ctx->side.end(s, r);
     }
     if (ctx->profile) NTG_CUDA(cudaEventRecord(ctx->ev[0], s));
@@ -1158,7 +1159,8 @@ static int chain_common(ntg_context *ctx, const void *d_bgra, int w, int h, cons
         long long nblocks = 0;
         chain_jobs(P, (const uint32_t *)d_bgra, *opt, xt, ws, (uint8_t *)d_blocks, jobs, nblocks);
         NTG_TRY(upload_jobs(ctx, jobs, s));
-        NTG_TRY(launch_encode(opt->format, ctx->d_jobs, (int)jobs.size(), nblocks, opt->quality, s));
+        NTG_TRY(launch_encode(opt->format, ctx->d_jobs, (int)jobs.size(), nblocks, opt->quality, s,
+                              opt->out_xform != NTG_XFORM_NONE && jobs.size() > 1));
     }
     if (ctx->profile) NTG_CUDA(cudaEventRecord(ctx->ev[2], s));
     return NTG_OK;
@@ -1460,6 +1462,7 @@ struct ntg_batch {
     struct Enc {
         int format, quality, first, njobs;
         long long nblocks;
+        bool transformed;  // an output transform on float levels
     };
     std::vector<Enc> encodes;
     MipTuning tune;
@@ -1589,11 +1592,13 @@ int batch_plan(ntg_batch *b) {
     std::vector<EncJob> ejobs;
     b->encodes.clear();
     for (auto &g : groups) {
-        ntg_batch::Enc e{g.first.first, g.first.second, (int)ejobs.size(), 0, 0};
+        ntg_batch::Enc e{g.first.first, g.first.second, (int)ejobs.size(), 0, 0, false};
         long long nb = 0;
-        for (size_t t : g.second)
+        for (size_t t : g.second) {
+            e.transformed = e.transformed || (b->opts[t].out_xform != NTG_XFORM_NONE && b->plans[t].lv.size() > 1);
             chain_jobs(b->plans[t], (const uint32_t *)b->io()[t].d_bgra, b->opts[t], b->xts[t], b->d_ws + b->base[t],
                        (uint8_t *)b->io()[t].d_blocks, ejobs, nb);
+        }
         e.njobs = (int)ejobs.size() - e.first;
         e.nblocks = nb;
         b->encodes.push_back(e);
@@ -1648,7 +1653,8 @@ int batch_encodes(ntg_batch *b, cudaStream_t s, int only_slot = -1) {
             }
             continue;
         }
-        NTG_TRY(launch_encode(e.format, b->denc() + e.first, e.njobs, e.nblocks, e.quality, s, b->enc_threads[enc_slot(e.format)]));
+        NTG_TRY(launch_encode(e.format, b->denc() + e.first, e.njobs, e.nblocks, e.quality, s, e.transformed,
+                              b->enc_threads[enc_slot(e.format)]));
     }
     return NTG_OK;
 }

@@ -279,7 +279,7 @@ __device__ int compute_sat(const Lane<float4> &col, int n, const Lane<float4> &s
 // whether the first colour in axis order projects above the last on frame_v (axis_reversed).
 // The table is a ZERO one: entry k holds the sum of the first k colours (entry 0 zero, n + 1
 // entries), so that a cumulative cluster end indexes it directly.
-__device__ int compute_sat_inplace(const Lane<float4> &col, int n, const f3 *frame_v = nullptr, bool *reversed = nullptr) {
+__device__ int compute_sat_inplace(const Lane<float4> &col, int n, const f3 *frame_v = nullptr, bool *reversed = nullptr, float *scatter = nullptr) {
     // computeCentroid / computeCovariance / firstEigenVector_PowerMethod as in compute_sat
     f3 c = mk3(0, 0, 0);
     float total = 0.0f;
@@ -293,6 +293,7 @@ __device__ int compute_sat_inplace(const Lane<float4> &col, int n, const f3 *fra
         m0 += a.x * b.x; m1 += a.x * b.y; m2 += a.x * b.z;
         m3 += a.y * b.y; m4 += a.y * b.z; m5 += a.z * b.z;
     }
+    if (scatter) *scatter = m0 + m3 + m5;
     f3 v;
     if (m0 == 0 && m3 == 0 && m5 == 0) {
         v = mk3(0, 0, 0);
@@ -1019,6 +1020,156 @@ __global__ void __launch_bounds__(32 * kFitWarps, NTG_BC1_MIN_CTAS) k_bc1(const 
 }
 
 // ---------------------------------------------------------------------------------------------
+// The cluster fits of large launches, one block per thread: each lane scans its own block's orderings (lane_scan), then the
+// warp evaluates its 32 blocks' possible winners exactly, 32 at a time whichever block they are of.
+//
+// Against two blocks per warp (k_bc1) the scan needs no loads of the orderings, reads a cluster sum once for two orderings
+// and keeps the rest of the fit at one lane per block; but it holds 404 bytes of shared memory per thread (16 warps on an
+// SM, 77,824 blocks in flight), knows only the lowest error so far when it flags an ordering (50 to 80 exact evaluations
+// per block instead of 15), and gathers the texels again for the output stage. Bound by the FMA pipe in the scan (154
+// cycles per scheduler and pair of orderings) and by latency in the evaluations. Measured, two blocks per warp and one
+// per thread: 1024x1024 323 and 374 us, 1400x1400 590 and 616, 1600x1600 766 and 766, 2048x2048 1,232 and 1,118 (second level
+// of a 4096x4096 texture 1,420 and 1,306), 4096x4096 4,972 and 4,112; with toSrgb on the way in, which every gather
+// repeats, 2048x2048 1,386 and 1,960. Every ordering evaluated exactly, one thread per block: 1,318, 1,326, 4,878, 1,650.
+constexpr int kLaneThreads = 64;
+constexpr long long kLaneBlocks = 150000;  // launches from here on, without an output transform on float texels
+static __device__ LanePairs g_lane_pairs;
+
+// One of the cluster fits of each lane's n colours (0: none; all lanes call it) by the warp: the end points to `ends`.
+// `prepare`: the colours are sorted and summed in place first, and the scan's constants set. `best`, `queue`: the warp's.
+template <bool UNIT>
+__device__ __noinline__ void lane_fit(const Lane<float4> &col, int n, bool prepare, bool four, f3 metric, ScanBlock *blk, float *ends,
+                                      unsigned long long *best, uint16_t *queue) {
+    if (prepare) {
+        float big = 0.0f, scatter;
+        bool whole = true;
+        for (int i = 0; i < n; i++) {
+            const float4 q = col[i];
+            big = fmaxf(big, max3_abs(q.x, q.y, q.z));
+            whole = whole && q.w == floorf(q.w);
+        }
+        compute_sat_inplace(col, n, nullptr, nullptr, &scatter);
+        const float4 s = col[n];
+        // lane_scan centres a sum after adding it up: 5 u W M more per unit of |d|, 15 in the end points' numerators
+        scan_begin(*blk, n, xyz(s), s.w, big, scatter, whole, metric, 46.0f + 5.0f, 47.0f + 15.0f, whole ? 0.0f : 67.0f);
+    }
+    const int lane = threadIdx.x & 31;
+    const uint32_t table = shared_address(&col[0]), words = shared_address(&col[17] - threadIdx.x) + 4 * threadIdx.x;
+    const float k = four ? 3.0f : 2.0f;
+    const int start = four ? g_lane_pairs.start4[n] : g_lane_pairs.start3[n];
+    int end = 0;
+    if (n > 0)
+        end = lane_scan<UNIT, kLaneThreads>(table, words, blk->mu[0], blk->mu[1], blk->mu[2], blk->W, blk->eta, 0.5f * k * blk->slack, n, start, 1, k,
+                                            make_float3(metric.x, metric.y, metric.z));
+    constexpr uint32_t stride = 16 * kLaneThreads;
+    const uint32_t table0 = table - 16 * lane;
+    const uint16_t *const pairs = four ? g_lane_pairs.four : g_lane_pairs.three;
+    auto eval = [&](int owner, int c0, int c1, int c2, f3 &ea, f3 &eb) {
+        const int on = __shfl_sync(kAll, n, owner);
+        const f3 om = UNIT ? mk3(1.0f, 1.0f, 1.0f) : mk3(__shfl_sync(kAll, metric.x, owner), __shfl_sync(kAll, metric.y, owner), __shfl_sync(kAll, metric.z, owner));
+        const uint32_t t = table0 + 16 * owner;
+        return fit_eval(four, load_shared(t + c0 * stride), load_shared(t + c1 * stride), load_shared(t + c2 * stride), load_shared(t + on * stride), om, ea, eb);
+    };
+    best[lane] = ~0ull;
+    __syncwarp();
+    const unsigned below = (1u << lane) - 1u;
+    uint32_t bits = 0;
+    int word = start >> 4, head = 0, tail = 0;
+    bool more = true;
+    while (more) {
+        while (bits == 0 && word < end) bits = load_word(words + 4 * kLaneThreads * word++);
+        const bool has = bits != 0;
+        const unsigned m = __ballot_sync(kAll, has);
+        more = m != 0;
+        if (has) {
+            queue[(tail + __popc(m & below)) & 63] = (uint16_t)(lane << 11 | 32 * (word - 1) | (__ffs(bits) - 1));
+            bits &= bits - 1;
+        }
+        tail += __popc(m);
+        __syncwarp();
+        if (tail - head < 32 && more) continue;
+        while (tail - head >= (more ? 32 : 1)) {
+            const bool valid = lane < tail - head;
+            const int it = queue[(head + (valid ? lane : 0)) & 63], owner = it >> 11, o = __ldg(pairs + ((it & 2047) >> 1)) + (it & 1);
+            const int c0 = o & 31, c1 = (o >> 5) & 31, c2 = o >> 10;
+            f3 ea, eb;
+            const float e = eval(owner, c0, c1, c2, ea, eb);
+            if (valid && e < FLT_MAX)
+                atomicMin(best + owner, (unsigned long long)float_order(e) << 32 | (unsigned)(four ? c2 << 10 | c0 << 5 | c1 : c2 << 10 | c0 << 5 | c2));
+            head += min(32, tail - head);
+        }
+        __syncwarp();
+    }
+    const unsigned long long won = best[lane];
+    const int o = won == ~0ull ? 0 : (int)(won & 0xffff);
+    f3 ea, eb;
+    eval(lane, (o >> 5) & 31, o & 31, o >> 10, ea, eb);
+    if (won == ~0ull) ea = eb = mk3(0, 0, 0);
+    ends[0] = ea.x; ends[1] = ea.y; ends[2] = ea.z; ends[3] = eb.x; ends[4] = eb.y; ends[5] = eb.z;
+}
+
+// icbc Level8.
+__global__ void __launch_bounds__(kLaneThreads, 8) k_bc1_lane(const EncJob *__restrict__ jobs, int njobs, long long nblocks) {
+    extern __shared__ float4 smem[];
+    __shared__ unsigned long long best[kLaneThreads / 32][32];
+    __shared__ uint16_t queue[kLaneThreads / 32][64];
+    const int T = kLaneThreads;
+    const int t = threadIdx.x;
+    long long gblk = (long long)blockIdx.x * T + t;
+    const bool live = gblk < nblocks;  // the others stay for the warp's evaluations
+    if (!live) gblk = nblocks - 1;
+    const EncJob &J = jobs[find_job(jobs, njobs, gblk)];
+    const int blk = (int)(gblk - J.first_block);
+    // texels, then reduced colours, then the summed-area table, each in the place of the one before
+    Lane<float4> in{smem + t, T};
+    Lane<float4> col = in;
+    const AlphaW wi{smem + t, T, J.alpha_mode == 1, valid_texels(J, blk)};
+    const f3 cw = mk3(J.cw[0], J.cw[1], J.cw[2]);
+    uint8_t *const out = J.out + 8 * (size_t)blk;
+    gather_block(J, blk, in, wi);
+    bool any_black = false;
+    const int cnt = reduce_colors(in, wi, col, any_black);
+    if (live && cnt <= 1) store_block(out, cnt == 0 ? Block1{0, 0, 0} : single_colour(col[0]));
+    const bool run = live && cnt > 1;
+    if (!__any_sync(kAll, run)) return;
+    const f3 metric = cw * cw;
+    const bool unit = __all_sync(kAll, metric.x == 1.0f && metric.y == 1.0f && metric.z == 1.0f) != 0;
+    ScanBlock sb;
+    float ends[12];
+    auto fit = [&](int n, bool prepare, bool four) {
+        if (unit) lane_fit<true>(col, n, prepare, four, metric, &sb, ends + (four ? 0 : 6), best[t >> 5], queue[t >> 5]);
+        else lane_fit<false>(col, n, prepare, four, metric, &sb, ends + (four ? 0 : 6), best[t >> 5], queue[t >> 5]);
+    };
+    fit(run ? cnt : 0, run, true);
+    int n3 = run ? cnt : 0;
+    if (run && any_black) {
+        gather_block(J, blk, in, wi);
+        bool again = false;
+        reduce_colors(in, wi, col, again);
+        int m = 0;
+        for (int i = 0; i < cnt; i++) {
+            float4 q = col[i];
+            if (is_black(xyz(q))) continue;
+            col[m++] = q;
+        }
+        n3 = m;
+    }
+    fit(n3, n3 > 0 && any_black, false);
+    if (!run) return;
+    const bool run3 = n3 > 0;
+    gather_block(J, blk, in, wi);
+    Block1 cf;
+    float cerr = output_block4(in, wi, cw, mk3(ends[0], ends[1], ends[2]), mk3(ends[3], ends[4], ends[5]), cf);
+    if (run3) {
+        Block1 c3;
+        float e3 = output_block3(in, wi, cw, true, mk3(ends[6], ends[7], ends[8]), mk3(ends[9], ends[10], ends[11]), c3);
+        if (e3 < cerr) { cerr = e3; cf = c3; }
+    }
+    // a NaN error leaves the block as k_bc1 does
+    store_block(out, cerr < FLT_MAX ? cf : Block1{0, 0, 0});
+}
+
+// ---------------------------------------------------------------------------------------------
 // Learned endpoint proposal (no counterpart in the reference). The network reads a block's texels
 // and proposes its two endpoints and the error of the full cluster fit. The proposal's palette
 // assigns each of the block's reduced colours, in the cluster fit's principal-axis order, to a
@@ -1520,8 +1671,13 @@ static int launch_bc1_fit(const EncJob *d_jobs, int njobs, long long nblocks, co
     return launch_status();
 }
 
-int launch_bc1(const EncJob *d_jobs, int njobs, long long nblocks, int quality, int threads, cudaStream_t stream) {
+int launch_bc1(const EncJob *d_jobs, int njobs, long long nblocks, int quality, int threads, bool transformed, cudaStream_t stream) {
     if (nblocks == 0) return 0;
+    if (quality == 1 && nblocks >= kLaneBlocks && !transformed) {
+        const size_t bytes = (size_t)kLaneThreads * (17 * sizeof(float4) + kLaneWords * sizeof(uint32_t));
+        k_bc1_lane<<<(unsigned)((nblocks + kLaneThreads - 1) / kLaneThreads), kLaneThreads, bytes, stream>>>(d_jobs, njobs, nblocks);
+        return launch_status();
+    }
     if (quality == 2) return launch_bc1_fit<8>(d_jobs, njobs, nblocks, nullptr, nullptr, stream);
     if (quality != 0) return launch_bc1_fit<7>(d_jobs, njobs, nblocks, nullptr, nullptr, stream);
     const int T = threads == 32 ? 32 : 64;  // blocks per CTA (one thread per 4x4 block)
@@ -1585,6 +1741,9 @@ int upload_tables_bc1(const HostTables &t) {
     ScanOrders<96> o3;
     float unit8[256];
     for (int v = 0; v < 256; v++) unit8[v] = (float)v / 255.0f;
+    LanePairs lp{};
+    lane_pairs(lp);
+    if (cudaMemcpyToSymbol(g_lane_pairs, &lp, sizeof lp) != cudaSuccess) return 3;
     scan_orders<3>(t.four, t.four_total[15], *o4);
     scan_orders<2>(t.three, t.three_total[15], o3);
     return cudaMemcpyToSymbol(c_tab, &t, sizeof t) == cudaSuccess && cudaMemcpyToSymbol(g_orders4, o4.get(), sizeof *o4) == cudaSuccess &&

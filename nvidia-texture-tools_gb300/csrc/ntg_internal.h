@@ -65,7 +65,8 @@ struct EncJob {
 };
 
 // threads = blocks per CTA (one thread per 4x4 block); 0 = the default shape.
-int launch_bc1(const EncJob *d_jobs, int njobs, long long nblocks, int quality, int threads, cudaStream_t s);
+// `transformed`: some job applies an output transform to float texels as it gathers them.
+int launch_bc1(const EncJob *d_jobs, int njobs, long long nblocks, int quality, int threads, bool transformed, cudaStream_t s);
 int launch_bc3(const EncJob *d_jobs, int njobs, long long nblocks, int quality, int threads, cudaStream_t s);
 int launch_bc5(const EncJob *d_jobs, int njobs, long long nblocks, int quality, int threads, cudaStream_t s);
 int launch_bc1a(const EncJob *d_jobs, int njobs, long long nblocks, int quality, int threads, cudaStream_t s);

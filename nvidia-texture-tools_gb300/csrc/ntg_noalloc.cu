@@ -152,7 +152,7 @@ extern "C" int ntg_encode_noalloc(ntg_context *ctx, int format, const float *d_r
         if (st != NTG_OK) return report_status(st, "quantise level");
     }
     const long long nblocks = (long long)((w + 3) / 4) * ((h + 3) / 4);
-    st = format == NTG_FORMAT_BC1    ? ntg::launch_bc1(d_job, 1, nblocks, quality, 0, s)
+    st = format == NTG_FORMAT_BC1    ? ntg::launch_bc1(d_job, 1, nblocks, quality, 0, false, s)
          : format == NTG_FORMAT_BC3  ? ntg::launch_bc3(d_job, 1, nblocks, quality, 0, s)
          : format == NTG_FORMAT_BC1A ? ntg::launch_bc1a(d_job, 1, nblocks, quality, 0, s)
          : format == NTG_FORMAT_BC4  ? ntg::launch_bc4(d_job, 1, nblocks, quality, 0, s)

@@ -390,4 +390,125 @@ __device__ __forceinline__ uint32_t spread_bits(uint32_t m) {
     return (m | (m << 1)) & 0x55555555u;
 }
 
+// ---- one block per thread ----
+
+// The pairs of orderings in the order in which lane_scan walks them - last end from 16 down to 0, second end, first end in
+// steps of two: last << 10 | second << 5 | first of the pair's first ordering; the other has the next first end. The walk
+// for n colours begins at start[n].
+constexpr int kLaneWords = 33;  // of 16 pairs
+struct LanePairs {
+    uint16_t four[16 * kLaneWords], three[96];
+    uint16_t start4[17], start3[17];
+};
+inline void lane_pairs(LanePairs &out) {
+    int n4 = 0, n3 = 0;
+    for (int c2 = 16; c2 >= 0; c2--) {
+        out.start4[c2] = (uint16_t)n4;
+        out.start3[c2] = (uint16_t)n3;
+        for (int c1 = 0; c1 <= c2; c1++)
+            for (int c0 = 0; c0 <= c1; c0 += 2) out.four[n4++] = (uint16_t)(c2 << 10 | c1 << 5 | c0);
+        for (int c0 = 0; c0 <= c2; c0 += 2) out.three[n3++] = (uint16_t)(c2 << 10 | c2 << 5 | c0);
+    }
+}
+
+// A thread's words of a [k][thread] array in shared memory.
+__device__ __forceinline__ uint32_t load_word(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void store_word(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+
+// The scan of a block's orderings by one thread, scan_rows' arithmetic on pairs that differ in the first end only, so that
+// two of the three table entries stay in registers. `table`: the thread's summed-area table (17 entries, 16 T bytes apart);
+// `words`: its flags (4 T bytes apart): bit 2 i + h for ordering h of a word's pair i, set where the ordering's scanned error
+// is within `slack` of the lowest so far or it is hard. `start`: the walk's first pair; `last`: the lowest last end. Returns
+// the number of words, from start / 16 on.
+template <bool UNIT, int T>
+__device__ __noinline__ int lane_scan(uint32_t table, uint32_t words, float mux, float muy, float muz, float W, float eta,
+                                        float slack, int n, int start, int last, float k, float3 metric) {
+    const uint32_t stride = 16 * T;
+    const float kW = k * W, cm = 0.5f * kW, ca = rcp_approx(kW), cd = 0.5f * ca;
+    const float u0 = 2.0f * k - 1.0f;
+    const float inf = __int_as_float(0x7f800000);
+    const float magic = 12582912.0f;
+    const f32x2 magic2 = f2_dup(magic), g31 = f2_dup(31.0f), g63 = f2_dup(63.0f);
+    const float mu[3] = {mux, muy, muz}, mt[3] = {metric.x, metric.y, metric.z};
+    float best = inf;
+    uint32_t bits = 0;
+    int pos = 2 * (start & 15), done = start >> 4;
+    words += 4 * T * (uint32_t)done;
+    const bool three = k == 2.0f;
+#pragma unroll 1
+    for (int c2 = n; c2 >= last; c2--) {
+        const float4 p2 = load_shared(table + c2 * stride);
+#pragma unroll 1
+        for (int c1 = three ? c2 : 0; c1 <= c2; c1++) {
+            const float4 p1 = three ? make_float4(0, 0, 0, 0) : load_shared(table + c1 * stride);
+            const float bx = p1.x + p2.x, by = p1.y + p2.y, bz = p1.z + p2.z, bw = -p1.w - p2.w;
+            const float qb = __fmaf_rn(3.0f, p1.w, p2.w);
+            uint32_t at = table;
+#pragma unroll 1
+            for (int c0 = 0; c0 <= c1; c0 += 2, at += 2 * stride) {
+                // the pair's second entry may lie one past the row's last (or on the flags): read, not used
+                const float4 r0 = load_shared(at), r1 = load_shared(at + stride);
+                const f32x2 nA = f2_pack(bw - r0.w, bw - r1.w), q = f2_pack(__fmaf_rn(u0, r0.w, qb), __fmaf_rn(u0, r1.w, qb));
+                const f32x2 v[3] = {f2_fma(nA, f2_dup(mux), f2_pack(r0.x + bx, r1.x + bx)), f2_fma(nA, f2_dup(muy), f2_pack(r0.y + by, r1.y + by)),
+                                    f2_fma(nA, f2_dup(muz), f2_pack(r0.z + bz, r1.z + bz))};
+                const f32x2 nD = f2_fma(nA, nA, f2_mul(q, f2_dup(-W)));
+                float d0, d1;
+                f2_unpack(nD, d0, d1);
+                const float rn0 = rcp_approx(d0), rn1 = rcp_approx(d1);
+                const f32x2 cD = f2_mul(nD, f2_dup(-cd)), rn2 = f2_pack(rn0, rn1);
+                float nA0, nA1, nB0, nB1;
+                f2_unpack(nA, nA0, nA1);
+                f2_unpack(f2_sub(f2_dup(-kW), nA), nB0, nB1);
+                const f32x2 nal = f2_mul(nA, f2_dup(ca));
+                float far0 = 0.0f, far1 = 0.0f;
+                f32x2 mm, gd;
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    const f32x2 grid = c == 1 ? g63 : g31;
+                    const float st = c == 1 ? 1.0f / 63.0f : 1.0f / 31.0f;
+                    float w0, w1;
+                    f2_unpack(f2_mul(v[c], rn2), w0, w1);
+                    const f32x2 ea = f2_pack(fma_sat(nB0, w0, mu[c]), fma_sat(nB1, w1, mu[c]));
+                    const f32x2 eb = f2_pack(fma_sat(-nA0, w0, mu[c]), fma_sat(-nA1, w1, mu[c]));
+                    const f32x2 na = f2_sub(magic2, f2_fma(ea, grid, magic2)), nb = f2_sub(magic2, f2_fma(eb, grid, magic2));
+                    float fa0, fa1, fb0, fb1;
+                    f2_unpack(f2_fma(ea, grid, na), fa0, fa1);
+                    f2_unpack(f2_fma(eb, grid, nb), fb0, fb1);
+                    far0 = max3_abs(far0, fa0, fb0);
+                    far1 = max3_abs(far1, fa1, fb1);
+                    const f32x2 nd = f2_mul(f2_sub(na, nb), f2_dup(st));
+                    const f32x2 mc = f2_fma(nal, nd, f2_fma(nb, f2_dup(-st), f2_dup(-mu[c]))), gc = f2_fma(cD, nd, v[c]);
+                    const f32x2 mw = UNIT ? mc : f2_mul(mc, f2_dup(mt[c])), gw = UNIT ? gc : f2_mul(gc, f2_dup(mt[c]));
+                    mm = c == 0 ? f2_mul(mw, mc) : f2_fma(mw, mc, mm);
+                    gd = c == 0 ? f2_mul(gw, nd) : f2_fma(gw, nd, gd);
+                }
+                float e0, e1;
+                f2_unpack(f2_fma(f2_dup(cm), mm, gd), e0, e1);
+                const bool h0 = !(far0 <= __fmaf_rn(-eta, fabsf(rn0), 0.4999f));
+                const bool h1 = !(far1 <= __fmaf_rn(-eta, fabsf(rn1), 0.4999f)), second = c0 < c1;
+                best = fminf(best, fminf(h0 ? inf : e0, h1 || !second ? inf : e1));
+                const float limit = best + slack;
+                if (h0 || e0 <= limit) bits |= 1u << pos;
+                if (second && (h1 || e1 <= limit)) bits |= 2u << pos;
+                pos += 2;
+                if (pos == 32) {
+                    store_word(words, bits);
+                    words += 4 * T;
+                    done++;
+                    bits = 0; pos = 0;
+                }
+            }
+        }
+    }
+    if (pos) {
+        store_word(words, bits);
+        done++;
+    }
+    return done;
+}
+
 }  // namespace ntg

@@ -90,3 +90,13 @@ def test_blocks_per_warp(ctx, oracle, fmt, blocks):
         img = contents(kind, w, h, blocks + len(kind))
         got = ctx.encode(fmt, torch.from_numpy(img).cuda(), w, h, quality=1, alpha_mode=1)
         assert np.array_equal(got.cpu().numpy(), image(img, w, h, 1, 1, threads=8)), kind
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_bc1_one_block_per_thread(ctx, oracle, kind):
+    """BC1 launches of 150,000 blocks and more, an odd count of them, against the oracle."""
+    w, h = 4, 4 * 150001
+    img = contents(kind, w, h, 77)
+    for alpha, cw in [(1, (1, 1, 1)), (0, (0.6, 1.0, 0.4))]:
+        got = ctx.encode(ntg.FORMAT_BC1, torch.from_numpy(img).cuda(), w, h, quality=1, alpha_mode=alpha, cw=cw)
+        assert np.array_equal(got.cpu().numpy(), oracle.bc1_image(img, w, h, alpha, 1, cw=cw, threads=16)), alpha
