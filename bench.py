@@ -75,21 +75,20 @@ PROPOSAL_TRAINING = {1: (0, 1, 2), 4: (3, 4)}
 INF = float("inf")
 BATCH_FRONTIER = [{1: (DESCENT | 4, INF)}, {1: (DESCENT | 8, 0.05)}, {1: (DESCENT | 4, INF), 4: (2, INF)},
                   {1: (2, INF)}]
-# DRAM bytes per block of the BC1 fit: one ncu capture of k_bc1<7> over 262,144 blocks of a 2048x2048
-# planar FP32 level (67,384,064 B read + 712,192 B written, profiles/k_bc1_7_cases_2048.md), per block;
+# DRAM bytes per block of the BC1 fit: one ncu capture of k_bc1_lane over 262,144 blocks of a 2048x2048
+# planar FP32 level (67.40 MB read + 1.79 MB written, profiles/k_bc1_lane_cases_2048.md), per block;
 # the batch's BC1 levels are planar FP32 too, so the traffic scales with the blocks
 # DRAM bytes (read + write) of the 4096 x 4096 chain's mip launches (k_tile2x_u8, 6 k_tile2x, k_mip_tail)
 # in one ncu capture of `bench.py --workload c1` (dram__bytes_read.sum + dram__bytes_write.sum).
 C1_MIP_TRAFFIC = 191867392
-BC1_TRAFFIC_PER_BLOCK = (67384064 + 712192) / 262144
+BC1_TRAFFIC_PER_BLOCK = (67400000 + 1790000) / 262144
 
-# FP32 operations of one ordering of icbc's cluster fits (src/nvtt/icbc.h:2501-2540 and 2200-2240 in
-# the scalar build), each multiply/add/min/max/round/reciprocal counted once: cluster_fit_four w3 1,
-# cluster differences 8, alpha2 4, beta2 4, alphabeta 2, alphax 12 = 31, cluster_fit_three 14, then
-# the shared solve/snap/residual: factor 4, betax 3, a 12, b 12, saturate + 5:6:5 rounding 36, e2 18,
-# e1 18, metric 5, compare 1 = 109.
-OPS_PER_ORDERING4 = 140
-OPS_PER_ORDERING3 = 123
+# FP32 instructions of one ordering in the BC1 fit's scan (lane_scan), a fused multiply-add counted once: cluster sums 4,
+# their weights 2, centring 3, D 2 and its reciprocal 1, its multiples 3, per channel 18 (the least-squares end
+# points 3, their snapping 4 and its distances 4, end point difference 2, error terms 5), the error 1, the test of
+# the distances 2, the lowest error 2, compares 2 = 76. The exact evaluations of the few possible winners are not counted.
+OPS_PER_ORDERING4 = 76
+OPS_PER_ORDERING3 = 76
 
 # FP32 operations of one cluster-split evaluation of squish's WeightedClusterFit::Compress4
 # (src/nvtt/squish/weightedclusterfit.cpp:505-545) as the kernel's inner loop runs it, each
@@ -775,7 +774,7 @@ def run_gpu_batch(args):
         roof = None
         if dominant == "bc1" and phases["bc1"] > 0:
             # the BC1 Level8 fit against the FP32 peak: orderings counted on the device by the same
-            # gather / reduce_colors the encoder runs, times the FP32 operations of one ordering
+            # gather / reduce_colors the encoder runs, times the FP32 instructions of one in the scan
             n4, n3 = batch.count_work()
             sm_mhz_b = clocks["sm_mhz"] or 2070.0
             peak_b = 152 * 128 * sm_mhz_b * 1e6
@@ -785,11 +784,11 @@ def run_gpu_batch(args):
             roof = {"bound": "fp32", "achieved": ach / 1e12, "peak": peak_b / 1e12, "unit": "TFLOP/s",
                     "frac": ach / peak_b,
                     "traffic": BC1_TRAFFIC_PER_BLOCK * nb1 if nb1 and BC1_TRAFFIC_PER_BLOCK else None,
-                    "kernel": "k_bc1<7> (icbc Level8 cluster fit)",
+                    "kernel": "k_bc1_lane (icbc Level8 cluster fit)",
                     "note": f"peak = 152 SMs x 128 FP32 lanes x median SM clock {sm_mhz_b:.0f} MHz; {n4} four-cluster x "
-                            f"{OPS_PER_ORDERING4} + {n3} three-cluster x {OPS_PER_ORDERING3} FP32 ops over the BC1 phase "
+                            f"{OPS_PER_ORDERING4} + {n3} three-cluster x {OPS_PER_ORDERING3} FP32 instructions of the scan over the BC1 phase "
                             f"({phases['bc1']:.3f} ms, one run outside the graph, CUDA events); traffic: DRAM bytes per "
-                            f"block of one ncu capture of k_bc1<7>, times the blocks"}
+                            f"block of one ncu capture of k_bc1_lane, times the blocks"}
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": dev_ms / args.steps, "higher_is_better": True,
                 "scaling": "strong" if world > 1 else "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
