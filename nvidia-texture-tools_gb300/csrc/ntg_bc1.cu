@@ -140,26 +140,6 @@ __device__ uint32_t indices3(const Lane<float4> &in, f3 cw, bool allow_black, co
     return idx;
 }
 
-// compute_indices, live branch (src/nvtt/icbc.h:2885-2941)
-__device__ uint32_t indices_any(const Lane<float4> &in, f3 cw, const Pal3 &pal) {
-    f3 p0 = pal.p[0] * cw, p1 = pal.p[1] * cw, p2 = pal.p[2] * cw, p3 = pal.p[3] * cw;
-    uint32_t idx = 0;
-#pragma unroll 4
-    for (int i = 0; i < 16; i++) {
-        f3 c = xyz(in[i]) * cw;
-        f3 t;
-        t = c - p0; float d0 = dot(t, t);
-        t = c - p1; float d1 = dot(t, t);
-        t = c - p2; float d2 = dot(t, t);
-        t = c - p3; float d3 = dot(t, t);
-        unsigned i1 = (d1 <= d0) & (d1 < d2) & (d1 < d3);
-        unsigned i2 = (d2 <= d0) & (d2 <= d1) & (d2 < d3);
-        unsigned i3 = (d3 <= d0) & (d3 <= d1) & (d3 <= d2);
-        idx |= (((i2 | i3) << 1) | (i1 | i3)) << (2 * i);
-    }
-    return idx;
-}
-
 // evaluate_mse over the input texels (src/nvtt/icbc.h:2733-2756)
 template <typename W>
 __device__ float block_mse(const Lane<float4> &in, const W &wi, f3 cw, const Pal3 &pal, uint32_t idx) {
@@ -195,13 +175,6 @@ __device__ float output_block3(const Lane<float4> &in, const W &wi, f3 cw, bool 
     palette_f(c0, c1, pal);
     o.c0 = c0; o.c1 = c1;
     o.idx = indices3(in, cw, allow_black, pal);
-    return block_mse(in, wi, cw, pal, o.idx);
-}
-
-template <typename W>
-__device__ __forceinline__ float mse_of(const Lane<float4> &in, const W &wi, f3 cw, const Block1 &o) {
-    Pal3 pal;
-    palette_f(o.c0, o.c1, pal);
     return block_mse(in, wi, cw, pal, o.idx);
 }
 
@@ -499,32 +472,6 @@ __device__ __forceinline__ float fit_eval(bool four, float4 v0, float4 v1, float
     return cf_eval(ax, p3(xyz(s)), a2, b2, ab, metric, a, b);
 }
 
-// refine_endpoints (src/nvtt/icbc.h:3329-3406), including the reference's use of the current
-// output's palette (not the candidate's) for index selection.
-template <typename W>
-__device__ float refine_endpoints(const Lane<float4> &in, const W &wi, f3 cw, float err, Block1 &o) {
-    const int8_t deltas[16][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {-1, 0, 0}, {0, -1, 0}, {0, 0, -1},
-                                  {1, 1, 0}, {1, 0, 1}, {0, 1, 1}, {-1, -1, 0}, {-1, 0, -1}, {0, -1, -1},
-                                  {-1, 1, 0}, {1, -1, 0}, {0, -1, 1}, {0, 1, -1}};
-    float best = err;
-    int last = 0;
-    for (int i = 0; i < 256; i++) {
-        Block1 r = o;
-        const int8_t *d = deltas[i % 16];
-        unsigned c = ((i / 16) & 1) ? r.c0 : r.c1;
-        unsigned cr = ((c >> 11) + d[0]) & 31, cg = (((c >> 5) & 63) + d[1]) & 63, cb = ((c & 31) + d[2]) & 31;
-        c = (cr << 11) | (cg << 5) | cb;
-        if ((i / 16) & 1) r.c0 = c; else r.c1 = c;
-        Pal3 pal;
-        palette_f(o.c0, o.c1, pal);
-        r.idx = indices_any(in, cw, pal);
-        float e = mse_of(in, wi, cw, r);
-        if (e < best) { best = e; o = r; last = i; }
-        if (i - last > 32) break;
-    }
-    return best;
-}
-
 __device__ __forceinline__ void store_block(uint8_t *dst, const Block1 &o) {
     uint2 v;
     v.x = (o.c0 & 0xFFFF) | (o.c1 << 16);
@@ -705,7 +652,7 @@ __global__ void __launch_bounds__(64) k_bc1_box(const EncJob *__restrict__ jobs,
 // each). One thread per block, every ordering evaluated exactly (165 instructions each), needed 117,000 blocks to
 // fill the GPU; here a 64x64 chain's 341 blocks spread over the SMs. One float level, before and after: 64x64 75
 // and 24 us (8 lanes per block before), 256x256 75 and 34, 1024x1024 416 and 316, 2048x2048 1,317 and 1,228,
-// 1024x1024 after toSrgb 503 and 360 (texels gathered once instead of three times), 512x512 at Level9 627 and 200.
+// 1024x1024 after toSrgb 503 and 360 (texels gathered once instead of three times), 512x512 at Level9 627 and 168.
 
 // reduce_colors (src/nvtt/icbc.h:1638-1683): the texels in order, each matched against the colours so far, which the
 // half's lanes hold one each. Returns the colour count.
@@ -889,8 +836,8 @@ __device__ __forceinline__ float half_output(const Half &H, float4 texel, f3 cw,
 }
 
 // refine_endpoints (src/nvtt/icbc.h:3329-3406), including the reference's use of the current output's palette
-// (not the candidate's) for index selection (compute_indices, live branch, src/nvtt/icbc.h:2885-2941). `run`: this
-// half's block takes part.
+// (not the candidate's) for index selection (compute_indices, live branch, src/nvtt/icbc.h:2885-2941): the indices change
+// with an improvement only, and a trial is its palette and its error. `run`: this half's block takes part.
 __device__ __forceinline__ float half_refine(const Half &H, float4 texel, f3 cw, float err, Block1 &o, bool run) {
     const int8_t deltas[16][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {-1, 0, 0}, {0, -1, 0}, {0, 0, -1},
                                   {1, 1, 0}, {1, 0, 1}, {0, 1, 1}, {-1, -1, 0}, {-1, 0, -1}, {0, -1, -1},
@@ -898,14 +845,8 @@ __device__ __forceinline__ float half_refine(const Half &H, float4 texel, f3 cw,
     float best = err;
     int last = 0;
     const f3 c = xyz(texel) * cw;
-#pragma unroll 1
-    for (int i = 0; i < 256; i++) {
-        Block1 r = o;
-        const int8_t *d = deltas[i % 16];
-        unsigned e = ((i / 16) & 1) ? r.c0 : r.c1;
-        const unsigned er = ((e >> 11) + d[0]) & 31, eg = (((e >> 5) & 63) + d[1]) & 63, eb = ((e & 31) + d[2]) & 31;
-        e = (er << 11) | (eg << 5) | eb;
-        if ((i / 16) & 1) r.c0 = e; else r.c1 = e;
+    unsigned code, idx;
+    auto index = [&]() {
         Pal3 pal;
         palette_half(o.c0, o.c1, pal);
         f3 t;
@@ -917,13 +858,27 @@ __device__ __forceinline__ float half_refine(const Half &H, float4 texel, f3 cw,
         const unsigned i2 = (d2 <= d0) & (d2 <= d1) & (d2 < d3);
         const unsigned i3 = (d3 <= d0) & (d3 <= d1) & (d3 <= d2);
         const unsigned hi = i2 | i3, lo = i1 | i3;
-        r.idx = (spread_bits(H.ballot(hi)) << 1) | spread_bits(H.ballot(lo));
+        code = (hi << 1) | lo;
+        idx = (spread_bits(H.ballot(hi)) << 1) | spread_bits(H.ballot(lo));
+    };
+    index();
+#pragma unroll 1
+    for (int i = 0; i < 256; i++) {
+        Block1 r = o;
+        const int8_t *d = deltas[i % 16];
+        unsigned e = ((i / 16) & 1) ? r.c0 : r.c1;
+        const unsigned er = ((e >> 11) + d[0]) & 31, eg = (((e >> 5) & 63) + d[1]) & 63, eb = ((e & 31) + d[2]) & 31;
+        e = (er << 11) | (eg << 5) | eb;
+        if ((i / 16) & 1) r.c0 = e; else r.c1 = e;
+        r.idx = idx;
         Pal3 rp;
         palette_half(r.c0, r.c1, rp);
-        const float x = half_mse(H, texel, cw, rp, (hi << 1) | lo);
-        if (run && x < best) { best = x; o = r; last = i; }
+        const float x = half_mse(H, texel, cw, rp, code);
+        const bool better = run && x < best;
+        if (better) { best = x; o = r; last = i; }
         if (i - last > 32) run = false;
         if (!__any_sync(kAll, run)) break;
+        if (__any_sync(kAll, better)) index();
     }
     return best;
 }
