@@ -805,6 +805,25 @@ __device__ __forceinline__ float half_mse(const Half &H, float4 texel, f3 cw, co
     return err;
 }
 
+// The same for two palettes.
+__device__ __forceinline__ void half_mse2(const Half &H, float4 texel, f3 cw, const Pal3 &pa, const Pal3 &pb, unsigned code, float &ea,
+                                          float &eb) {
+    const f3 a = code == 0 ? pa.p[0] : (code == 1 ? pa.p[1] : (code == 2 ? pa.p[2] : pa.p[3]));
+    const f3 b = code == 0 ? pb.p[0] : (code == 1 ? pb.p[1] : (code == 2 ? pb.p[2] : pb.p[3]));
+    const f3 da = ((a - xyz(texel)) * cw) * 255.0f, db = ((b - xyz(texel)) * cw) * 255.0f;
+    __syncwarp();
+    H.s->stage[H.hl] = texel.w * dot(da, da);
+    H.s->stage[16 + H.hl] = texel.w * dot(db, db);
+    __syncwarp();
+    ea = eb = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float4 s = reinterpret_cast<const float4 *>(H.s->stage)[i], t = reinterpret_cast<const float4 *>(H.s->stage)[4 + i];
+        ea += s.x; ea += s.y; ea += s.z; ea += s.w;
+        eb += t.x; eb += t.y; eb += t.z; eb += t.w;
+    }
+}
+
 // output_block4 / output_block3 (compute_indices4 / compute_indices3, src/nvtt/icbc.h:2803-2882).
 template <bool FOUR>
 __device__ __forceinline__ float half_output(const Half &H, float4 texel, f3 cw, f3 v0, f3 v1, Block1 &o) {
@@ -862,8 +881,7 @@ __device__ __forceinline__ float half_refine(const Half &H, float4 texel, f3 cw,
         idx = (spread_bits(H.ballot(hi)) << 1) | spread_bits(H.ballot(lo));
     };
     index();
-#pragma unroll 1
-    for (int i = 0; i < 256; i++) {
+    auto trial = [&](int i) {
         Block1 r = o;
         const int8_t *d = deltas[i % 16];
         unsigned e = ((i / 16) & 1) ? r.c0 : r.c1;
@@ -871,14 +889,31 @@ __device__ __forceinline__ float half_refine(const Half &H, float4 texel, f3 cw,
         e = (er << 11) | (eg << 5) | eb;
         if ((i / 16) & 1) r.c0 = e; else r.c1 = e;
         r.idx = idx;
-        Pal3 rp;
-        palette_half(r.c0, r.c1, rp);
-        const float x = half_mse(H, texel, cw, rp, code);
+        return r;
+    };
+    // True where an error below the best is found; the block takes it.
+    auto take = [&](int i, const Block1 &r, float x) {
         const bool better = run && x < best;
         if (better) { best = x; o = r; last = i; }
         if (i - last > 32) run = false;
+        return __any_sync(kAll, better) != 0;
+    };
+    // two trials at a time: the second holds unless the first improves one of the blocks, and is tried again then
+#pragma unroll 1
+    for (int i = 0; i < 256;) {
+        const Block1 r0 = trial(i), r1 = trial(i + 1);
+        Pal3 p0, p1;
+        palette_half(r0.c0, r0.c1, p0);
+        palette_half(r1.c0, r1.c1, p1);
+        float x0, x1;
+        half_mse2(H, texel, cw, p0, p1, code, x0, x1);
+        bool better = take(i++, r0, x0);
         if (!__any_sync(kAll, run)) break;
-        if (__any_sync(kAll, better)) index();
+        if (!better && i < 256) {
+            better = take(i++, r1, x1);
+            if (!__any_sync(kAll, run)) break;
+        }
+        if (better) index();
     }
     return best;
 }
