@@ -652,7 +652,7 @@ __global__ void __launch_bounds__(64) k_bc1_box(const EncJob *__restrict__ jobs,
 // each). One thread per block, every ordering evaluated exactly (165 instructions each), needed 117,000 blocks to
 // fill the GPU; here a 64x64 chain's 341 blocks spread over the SMs. One float level, before and after: 64x64 75
 // and 24 us (8 lanes per block before), 256x256 75 and 34, 1024x1024 416 and 316, 2048x2048 1,317 and 1,228,
-// 1024x1024 after toSrgb 503 and 360 (texels gathered once instead of three times), 512x512 at Level9 627 and 168.
+// 1024x1024 after toSrgb 503 and 360 (texels gathered once instead of three times), 512x512 at Level9 627 and 154.
 
 // reduce_colors (src/nvtt/icbc.h:1638-1683): the texels in order, each matched against the colours so far, which the
 // half's lanes hold one each. Returns the colour count.
@@ -805,11 +805,20 @@ __device__ __forceinline__ float half_mse(const Half &H, float4 texel, f3 cw, co
     return err;
 }
 
-// The same for two palettes.
-__device__ __forceinline__ void half_mse2(const Half &H, float4 texel, f3 cw, const Pal3 &pa, const Pal3 &pb, unsigned code, float &ea,
-                                          float &eb) {
-    const f3 a = code == 0 ? pa.p[0] : (code == 1 ? pa.p[1] : (code == 2 ? pa.p[2] : pa.p[3]));
-    const f3 b = code == 0 ? pb.p[0] : (code == 1 ? pb.p[1] : (code == 2 ? pb.p[2] : pb.p[3]));
+// Entry `code` of a block's palette; `unit8` is c_unit8 in shared memory, where lanes may read different entries at once.
+__device__ __forceinline__ f3 palette_entry(const Block1 &o, unsigned code, const float *unit8) {
+    Pal8 p;
+    palette_d3d10(o.c0, o.c1, p);
+    const int r = code == 0 ? p.r[0] : (code == 1 ? p.r[1] : (code == 2 ? p.r[2] : p.r[3]));
+    const int g = code == 0 ? p.g[0] : (code == 1 ? p.g[1] : (code == 2 ? p.g[2] : p.g[3]));
+    const int b = code == 0 ? p.b[0] : (code == 1 ? p.b[1] : (code == 2 ? p.b[2] : p.b[3]));
+    return mk3(unit8[r], unit8[g], unit8[b]);
+}
+
+// The same for the end points of two trials.
+__device__ __forceinline__ void half_mse2(const Half &H, float4 texel, f3 cw, const Block1 &ra, const Block1 &rb, unsigned code,
+                                          const float *unit8, float &ea, float &eb) {
+    const f3 a = palette_entry(ra, code, unit8), b = palette_entry(rb, code, unit8);
     const f3 da = ((a - xyz(texel)) * cw) * 255.0f, db = ((b - xyz(texel)) * cw) * 255.0f;
     __syncwarp();
     H.s->stage[H.hl] = texel.w * dot(da, da);
@@ -857,7 +866,7 @@ __device__ __forceinline__ float half_output(const Half &H, float4 texel, f3 cw,
 // refine_endpoints (src/nvtt/icbc.h:3329-3406), including the reference's use of the current output's palette
 // (not the candidate's) for index selection (compute_indices, live branch, src/nvtt/icbc.h:2885-2941): the indices change
 // with an improvement only, and a trial is its palette and its error. `run`: this half's block takes part.
-__device__ __forceinline__ float half_refine(const Half &H, float4 texel, f3 cw, float err, Block1 &o, bool run) {
+__device__ __forceinline__ float half_refine(const Half &H, float4 texel, f3 cw, float err, Block1 &o, bool run, const float *unit8) {
     const int8_t deltas[16][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {-1, 0, 0}, {0, -1, 0}, {0, 0, -1},
                                   {1, 1, 0}, {1, 0, 1}, {0, 1, 1}, {-1, -1, 0}, {-1, 0, -1}, {0, -1, -1},
                                   {-1, 1, 0}, {1, -1, 0}, {0, -1, 1}, {0, 1, -1}};
@@ -898,15 +907,14 @@ __device__ __forceinline__ float half_refine(const Half &H, float4 texel, f3 cw,
         if (i - last > 32) run = false;
         return __any_sync(kAll, better) != 0;
     };
-    // two trials at a time: the second holds unless the first improves one of the blocks, and is tried again then
+    // Two trials at a time: the second holds unless the first improves one of the blocks, and is tried again then. Bound by
+    // latency, a palette and a serial sum of 16 terms per trial. 640x360 level: 205 us with the indices computed for every
+    // trial, 174 without, 161 with two at a time, 154 with the palette's table in shared memory.
 #pragma unroll 1
     for (int i = 0; i < 256;) {
         const Block1 r0 = trial(i), r1 = trial(i + 1);
-        Pal3 p0, p1;
-        palette_half(r0.c0, r0.c1, p0);
-        palette_half(r1.c0, r1.c1, p1);
         float x0, x1;
-        half_mse2(H, texel, cw, p0, p1, code, x0, x1);
+        half_mse2(H, texel, cw, r0, r1, code, unit8, x0, x1);
         bool better = take(i++, r0, x0);
         if (!__any_sync(kAll, run)) break;
         if (!better && i < 256) {
@@ -949,6 +957,11 @@ __global__ void __launch_bounds__(32 * kFitWarps, NTG_BC1_MIN_CTAS) k_bc1(const 
                                                                          const unsigned long long *__restrict__ count,
                                                                          int per_warp) {
     __shared__ WarpScratch scratch[kFitWarps];
+    __shared__ float unit8[LEVEL == 8 ? 256 : 1];
+    if (LEVEL == 8) {
+        for (int i = threadIdx.x; i < 256; i += 32 * kFitWarps) unit8[i] = c_unit8[i];
+        __syncthreads();
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     WarpScratch &w = scratch[warp];
     const Half H{lane & 15, lane & 16, &w.half[lane >> 4]};
@@ -1005,7 +1018,7 @@ __global__ void __launch_bounds__(32 * kFitWarps, NTG_BC1_MIN_CTAS) k_bc1(const 
     Block1 o{0, 0, 0};
     float err = FLT_MAX;
     if (cerr < err) { o = cf; err = cerr; }
-    if (LEVEL == 8) err = half_refine(H, texel, cw, err, o, fit);
+    if (LEVEL == 8) err = half_refine(H, texel, cw, err, o, fit, unit8);
     if (fit && H.hl == 0) store_block(out, o);
 }
 
