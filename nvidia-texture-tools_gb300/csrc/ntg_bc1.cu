@@ -4,8 +4,9 @@
 //   Quality_Normal     -> icbc Level8: 4- and 3-colour cluster fit over all orderings
 //   Quality_Production -> icbc Level9: Level8 + endpoint refinement
 // The cluster fits (k_bc1) take two blocks per warp and search one block's orderings with all its lanes,
-// through the scan of ntg_scan.cuh; Level1 (k_bc1_box) and the learned path's kernels take one block per
-// thread, the block's texels, reduced colours and summed-area table in shared memory.
+// through the scan of ntg_scan.cuh, or in large launches scan one block per lane (k_bc1_lane); Level1
+// (k_bc1_box) and the learned path's kernels take one block per thread, the block's texels, reduced
+// colours and summed-area table in shared memory.
 // Built with --fmad=false: results are bit-identical to the reference's scalar build.
 #include <memory>
 
@@ -651,7 +652,7 @@ __global__ void __launch_bounds__(64) k_bc1_box(const EncJob *__restrict__ jobs,
 // Bound by the FMA pipe: 19 rows of 64 orderings at about 112 instructions a row, half of them packed (two cycles
 // each). One thread per block, every ordering evaluated exactly (165 instructions each), needed 117,000 blocks to
 // fill the GPU; here a 64x64 chain's 341 blocks spread over the SMs. One float level, before and after: 64x64 75
-// and 24 us (8 lanes per block before), 256x256 75 and 34, 1024x1024 416 and 316, 2048x2048 1,317 and 1,228,
+// and 21 us (8 lanes per block before), 256x256 75 and 35, 1024x1024 418 and 323, 2048x2048 1,317 and 1,232,
 // 1024x1024 after toSrgb 503 and 360 (texels gathered once instead of three times), 512x512 at Level9 627 and 154.
 
 // reduce_colors (src/nvtt/icbc.h:1638-1683): the texels in order, each matched against the colours so far, which the

@@ -12,8 +12,8 @@ no fallback (the pruned search's cost does not depend on the proposal's quality)
   mips_tma           k_tile2x_f32                                (one Kaiser 2:1 step from a 2N x N FP32 level)
   mips_odd           k_poly, k_mip_tail                          (odd sizes: the general scale kernel)
   mips_box           k_set_image, k_fast_down                    (box filter)
-  bc1                k_bc1<7> (Normal)     bc1_fastest  k_bc1_box   bc1_production  k_bc1<8>
-  bc3                k_bc3<1>              bc1a         k_bc1a       bc4  k_bc4<1>    bc5  k_bc5<1>
+  bc1                k_bc1_lane (Normal; k_bc1<7> with --size 1024)   bc1_fastest  k_bc1_box   bc1_production  k_bc1<8>
+  bc3                k_bc3<1> (k_squish<0> with --size 512)   bc1a  k_bc1a   bc4  k_bc4<1>   bc5  k_bc5<1>
   decode_rms         k_decode, k_error_sums
   learned_bc1        chain mips, k_bc1_features, k_mlp_infer, k_bc1_learned, k_bc1<7> over the list
   learned_bc3        chain mips, k_bc3_features, k_mlp_infer, k_bc3_learned, k_bc3<1> over the list
