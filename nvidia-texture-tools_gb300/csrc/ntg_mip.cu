@@ -187,7 +187,7 @@ __global__ void k_fast_down(const MipJob *__restrict__ jobs, int njobs, long lon
                 v[0] = s_lut[(p >> 16) & 255]; v[1] = s_lut[(p >> 8) & 255]; v[2] = s_lut[p & 255]; v[3] = s_lut[256 + (p >> 24)];
             } else {
 #pragma unroll
-                for (int c = 0; c < 4; c++) v[c] = __ldg(L.src + c * sn + i);
+                for (int c = 0; c < 4; c++) v[c] = load_level(L.src + c * sn + i);
             }
         };
         float v[4];
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(PTHREADS) k_poly(const MipJob *__restrict__ jo
                 const uint32_t p = __ldg(L.bgra8 + s);
                 s_in[r * rx + x] = make_float4(s_lut[(p >> 16) & 255], s_lut[(p >> 8) & 255], s_lut[p & 255], s_lut[256 + (p >> 24)]);
             } else {
-                s_in[r * rx + x] = make_float4(__ldg(L.src + s), __ldg(L.src + sn + s), __ldg(L.src + 2 * sn + s), __ldg(L.src + 3 * sn + s));
+                s_in[r * rx + x] = make_float4(load_level(L.src + s), load_level(L.src + sn + s), load_level(L.src + 2 * sn + s), load_level(L.src + 3 * sn + s));
             }
         }
     }
@@ -424,7 +424,7 @@ template <> struct RawTexel<false> { float4 v; };
 template <bool SRC_U8>
 __device__ __forceinline__ void fetch_raw(const MipJob &L, size_t s, size_t sn, RawTexel<SRC_U8> &r) {
     if constexpr (SRC_U8) r.v = __ldg(L.bgra8 + s);
-    else r.v = make_float4(__ldg(L.src + s), __ldg(L.src + sn + s), __ldg(L.src + 2 * sn + s), __ldg(L.src + 3 * sn + s));
+    else r.v = make_float4(load_level(L.src + s), load_level(L.src + sn + s), load_level(L.src + 2 * sn + s), load_level(L.src + 3 * sn + s));
 }
 
 template <int WS, bool WEIGHTED, bool SRC_U8>
@@ -892,6 +892,8 @@ __global__ void __launch_bounds__(1024, 1) k_tile2x_f32(const MipJob *__restrict
     float kx[WS];
 #pragma unroll
     for (int j = 0; j < WS; j++) kx[j] = __ldg(J0.kx + j);
+    // the source level was written through the generic proxy, by a kernel that may have ended during this one
+    if ((order & EARLY) && tma_issuer()) asm volatile("fence.proxy.async.global;" ::: "memory");
     __syncthreads();  // barriers initialised before any thread waits on them
 
     // iteration i X-filters tile blockIdx + i g (t0, window in buffer i % NB) and Y-filters tile
@@ -1148,7 +1150,7 @@ __global__ void __launch_bounds__(1024) k_mip_tail(const MipJob *__restrict__ jo
         const int n = L.W * L.H;
         for (int i = tid; i < n; i += nt) {
             if (L.src) {
-                lv0[i] = make_float4(__ldg(L.src + i), __ldg(L.src + (size_t)n + i), __ldg(L.src + 2 * (size_t)n + i), __ldg(L.src + 3 * (size_t)n + i));
+                lv0[i] = make_float4(load_level(L.src + i), load_level(L.src + (size_t)n + i), load_level(L.src + 2 * (size_t)n + i), load_level(L.src + 3 * (size_t)n + i));
             } else {
                 const uint32_t q = __ldg(L.bgra8 + i);
                 lv0[i] = make_float4(__ldg(L.lut + ((q >> 16) & 255)), __ldg(L.lut + ((q >> 8) & 255)), __ldg(L.lut + (q & 255)),

@@ -90,3 +90,20 @@ def test_levels(ctx, filt):
                 assert torch.equal(got, ctx.mip_chain(img, w, h, opt)), (w, h, levels)
             finally:
                 ctx.profile(False)
+
+
+@pytest.mark.parametrize("filt", [ntg.FILTER_BOX, ntg.FILTER_TRIANGLE, ntg.FILTER_KAISER])
+def test_levels_sharing_sectors(ctx, filt):
+    """Returned levels whose boundaries fall inside a 32-byte sector (an odd number of texels so far), two images in turn
+    into one buffer, so that a sector read before its level is written still holds the other image's."""
+    for w, h in [(513, 513), (1025, 771), (257, 1027)]:
+        opt = ntg.ChainOptions.make(filter=filt)
+        images = [image(w, h, 2 * w), image(w, h, 2 * w + 1)]
+        ctx.profile(True)
+        try:
+            want = [ctx.mip_chain(i, w, h, opt).clone() for i in images]
+        finally:
+            ctx.profile(False)
+        out = torch.zeros_like(want[0])
+        for k in range(20):
+            assert torch.equal(ctx.mip_chain(images[k & 1], w, h, opt, out=out), want[k & 1]), (w, h, k)
