@@ -66,7 +66,11 @@ typedef struct ntg_context ntg_context;
 /* Per-device state: constant tables, a grow-only scratch workspace and staging buffers.
  * Replaces the reference's CudaContext (src/nvtt/Context.cpp:81-98). The first context on a device
  * also builds that device's sRGB correction tables (about 55 MB of device memory, held until exit);
- * later contexts on the device allocate nothing until their first call that needs scratch. */
+ * later contexts on the device allocate nothing until their first call that needs scratch.
+ * Calls may come from several threads. Those that use the workspace or the job lists (encode, resize,
+ * mip level, chains) run one after the other on the GPU also when their streams differ: a call's
+ * stream waits for the context's previous such call. Calls recorded into a CUDA graph are not part
+ * of that order: a replay must not overlap other calls of the context. */
 int ntg_create(int device, ntg_context **out);
 int ntg_destroy(ntg_context *ctx);
 const char *ntg_last_error_string(void);

@@ -135,6 +135,14 @@ struct XformTables {
 
 }  // namespace
 
+// True while `s` records a graph: a stream that joins the recording stays part of it until it ends, which may be after
+// another call wants the side stream.
+static bool recording(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) { cudaGetLastError(); return true; }
+    return st != cudaStreamCaptureStatusNone;
+}
+
 // A second stream for work that runs beside a call's own, and the events that tie the two: the call's stream waits for it
 // before the call returns, so whatever is ordered after the call is ordered after both. Its priority is the highest, so
 // that the few CTAs of a small launch don't queue behind the thousands of an encoder.
@@ -189,11 +197,14 @@ struct ntg_context {
     bool profile = false;       // record phase events in chain calls
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     SideStream side;            // see Overlap
+    cudaEvent_t used = nullptr;          // see SharedUse
+    unsigned long long used_stream = 0;  // the stream it was recorded on last (its id); 0: not recorded
 
     ~ntg_context() {
         cudaSetDevice(device);
         for (cudaEvent_t e : ev)
             if (e) cudaEventDestroy(e);
+        if (used) cudaEventDestroy(used);
         for (void *p : owned) cudaFree(p);
         if (ws) cudaFree(ws);
         if (d_jobs) cudaFree(d_jobs);
@@ -311,6 +322,35 @@ struct ntg_context {
 };
 
 namespace {
+
+// A call's use of what all calls of a context share on the GPU: the workspace and the job lists, which a call on another
+// stream would overwrite (or free) under the kernels of the one before. From begin() on the call's stream is ordered after
+// every earlier use; the end of the scope marks this one's, whether the call failed or not. Streams are told apart by id: a
+// handle may be that of a stream destroyed since. A stream that records a graph can neither wait for work outside the
+// recording nor mark work that has yet to run: such calls stay out.
+class SharedUse {
+    ntg_context *const ctx;
+    const cudaStream_t s;
+    unsigned long long id = 0;
+    bool active = false;
+
+  public:
+    SharedUse(ntg_context *c, cudaStream_t stream) : ctx(c), s(stream) {}
+    SharedUse(const SharedUse &) = delete;
+    SharedUse &operator=(const SharedUse &) = delete;
+    int begin() {
+        if (recording(s)) return NTG_OK;
+        if (!ctx->used) NTG_CUDA(cudaEventCreateWithFlags(&ctx->used, cudaEventDisableTiming));
+        NTG_CUDA(cudaStreamGetId(s, &id));
+        if (ctx->used_stream && ctx->used_stream != id + 1) NTG_CUDA(cudaStreamWaitEvent(s, ctx->used, 0));
+        active = true;
+        return NTG_OK;
+    }
+    bool is_recording() const { return !active; }  // after begin()
+    ~SharedUse() {
+        if (active && cudaEventRecord(ctx->used, s) == cudaSuccess) ctx->used_stream = id + 1;
+    }
+};
 
 // Largest source window (columns) any PTW-wide run of outputs of this axis can touch.
 int max_window(const AxisTable &t, int tile) {
@@ -774,14 +814,6 @@ Overlap chain_overlap(const ChainPlan &P, const ntg_chain_options &o, size_t tai
     return v;
 }
 
-// True while `s` records a graph: a stream that joins the recording stays part of it until it ends, which may be after
-// another call wants the side stream.
-bool recording(cudaStream_t s) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) { cudaGetLastError(); return true; }
-    return st != cudaStreamCaptureStatusNone;
-}
-
 // Surface::toLinear/toGamma return early for gamma == 1 (nv::equal, src/nvtt/Surface.cpp:1470-1488).
 ntg_chain_options normalized(const ntg_chain_options &o) {
     ntg_chain_options n = o;
@@ -956,6 +988,8 @@ int ntg_mip_level(ntg_context *ctx, const float *d_src, int w, int h, float *d_d
     std::vector<std::vector<MipLaunch>> stages(1);
     group_launches(items, ctx->tune, all, stages[0]);
     cudaStream_t s = S(stream);
+    SharedUse use(ctx, s);
+    NTG_TRY(use.begin());
     NTG_TRY(upload_mip_jobs(ctx, all, s));
     return run_stages(stages, ctx->d_mipjobs, s);
 }
@@ -982,6 +1016,8 @@ int ntg_resize(ntg_context *ctx, const float *d_src, int w, int h, float *d_dst,
     const AxisTable *ax = ctx->axis(filter, fw, p[0], p[1], w, dw);
     const AxisTable *ay = ctx->axis(filter, fw, p[0], p[1], h, dh);
     if (!ax || !ay) return fail(NTG_ERROR_CUDA, "polyphase table upload failed");
+    SharedUse use(ctx, s);
+    NTG_TRY(use.begin());
     uint8_t *tmp = nullptr;
     NTG_TRY(ctx->workspace((size_t)dw * h * 4 * sizeof(float), s, &tmp));
     return launched(launch_resize(d_src, w, h, (float *)tmp, dw, dh, ax->d_w, ax->d_left, ax->ws, ay->d_w, ay->d_left,
@@ -1078,6 +1114,8 @@ int ntg_encode(ntg_context *ctx, int format, const float *d_rgba, int w, int h, 
     std::lock_guard<std::mutex> lk(ctx->mu);
     NTG_TRY(ensure_device(ctx));
     cudaStream_t s = S(stream);
+    SharedUse use(ctx, s);
+    NTG_TRY(use.begin());
     uint32_t *q = nullptr;
     if (format != NTG_FORMAT_BC1 && out_xform != NTG_XFORM_NONE) {
         // the 8-bit formats quantise the transformed level first (ColorBlock::init on the toGamma'd copy)
@@ -1123,10 +1161,12 @@ static int chain_common(ntg_context *ctx, const void *d_bgra, int w, int h, cons
     const ChainPlan P = plan_chain(w, h, *opt, d_levels != nullptr);
     const XformTables *xt = ctx->xform(opt->in_xform, opt->out_xform, opt->gamma);
     if (!xt) return fail(NTG_ERROR_CUDA, "table upload failed");
+    SharedUse use(ctx, s);
+    NTG_TRY(use.begin());
     uint8_t *ws = reinterpret_cast<uint8_t *>(d_levels);  // levels that the call returns are built where they belong
     if (!d_levels) NTG_TRY(ctx->workspace(std::max<size_t>(P.bytes, 256), s, &ws));
     const size_t tail = tail_start(P, ctx->tune);
-    const bool overlap = !ctx->profile && !recording(s);
+    const bool overlap = !ctx->profile && !use.is_recording();
     const Overlap ov = d_blocks && overlap ? chain_overlap(P, *opt, tail) : Overlap();
     if (ov.split) {
         NTG_TRY(ctx->side.create());
@@ -1203,6 +1243,8 @@ static int chain_learned(ntg_context *ctx, ntg_mlp *mlp, const void *d_bgra, int
     const size_t xoff = base, yoff = align256(xoff + (size_t)nb * 48 * 4), loff = align256(yoff + (size_t)nb * 16 * 4),
                  soff = align256(loff + (size_t)nb * 8);
     const size_t need = mode == LEARN_ENCODE ? soff + 256 : base;
+    SharedUse use(ctx, s);
+    NTG_TRY(use.begin());
     uint8_t *ws = nullptr;
     NTG_TRY(ctx->workspace(need, s, &ws));
     NTG_TRY(build_levels(ctx, P, (const uint32_t *)d_bgra, *opt, xt, ws, s));

@@ -107,3 +107,43 @@ def test_levels_sharing_sectors(ctx, filt):
         out = torch.zeros_like(want[0])
         for k in range(20):
             assert torch.equal(ctx.mip_chain(images[k & 1], w, h, opt, out=out), want[k & 1]), (w, h, k)
+
+
+def test_streams_on_one_context(ctx):
+    """Calls on several streams of one context, no synchronisation between them: each waits for the one before, whose
+    workspace and job lists it would overwrite. Small and large calls in turn, so that the workspace and the lists grow (and
+    are freed) under a running call too."""
+    calls = []
+    for k, (w, h, fmt) in enumerate([(1024, 1024, ntg.FORMAT_BC3), (64, 64, ntg.FORMAT_BC1), (1500, 700, ntg.FORMAT_BC1),
+                                     (256, 256, ntg.FORMAT_BC5), (2048, 1024, ntg.FORMAT_BC1), (333, 517, ntg.FORMAT_BC3)]):
+        opt = ntg.ChainOptions.make(format=fmt, filter=ntg.FILTER_KAISER, in_xform=ntg.XFORM_SRGB, out_xform=ntg.XFORM_SRGB)
+        calls.append((image(w, h, k), w, h, opt))
+    want = [serial(ctx, *c) for c in calls]
+    own = ntg.Context(0)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    torch.cuda.synchronize()
+    got = []
+    for k in range(4 * len(calls)):
+        with torch.cuda.stream(streams[k % 3]):
+            got.append(own.compress_chain(*calls[k % len(calls)]))
+    torch.cuda.synchronize()
+    for k, blocks in enumerate(got):
+        assert torch.equal(blocks, want[k % len(calls)]), k
+
+    errors = []
+
+    def work(t):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            for k in range(8):
+                blocks = own.compress_chain(*calls[(k + t) % len(calls)])
+                stream.synchronize()
+                if not torch.equal(blocks, want[(k + t) % len(calls)]):
+                    errors.append((t, k))
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    own.close()
