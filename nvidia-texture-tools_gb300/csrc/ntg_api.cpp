@@ -1163,8 +1163,11 @@ static int chain_common(ntg_context *ctx, const void *d_bgra, int w, int h, cons
     if (!xt) return fail(NTG_ERROR_CUDA, "table upload failed");
     SharedUse use(ctx, s);
     NTG_TRY(use.begin());
-    uint8_t *ws = reinterpret_cast<uint8_t *>(d_levels);  // levels that the call returns are built where they belong
-    if (!d_levels) NTG_TRY(ctx->workspace(std::max<size_t>(P.bytes, 256), s, &ws));
+    // levels that the call returns are built where they belong, unless that is where the image lies, which the filters read
+    const uintptr_t image = (uintptr_t)d_bgra, out = (uintptr_t)d_levels;
+    const bool in_place = d_levels && image < out + P.bytes && out < image + (size_t)w * h * 4;
+    uint8_t *ws = reinterpret_cast<uint8_t *>(d_levels);
+    if (!d_levels || in_place) NTG_TRY(ctx->workspace(std::max<size_t>(P.bytes, 256), s, &ws));
     const size_t tail = tail_start(P, ctx->tune);
     const bool overlap = !ctx->profile && !use.is_recording();
     const Overlap ov = d_blocks && overlap ? chain_overlap(P, *opt, tail) : Overlap();
@@ -1194,6 +1197,7 @@ static int chain_common(ntg_context *ctx, const void *d_bgra, int w, int h, cons
     if (ctx->profile) NTG_CUDA(cudaEventRecord(ctx->ev[0], s));
     NTG_TRY(build_levels(ctx, P, (const uint32_t *)d_bgra, *opt, xt, ws, s, overlap));
     if (ctx->profile) NTG_CUDA(cudaEventRecord(ctx->ev[1], s));
+    if (in_place) NTG_CUDA(cudaMemcpyAsync(d_levels, ws, P.bytes, cudaMemcpyDeviceToDevice, s));
     if (d_blocks) {
         std::vector<EncJob> jobs;
         long long nblocks = 0;

@@ -147,3 +147,18 @@ def test_streams_on_one_context(ctx):
         t.join()
     assert not errors
     own.close()
+
+
+@pytest.mark.parametrize("filt", [ntg.FILTER_BOX, ntg.FILTER_KAISER])
+@pytest.mark.parametrize("where", [0, 1])
+def test_levels_over_the_image(ctx, filt, where):
+    """Levels returned into the buffer that holds the image, at its start or its end."""
+    for w, h in [(64, 64), (65, 33), (512, 300), (1024, 1024)]:
+        img = image(w, h, w + h)
+        opt = ntg.ChainOptions.make(filter=filt)
+        want = ctx.mip_chain(img, w, h, opt)
+        buf = torch.empty_like(want)
+        at = 0 if where == 0 else buf.numel() - w * h
+        inside = buf[at:at + w * h]
+        inside.copy_(img.reshape(-1).view(torch.float32))
+        assert torch.equal(ctx.mip_chain(inside, w, h, opt, out=buf), want), (w, h)
