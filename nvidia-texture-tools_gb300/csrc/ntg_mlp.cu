@@ -950,6 +950,7 @@ int forward(ntg_mlp *m, const float *d_x, int batch, cudaStream_t s) {
 
 // Forward and backward: the batch's loss into m->loss, its gradient into the flat vector m->g.
 int backprop(ntg_mlp *m, const float *d_x, const float *d_t, int batch, cudaStream_t s) {
+    if (batch % 8) return mlp_fail(NTG_ERROR_INVALID_INPUT, "training batches are multiples of 8");
     static std::atomic<unsigned long long> configured{0};
     if (first_use_on_device(configured)) {
         cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F_BYTES);

@@ -31,3 +31,19 @@ def test_gradients_match_oracle(batch, offset):
             assert np.linalg.norm(g[a:b] - ref[a:b]) < 2e-2 * np.linalg.norm(ref[a:b]), (a, b)
     finally:
         net.close()
+
+
+@pytest.mark.parametrize("batch", [1, 5, 129, 257])
+def test_batches_are_multiples_of_eight(batch):
+    """Other batches are refused, as they always were, and leave the network as it was."""
+    net = ntg.MLP(seed=3)
+    try:
+        x, t = torch.rand((batch, 48), device="cuda"), torch.rand((batch, 8), device="cuda")
+        before = net.get_params()
+        for call in (net.gradients, net.train_step):
+            with pytest.raises(ntg.NtgError) as e:
+                call(x, t)
+            assert e.value.code == ntg.NTG_ERROR_INVALID_INPUT
+        assert np.array_equal(net.get_params(), before)
+    finally:
+        net.close()
