@@ -86,25 +86,40 @@ __global__ void __launch_bounds__(128) k_decode(int format, const uint8_t *__res
     }
 }
 
-// A sum of floats kept as an unevaluated pair, exact but for the roundings of `lo` (Knuth's TwoSum): 2^-47 of the sum for a
-// few terms, below what the same terms lose one by one in a long sum of doubles.
-struct PairSum {
-    float hi = 0.0f, lo = 0.0f;
+// A sum of non-negative floats kept as an unevaluated triple, each part the rounding error of the one before it (Knuth's
+// TwoSum): exact but for the roundings of `lo`, 2^-61 of the sum for a step's twelve terms and less for a partial sum that
+// joins another, where each addition in double rounds 2^-53. (A pair lost up to 2^-45 of twelve squares of unlike size.)
+struct TripleSum {
+    float hi = 0.0f, mid = 0.0f, lo = 0.0f;
     __device__ __forceinline__ void add(float x) {
-        const float s = hi + x, t = s - hi;
-        lo += (hi - (s - t)) + (x - t);
+        float s = hi + x, t = s - hi;
+        const float e = (hi - (s - t)) + (x - t);
         hi = s;
+        s = mid + e;
+        t = s - mid;
+        lo += (mid - (s - t)) + (e - t);
+        mid = s;
     }
+    __device__ __forceinline__ void add(const TripleSum &o) {
+        add(o.hi); add(o.mid); add(o.lo);
+        float s = hi + mid;  // the parts apart again, so that `lo` stays below 2^-47 of the sum
+        mid -= s - hi; hi = s;
+        s = mid + lo;
+        lo -= s - mid; mid = s;
+    }
+    __device__ __forceinline__ double value() const { return (double)hi + ((double)mid + (double)lo); }
 };
 
-// Squared-error sums in double, reduced per CTA and accumulated atomically; four texels a step. The terms of a step are
-// summed as pairs of floats first: the double unit takes two additions a clock and SM, and one addition per
-// term (with its conversion) held the kernel to 74 us for 2048x2048 where reading the images takes 20; with a
-// quarter of them it takes 26 us. VEC: planes on 16-byte boundaries.
+// Squared-error sums, reduced per CTA in double and accumulated atomically; four texels a step. A thread's terms are
+// summed as triples of floats: the double unit takes two additions a clock and SM, and one addition per term (with
+// its conversion) held the kernel to 74 us for 2048x2048 where reading the images takes 20. 29 us with the launch and the
+// zeroing before it, 36 with a conversion of every step's triple. VEC: planes on 16-byte boundaries.
 template <bool VEC>
 __global__ void k_error_sums(const float *__restrict__ ref, const float *__restrict__ img, size_t n, int alpha_mode,
                              double *__restrict__ sums) {
+    constexpr float kFar = 1e37f;
     double c = 0, al = 0;
+    TripleSum rc, ra;
     const size_t steps = (n + 3) / 4;
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < steps; q += (size_t)gridDim.x * blockDim.x) {
         float p[4][4], t[4][4];  // [plane][texel] of ref and img
@@ -124,7 +139,7 @@ __global__ void k_error_sums(const float *__restrict__ ref, const float *__restr
             }
         }
         float e[4][4];
-        PairSum cs, as;
+        TripleSum cs, as;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             float wgt = 1;
@@ -139,10 +154,15 @@ __global__ void k_error_sums(const float *__restrict__ ref, const float *__restr
             e[3][j] = da * da;
             as.add(e[3][j]);
         }
-        if (fabsf(cs.hi) <= FLT_MAX && fabsf(as.hi) <= FLT_MAX) {
-            c += (double)cs.hi + (double)cs.lo;
-            al += (double)as.hi + (double)as.lo;
-        } else {  // infinities, NaN, or a sum beyond float's range
+        if (cs.hi <= kFar && as.hi <= kFar) {
+            rc.add(cs);
+            ra.add(as);
+            if (rc.hi > kFar || ra.hi > kFar) {
+                c += rc.value();
+                al += ra.value();
+                rc = ra = TripleSum();
+            }
+        } else {  // infinities, NaN, or sums towards the end of float's range
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 c += (double)e[0][j]; c += (double)e[1][j]; c += (double)e[2][j];
@@ -150,6 +170,8 @@ __global__ void k_error_sums(const float *__restrict__ ref, const float *__restr
             }
         }
     }
+    c += rc.value();
+    al += ra.value();
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         c += __shfl_down_sync(0xffffffffu, c, o);

@@ -52,3 +52,20 @@ def test_error_sums_match_float64(ctx, w, h, offset, mode):
     a[0] = np.inf
     got, want = sums(a, b), ref(a, b)
     assert got[0] == want[0] == np.inf and np.isclose(got[1], want[1], rtol=2.4e-10)
+
+
+def test_error_sums_lose_no_bits_of_double(ctx):
+    """One step of the kernel, squares of unlike size: the sums of a thread's 12 and 4 terms are as exact as double
+    additions make them, 2^-53 for each; and of a whole image, whose longest chain of additions in double would be the
+    112 terms of a thread and the 26 of its CTA and the atomics'."""
+    import math
+    for w, h, seeds, steps in [(2, 2, 64, 12), (1024, 1024, 2, 200)]:
+        n = w * h
+        for seed in range(seeds):
+            rng = np.random.default_rng(seed)
+            a = (rng.random(4 * n) * 10.0 ** -rng.uniform(0, 4, 4 * n)).astype(np.float32)
+            d = torch.from_numpy(a).cuda()
+            got = ctx.error_sums(d, torch.zeros_like(d), w, h).cpu().numpy()
+            terms = (a * a).reshape(4, n)
+            for have, want in zip(got, (math.fsum(map(float, terms[:3].reshape(-1))), math.fsum(map(float, terms[3])))):
+                assert abs(have - want) <= steps * 2.0 ** -53 * want, (w, seed)
