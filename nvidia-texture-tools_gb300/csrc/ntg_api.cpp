@@ -747,6 +747,14 @@ int launch_encode(int format, const EncJob *d_jobs, int njobs, long long nblocks
     return launched(r, "encoder launch");
 }
 
+// The full BC1 fit of the blocks that the pruned one listed.
+int bc1_listed(const EncJob *d_jobs, int njobs, const long long *list, const unsigned long long *d_count, long long max_count,
+               bool transformed, cudaStream_t s) {
+    NTG_TRY(launched(launch_bc1_list(d_jobs, njobs, list, d_count, max_count, transformed, s), "full fit of the listed blocks"));
+    if (!bc1_list_may_be_long(max_count, transformed)) return NTG_OK;
+    return launched(launch_bc1_long_list(d_jobs, njobs, list, d_count, max_count, s), "full fit of a long list");
+}
+
 // Encode jobs of a chain's levels from..to - 1: level 0 from the input bytes (through the composed transform tables),
 // the other levels from the workspace.
 void chain_jobs(const ChainPlan &P, const uint32_t *d_bgra, const ntg_chain_options &o, const XformTables *xt,
@@ -1281,7 +1289,7 @@ static int chain_learned(ntg_context *ctx, ntg_mlp *mlp, const void *d_bgra, int
         NTG_TRY(launched(launch_bc3_list(ctx->d_jobs, nj, list, stats + 1, nblocks, s), "full fit of the listed blocks"));
     } else {
         NTG_TRY(launched(launch_bc1_learned(ctx->d_jobs, nj, nblocks, y, radius, margin, list, stats, s), "pruned fit"));
-        NTG_TRY(launched(launch_bc1_list(ctx->d_jobs, nj, list, stats + 1, nblocks, s), "full fit of the listed blocks"));
+        NTG_TRY(bc1_listed(ctx->d_jobs, nj, list, stats + 1, nblocks, opt->out_xform != NTG_XFORM_NONE && nj > 1, s));
     }
     if (h_stats) {
         NTG_CUDA(cudaMemcpyAsync(h_stats, stats, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
@@ -1663,7 +1671,8 @@ int batch_plan(ntg_batch *b) {
     NTG_CUDA(cudaMemcpy(de, ejobs.data(), ejobs.size() * sizeof(EncJob), cudaMemcpyHostToDevice));
     b->launches = (int)b->encodes.size();
     for (const auto &e : b->encodes)
-        if (learned_group(b, e)) b->launches += 3;  // features, network, pruned fit, full-fit list
+        if (learned_group(b, e))  // features, network, pruned fit, full-fit list (for BC1 a second one where it may be long)
+            b->launches += 3 + (e.format == NTG_FORMAT_BC1 && bc1_list_may_be_long(e.nblocks, e.transformed));
     for (const auto &st : b->stages) b->launches += (int)st.size();
     return NTG_OK;
 }
@@ -1695,7 +1704,7 @@ int batch_encodes(ntg_batch *b, cudaStream_t s, int only_slot = -1) {
             } else {
                 NTG_TRY(launched(launch_bc1_learned(jobs, e.njobs, e.nblocks, y, b->radius[k], b->margin[k], list, stats, s),
                                  "pruned fit"));
-                NTG_TRY(launched(launch_bc1_list(jobs, e.njobs, list, stats + 1, e.nblocks, s), "full fit of the listed blocks"));
+                NTG_TRY(bc1_listed(jobs, e.njobs, list, stats + 1, e.nblocks, e.transformed, s));
             }
             continue;
         }

@@ -8,6 +8,7 @@
 // (k_bc1_box) and the learned path's kernels take one block per thread, the block's texels, reduced
 // colours and summed-area table in shared memory.
 // Built with --fmad=false: results are bit-identical to the reference's scalar build.
+#include <algorithm>
 #include <memory>
 
 #include "ntg.h"
@@ -951,12 +952,14 @@ __device__ __forceinline__ float4 gather_texel(const EncJob &J, int blk, int k) 
 #define NTG_BC1_MIN_CTAS 5
 #endif
 
-// icbc Level8 (LEVEL 7) and Level9 (LEVEL 8).
-template <int LEVEL>
+// icbc Level8 (LEVEL 7) and Level9 (LEVEL 8). LIST: a subset of the jobs' blocks (the learned path's fallbacks), the first
+// *count of at most nblocks entries of `list`, if there are fewer than `limit` of them: the length is known on the device
+// alone (see launch_bc1_list).
+template <int LEVEL, bool LIST>
 __global__ void __launch_bounds__(32 * kFitWarps, NTG_BC1_MIN_CTAS) k_bc1(const EncJob *__restrict__ jobs, int njobs, long long nblocks,
                                                                          const long long *__restrict__ list,
                                                                          const unsigned long long *__restrict__ count,
-                                                                         int per_warp) {
+                                                                         int per_warp, long long limit) {
     __shared__ WarpScratch scratch[kFitWarps];
     __shared__ float unit8[LEVEL == 8 ? 256 : 1];
     if (LEVEL == 8) {
@@ -966,61 +969,63 @@ __global__ void __launch_bounds__(32 * kFitWarps, NTG_BC1_MIN_CTAS) k_bc1(const 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     WarpScratch &w = scratch[warp];
     const Half H{lane & 15, lane & 16, &w.half[lane >> 4]};
-    // `list`: a subset of the jobs' blocks (the learned path's fallbacks), *count long
-    const long long total = list ? min(nblocks, (long long)*count) : nblocks;
-    const long long first = per_warp * ((long long)blockIdx.x * kFitWarps + warp);
-    if (first >= total) return;
-    long long gblk = first + (lane >> 4);
-    const bool live = (lane >> 4) < per_warp && gblk < total;  // a half without a block follows the other's
-    if (!live) gblk = first;
-    if (list) gblk = list[gblk];
-    const EncJob &J = jobs[find_job(jobs, njobs, gblk)];
-    const int blk = (int)(gblk - J.first_block);
-    const f3 cw = mk3(J.cw[0], J.cw[1], J.cw[2]);
-    const f3 metric = cw * cw;
-    const bool unit = __all_sync(kAll, metric.x == 1.0f && metric.y == 1.0f && metric.z == 1.0f) != 0;
-    uint8_t *const out = J.out + 8 * (size_t)blk;
-
-    const float4 texel = gather_texel(J, blk, H.hl);
-    float4 q;
-    const int cnt = half_reduce(H, texel, q);
-    const bool black = H.ballot(texel.w > 0 && is_black(xyz(texel))) != 0;
-    if (live && H.hl == 0 && cnt <= 1) store_block(out, cnt == 0 ? Block1{0, 0, 0} : single_colour(q));
-    const bool fit = live && cnt > 1;
-    if (!__any_sync(kAll, fit)) return;
-
-    // compress_dxt1_cluster_fit (src/nvtt/icbc.h:3292-3325); both fits first, then the output stage
-    // (pure functions of the texels and the endpoints, so their order does not matter)
-    half_sat(H, q, cnt, metric, 0);
-    int n3 = fit ? cnt : 0;
-    if (__any_sync(kAll, fit && black)) {
-        // skip_blacks: the other colours, moved up to the first lanes
-        const unsigned keep = H.ballot(H.hl < cnt && !is_black(xyz(q)));
-        const int src = (int)__fns(keep, 0, H.hl + 1) & 15;
-        const float4 c = make_float4(H.get(q.x, src), H.get(q.y, src), H.get(q.z, src), H.get(q.w, src));
-        if (fit && black) n3 = __popc(keep);
-        half_sat(H, c, __popc(keep), metric, 1);
-    }
 #pragma unroll 1
-    for (int b = 0; b < 2; b++) {
-        const int n4 = __shfl_sync(kAll, fit ? cnt : 0, 16 * b), bn3 = __shfl_sync(kAll, n3, 16 * b);
-        const bool own3 = __shfl_sync(kAll, (int)black, 16 * b) != 0;
-        if (n4 > 0) warp_fit(w, b, n4, bn3, own3, unit);
+    for (int pass = 0; pass == 0 || LIST; pass++) {
+        const long long total = LIST ? min(nblocks, (long long)*count) : nblocks;  // not kept in a register over the pass
+        const long long first = per_warp * (((LIST ? (long long)pass * gridDim.x : 0) + blockIdx.x) * kFitWarps + warp);
+        if (first >= total || (LIST && total >= limit)) return;
+        long long gblk = first + (lane >> 4);
+        const bool live = (lane >> 4) < per_warp && gblk < total;  // a half without a block follows the other's
+        if (!live) gblk = first;
+        if (LIST) gblk = list[gblk];
+        const EncJob &J = jobs[find_job(jobs, njobs, gblk)];
+        const int blk = (int)(gblk - J.first_block);
+        const f3 cw = mk3(J.cw[0], J.cw[1], J.cw[2]);
+        const f3 metric = cw * cw;
+        const bool unit = __all_sync(kAll, metric.x == 1.0f && metric.y == 1.0f && metric.z == 1.0f) != 0;
+        uint8_t *const out = J.out + 8 * (size_t)blk;
+
+        const float4 texel = gather_texel(J, blk, H.hl);
+        float4 q;
+        const int cnt = half_reduce(H, texel, q);
+        const bool black = H.ballot(texel.w > 0 && is_black(xyz(texel))) != 0;
+        if (live && H.hl == 0 && cnt <= 1) store_block(out, cnt == 0 ? Block1{0, 0, 0} : single_colour(q));
+        const bool fit = live && cnt > 1;
+        if (!__any_sync(kAll, fit)) continue;
+
+        // compress_dxt1_cluster_fit (src/nvtt/icbc.h:3292-3325); both fits first, then the output stage
+        // (pure functions of the texels and the endpoints, so their order does not matter)
+        half_sat(H, q, cnt, metric, 0);
+        int n3 = fit ? cnt : 0;
+        if (__any_sync(kAll, fit && black)) {
+            // skip_blacks: the other colours, moved up to the first lanes
+            const unsigned keep = H.ballot(H.hl < cnt && !is_black(xyz(q)));
+            const int src = (int)__fns(keep, 0, H.hl + 1) & 15;
+            const float4 c = make_float4(H.get(q.x, src), H.get(q.y, src), H.get(q.z, src), H.get(q.w, src));
+            if (fit && black) n3 = __popc(keep);
+            half_sat(H, c, __popc(keep), metric, 1);
+        }
+#pragma unroll 1
+        for (int b = 0; b < 2; b++) {
+            const int n4 = __shfl_sync(kAll, fit ? cnt : 0, 16 * b), bn3 = __shfl_sync(kAll, n3, 16 * b);
+            const bool own3 = __shfl_sync(kAll, (int)black, 16 * b) != 0;
+            if (n4 > 0) warp_fit(w, b, n4, bn3, own3, unit);
+        }
+        const float *const ends = H.s->ends;
+        const f3 s0 = mk3(ends[0], ends[1], ends[2]), s1 = mk3(ends[3], ends[4], ends[5]);
+        const f3 t0 = mk3(ends[6], ends[7], ends[8]), t1 = mk3(ends[9], ends[10], ends[11]);
+        Block1 cf, c3;
+        float cerr = half_output<true>(H, texel, cw, s0, s1, cf);
+        const float e3 = half_output<false>(H, texel, cw, t0, t1, c3);
+        if (n3 > 0 && e3 < cerr) { cerr = e3; cf = c3; }
+        // taken only when its error compares below FLT_MAX: a NaN error leaves the block as the
+        // reference leaves it unwritten (this build writes zeros there)
+        Block1 o{0, 0, 0};
+        float err = FLT_MAX;
+        if (cerr < err) { o = cf; err = cerr; }
+        if (LEVEL == 8) err = half_refine(H, texel, cw, err, o, fit, unit8);
+        if (fit && H.hl == 0) store_block(out, o);
     }
-    const float *const ends = H.s->ends;
-    const f3 s0 = mk3(ends[0], ends[1], ends[2]), s1 = mk3(ends[3], ends[4], ends[5]);
-    const f3 t0 = mk3(ends[6], ends[7], ends[8]), t1 = mk3(ends[9], ends[10], ends[11]);
-    Block1 cf, c3;
-    float cerr = half_output<true>(H, texel, cw, s0, s1, cf);
-    const float e3 = half_output<false>(H, texel, cw, t0, t1, c3);
-    if (n3 > 0 && e3 < cerr) { cerr = e3; cf = c3; }
-    // taken only when its error compares below FLT_MAX: a NaN error leaves the block as the
-    // reference leaves it unwritten (this build writes zeros there)
-    Block1 o{0, 0, 0};
-    float err = FLT_MAX;
-    if (cerr < err) { o = cf; err = cerr; }
-    if (LEVEL == 8) err = half_refine(H, texel, cw, err, o, fit, unit8);
-    if (fit && H.hl == 0) store_block(out, o);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1037,6 +1042,7 @@ __global__ void __launch_bounds__(32 * kFitWarps, NTG_BC1_MIN_CTAS) k_bc1(const 
 // repeats, 2048x2048 1,386 and 1,960. Every ordering evaluated exactly, one thread per block: 1,318, 1,326, 4,878, 1,650.
 constexpr int kLaneThreads = 64;
 constexpr long long kLaneBlocks = 150000;  // launches from here on, without an output transform on float texels
+constexpr size_t kLaneBytes = (size_t)kLaneThreads * (17 * sizeof(float4) + kLaneWords * sizeof(uint32_t));
 static __device__ LanePairs g_lane_pairs;
 
 // One of the cluster fits of each lane's n colours (0: none; all lanes call it) by the warp: the end points to `ends`.
@@ -1112,16 +1118,22 @@ __device__ __noinline__ void lane_fit(const Lane<float4> &col, int n, bool prepa
     ends[0] = ea.x; ends[1] = ea.y; ends[2] = ea.z; ends[3] = eb.x; ends[4] = eb.y; ends[5] = eb.z;
 }
 
-// icbc Level8.
-__global__ void __launch_bounds__(kLaneThreads, 8) k_bc1_lane(const EncJob *__restrict__ jobs, int njobs, long long nblocks) {
+// icbc Level8. LIST: the blocks of a list as in k_bc1, if there are kLaneBlocks of them or more.
+template <bool LIST>
+__global__ void __launch_bounds__(kLaneThreads, 8) k_bc1_lane(const EncJob *__restrict__ jobs, int njobs, long long nblocks,
+                                                              const long long *__restrict__ list,
+                                                              const unsigned long long *__restrict__ count) {
     extern __shared__ float4 smem[];
     __shared__ unsigned long long best[kLaneThreads / 32][32];
     __shared__ uint16_t queue[kLaneThreads / 32][64];
     const int T = kLaneThreads;
     const int t = threadIdx.x;
+    const long long total = LIST ? min(nblocks, (long long)*count) : nblocks;
     long long gblk = (long long)blockIdx.x * T + t;
-    const bool live = gblk < nblocks;  // the others stay for the warp's evaluations
-    if (!live) gblk = nblocks - 1;
+    if (LIST && (total < kLaneBlocks || gblk - t >= total)) return;
+    const bool live = gblk < total;  // the others stay for the warp's evaluations
+    if (!live) gblk = total - 1;
+    if (LIST) gblk = list[gblk];
     const EncJob &J = jobs[find_job(jobs, njobs, gblk)];
     const int blk = (int)(gblk - J.first_block);
     // texels, then reduced colours, then the summed-area table, each in the place of the one before
@@ -1668,22 +1680,21 @@ static size_t bc1_fit_smem(int T) { return (size_t)T * 17 * sizeof(float4); }
 static size_t bc1_work_smem(int T) { return (size_t)T * (16 * sizeof(float4) + 16 * sizeof(float)); }
 
 template <int LEVEL>
-static int launch_bc1_fit(const EncJob *d_jobs, int njobs, long long nblocks, const long long *list, const unsigned long long *count,
-                          cudaStream_t stream) {
+static int launch_bc1_fit(const EncJob *d_jobs, int njobs, long long nblocks, cudaStream_t stream) {
     const int per_warp = fit_blocks_per_warp(nblocks), per = per_warp * kFitWarps;
-    k_bc1<LEVEL><<<(unsigned)((nblocks + per - 1) / per), 32 * kFitWarps, 0, stream>>>(d_jobs, njobs, nblocks, list, count, per_warp);
+    k_bc1<LEVEL, false><<<(unsigned)((nblocks + per - 1) / per), 32 * kFitWarps, 0, stream>>>(d_jobs, njobs, nblocks, nullptr, nullptr, per_warp, 0);
     return launch_status();
 }
 
 int launch_bc1(const EncJob *d_jobs, int njobs, long long nblocks, int quality, int threads, bool transformed, cudaStream_t stream) {
     if (nblocks == 0) return 0;
     if (quality == 1 && nblocks >= kLaneBlocks && !transformed) {
-        const size_t bytes = (size_t)kLaneThreads * (17 * sizeof(float4) + kLaneWords * sizeof(uint32_t));
-        k_bc1_lane<<<(unsigned)((nblocks + kLaneThreads - 1) / kLaneThreads), kLaneThreads, bytes, stream>>>(d_jobs, njobs, nblocks);
+        k_bc1_lane<false><<<(unsigned)((nblocks + kLaneThreads - 1) / kLaneThreads), kLaneThreads, kLaneBytes, stream>>>(d_jobs, njobs, nblocks,
+                                                                                                                     nullptr, nullptr);
         return launch_status();
     }
-    if (quality == 2) return launch_bc1_fit<8>(d_jobs, njobs, nblocks, nullptr, nullptr, stream);
-    if (quality != 0) return launch_bc1_fit<7>(d_jobs, njobs, nblocks, nullptr, nullptr, stream);
+    if (quality == 2) return launch_bc1_fit<8>(d_jobs, njobs, nblocks, stream);
+    if (quality != 0) return launch_bc1_fit<7>(d_jobs, njobs, nblocks, stream);
     const int T = threads == 32 ? 32 : 64;  // blocks per CTA (one thread per 4x4 block)
     k_bc1_box<<<(unsigned)((nblocks + T - 1) / T), T, bc1_fit_smem(T), stream>>>(d_jobs, njobs, nblocks);
     return launch_status();
@@ -1732,12 +1743,29 @@ int launch_bc1_work(const EncJob *d_jobs, int njobs, long long nblocks, unsigned
     return launch_status();
 }
 
-// The full Level8 fit over a list of blocks of the jobs (the learned path's fallbacks); the list's
-// length stays on the device, so the sequence needs no host round trip.
+// The full Level8 fit over a list of blocks of the jobs (the learned path's fallbacks). The list's length stays on the device,
+// so the sequence needs no host round trip: k_bc1's warps stride over a list below kLaneBlocks, and where longer ones may come
+// (not with an output transform on float texels, `transformed`) launch_bc1_long_list takes those. Most calls list few blocks
+// or none, and a grid of warps for every block that might be listed cost an 8192x8192 chain with none 340 of 10,970 us; with
+// 6,080 CTAs at most 50 us remain (10,690; 10,650 with the list's full fit by one thread per block). All of its blocks listed: 36.8 ms by such a
+// grid, 38.4 by warps that stride, 32.5 by k_bc1_lane, 37.1 with one thread per block and every ordering evaluated exactly.
+bool bc1_list_may_be_long(long long max_count, bool transformed) { return max_count >= kLaneBlocks && !transformed; }
+
 int launch_bc1_list(const EncJob *d_jobs, int njobs, const long long *list, const unsigned long long *d_count,
-                    long long max_count, cudaStream_t s) {
+                    long long max_count, bool transformed, cudaStream_t s) {
     if (max_count == 0) return 0;
-    return launch_bc1_fit<7>(d_jobs, njobs, max_count, list, d_count, s);
+    const int per_warp = fit_blocks_per_warp(max_count), per = per_warp * kFitWarps;
+    const long long limit = bc1_list_may_be_long(max_count, transformed) ? kLaneBlocks : max_count + 1;
+    const long long grid = std::min<long long>((max_count + per - 1) / per, 8 * 152 * NTG_BC1_MIN_CTAS);
+    k_bc1<7, true><<<(unsigned)grid, 32 * kFitWarps, 0, s>>>(d_jobs, njobs, max_count, list, d_count, per_warp, limit);
+    return launch_status();
+}
+
+int launch_bc1_long_list(const EncJob *d_jobs, int njobs, const long long *list, const unsigned long long *d_count,
+                         long long max_count, cudaStream_t s) {
+    k_bc1_lane<true><<<(unsigned)((max_count + kLaneThreads - 1) / kLaneThreads), kLaneThreads, kLaneBytes, s>>>(d_jobs, njobs, max_count,
+                                                                                                              list, d_count);
+    return launch_status();
 }
 
 int upload_tables_bc1(const HostTables &t) {

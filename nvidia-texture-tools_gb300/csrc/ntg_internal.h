@@ -95,9 +95,13 @@ int launch_bc3_list(const EncJob *d_jobs, int njobs, const long long *list, cons
 // Orderings the Level8 fit evaluates over the jobs' blocks (four-cluster, three-cluster), added to
 // work[0], work[1] (measurement only).
 int launch_bc1_work(const EncJob *d_jobs, int njobs, long long nblocks, unsigned long long *work, cudaStream_t s);
-// The full fit over the first *d_count entries of `list` (at most max_count; no host round trip).
+// The full fit over the first *d_count entries of `list` (at most max_count; no host round trip). `transformed` as in
+// launch_bc1. Where bc1_list_may_be_long, launch_bc1_long_list too: by the length one of the two does the work.
 int launch_bc1_list(const EncJob *d_jobs, int njobs, const long long *list, const unsigned long long *d_count,
-                    long long max_count, cudaStream_t s);
+                    long long max_count, bool transformed, cudaStream_t s);
+bool bc1_list_may_be_long(long long max_count, bool transformed);
+int launch_bc1_long_list(const EncJob *d_jobs, int njobs, const long long *list, const unsigned long long *d_count,
+                         long long max_count, cudaStream_t s);
 }  // namespace ntg
 struct ntg_mlp;
 struct ntg_context;

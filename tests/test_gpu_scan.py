@@ -100,3 +100,20 @@ def test_bc1_one_block_per_thread(ctx, oracle, kind):
     for alpha, cw in [(1, (1, 1, 1)), (0, (0.6, 1.0, 0.4))]:
         got = ctx.encode(ntg.FORMAT_BC1, torch.from_numpy(img).cuda(), w, h, quality=1, alpha_mode=alpha, cw=cw)
         assert np.array_equal(got.cpu().numpy(), oracle.bc1_image(img, w, h, alpha, 1, cw=cw, threads=16)), alpha
+
+
+@pytest.mark.parametrize("xform", [ntg.XFORM_NONE, ntg.XFORM_SRGB])
+@pytest.mark.parametrize("size", [8, 200, 700, 1700])
+def test_listed_blocks_get_the_full_fit(ctx, size, xform):
+    """The learned path's fallbacks: with a margin that lists every block the result is the plain fit's, at 1700x1700 from lists
+    of more than 150,000 blocks (240,833), which a kernel of their own takes, or with a transform more blocks than the grid."""
+    rng = np.random.default_rng(size)
+    img = torch.from_numpy(rng.integers(0, 256, (size, size, 4), dtype=np.uint8)).cuda()
+    opt = ntg.ChainOptions.make(format=ntg.FORMAT_BC1, in_xform=xform, out_xform=xform)
+    net = ntg.MLP(seed=1)
+    try:
+        got, stats = ctx.compress_chain_learned(net, img, size, size, opt, radius=1, margin=-1.0)
+        assert size == 8 or stats["full_fit"] > 9 * stats["kept"]  # a block that its palette holds exactly is not listed
+        assert torch.equal(got, ctx.compress_chain(img, size, size, opt))
+    finally:
+        net.close()
