@@ -117,3 +117,18 @@ def test_listed_blocks_get_the_full_fit(ctx, size, xform):
         assert torch.equal(got, ctx.compress_chain(img, size, size, opt))
     finally:
         net.close()
+
+
+@pytest.mark.parametrize("cw", [(3, 3, 3), (0.1, 5, 2), (100, 1, 0), (2e5, 1e6, 9e5), (1e7, 1e7, 1e7)])
+@pytest.mark.parametrize("fmt", [ntg.FORMAT_BC1, ntg.FORMAT_BC1A, ntg.FORMAT_BC3])
+def test_colour_weights_of_any_size(ctx, oracle, fmt, cw):
+    """Colour weights above 1, whose squares scale the scan's errors and bound: up to the largest that it takes (2^20)
+    and beyond it."""
+    image = {ntg.FORMAT_BC1: oracle.bc1_image, ntg.FORMAT_BC3: oracle.bc3_image,
+             ntg.FORMAT_BC1A: lambda i, w, h, alpha, q, **kw: oracle.bc1a_image(i, w, h, alpha, **kw)}[fmt]
+    w, h = 61, 130
+    for kind in KINDS:
+        img = contents(kind, w, h, len(kind))
+        for alpha in (0, 1):
+            got = ctx.encode(fmt, torch.from_numpy(img).cuda(), w, h, quality=1, alpha_mode=alpha, cw=cw)
+            assert np.array_equal(got.cpu().numpy(), image(img, w, h, alpha, 1, cw=cw, threads=8)), (kind, alpha)
