@@ -251,11 +251,14 @@ int ntg_batch_launch_alternate(ntg_batch *batch, void *stream);
 int ntg_batch_process_host(ntg_batch *batch, int count, const void *const *const *h_bgra, void *const *const *h_blocks,
                            void *stream);
 /* Times candidate launch shapes on this batch (rows per strip and threads per CTA of the 2:1 mip
- * kernel, the tail threshold, blocks per CTA of each encoder), keeps the fastest, recaptures the
- * graph and stores the choice in the tuning cache. Synchronises `stream`. */
+ * kernel, the tail threshold, blocks per CTA of each encoder that takes one thread per block), keeps
+ * the fastest, recaptures the graph and stores the choice in the tuning cache. Synchronises
+ * `stream`. */
 int ntg_batch_autotune(ntg_batch *batch, void *stream);
 /* Texels of all levels, 4x4 blocks, kernel launches per replay, and the launch shapes in use:
  * shape[] = {strip, threads, tail texels, bc1 blocks/CTA, bc3 blocks/CTA, bc5 blocks/CTA}.
+ * The BC1 entry shapes Fastest launches only, the BC3 entry (BC3, BC1a) Fastest and Highest and
+ * launches above 68,096 blocks; the other kernels fix their own shape, and the entry is unused.
  * Any pointer may be NULL. */
 int ntg_batch_info(const ntg_batch *batch, long long *texels, long long *blocks, int *launches, int shape[6]);
 /* Runs the batch's phases once each, outside the graph, timed with CUDA events on `stream`:

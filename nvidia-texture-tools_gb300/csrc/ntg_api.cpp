@@ -603,13 +603,14 @@ void group_launches(const std::vector<std::pair<MipKey, MipJob>> &items, const M
     }
 }
 
+bool narrow_filter(const ChainPlan &P) { return P.fast_box || P.width <= 1.0f; }
+
 // First destination level of a chain that its tail launch computes (lv.size() = no tail).
 // A narrow filter's tail begins at sources four times larger (64x64 instead of 32x32): a tail level's time grows with its
 // taps, a launch's does not. Measured for chains from 64 to 512 texels wide: box and triangle 2 to 4 us faster from 64x64,
 // Kaiser (13 taps) 2 us slower.
 size_t tail_start(const ChainPlan &P, const MipTuning &tune) {
-    const bool narrow = P.fast_box || P.width <= 1.0f;
-    const long long limit = std::min<long long>(tune.tail_texels * (narrow ? 4 : 1), tail_max_texels());
+    const long long limit = std::min<long long>((long long)tune.tail_texels * (narrow_filter(P) ? 4 : 1), tail_max_texels());
     for (size_t l = 1; l < P.lv.size(); l++) {
         const Level &S = P.lv[l - 1];
         // the X pass plane (H x max(1, W/2)) must fit the tail's half-size buffer as well: a 1-wide
@@ -2050,9 +2051,13 @@ int ntg_batch_autotune(ntg_batch *b, void *stream) {
     const MipTuning keep = b->tune;
     MipTuning best = keep;
     float best_ms = 1e30f;
+    // narrow filters' tails begin at 4,096 texels with either threshold (tail_start)
+    bool wide = false;
+    for (const ChainPlan &P : b->plans) wide = wide || !narrow_filter(P);
     for (int tail : {1024, 4096})
         for (int threads : {256, 512})
             for (int strip : {8, 16, 32}) {
+                if (tail > 1024 && !wide) continue;
                 b->tune.strip = strip;
                 b->tune.threads = threads;
                 b->tune.tail_texels = tail;
@@ -2063,12 +2068,21 @@ int ntg_batch_autotune(ntg_batch *b, void *stream) {
             }
     b->tune = best;
     NTG_TRY(batch_plan(b));
-    // encoder blocks per CTA, per format present
+    // encoder blocks per CTA, per format present; one run where no launch reads them, the shape kept
     float enc_total = 0;
     for (int slot = 0; slot < 3; slot++) {
-        bool present = false;
-        for (const auto &e : b->encodes) present = present || enc_slot(e.format) == slot;
+        bool present = false, shaped = false;
+        for (const auto &e : b->encodes) {
+            if (enc_slot(e.format) != slot) continue;
+            present = true;
+            shaped = shaped || (!learned_group(b, e) && encoder_takes_threads(e.format, e.quality, e.nblocks));
+        }
         if (!present) continue;
+        if (!shaped) {
+            enc_total += time_ms(s, [&] { return batch_encodes(b, s, slot); }, 1, &status);
+            NTG_TRY(status);
+            continue;
+        }
         int best_t = b->enc_threads[slot];
         float best_e = 1e30f;
         for (int threads : {32, 64, 128}) {

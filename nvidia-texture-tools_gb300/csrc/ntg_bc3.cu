@@ -1439,6 +1439,13 @@ int launch_bc3_list(const EncJob *d_jobs, int njobs, const long long *list, cons
 // 180, 1024x1024 (65,536) 382 and 365, 2048x2048 1,185 and 1,500; BC1a: 256x256 194 and 45, 1024x1024 392 and 337.
 constexpr long long kSquishWarpBlocks = 68096;
 
+bool encoder_takes_threads(int format, int quality, long long nblocks) {
+    if (format == NTG_FORMAT_BC1) return quality == 0;
+    if (format == NTG_FORMAT_BC1A) return nblocks > kSquishWarpBlocks;
+    if (format == NTG_FORMAT_BC3) return quality == 0 || quality == 3 || nblocks > kSquishWarpBlocks;
+    return true;
+}
+
 template <bool DXT1>
 static int launch_squish(const EncJob *d_jobs, int njobs, long long nblocks, cudaStream_t stream) {
     const int per_warp = fit_blocks_per_warp(nblocks), per = per_warp * kFitWarps;

@@ -64,7 +64,9 @@ struct EncJob {
     long long first_block;    // index of this job's first block in the launch
 };
 
-// threads = blocks per CTA (one thread per 4x4 block); 0 = the default shape.
+// threads = blocks per CTA of the kernels that take one thread per 4x4 block; 0 = the default shape. Ignored by the others, the
+// warps' kernels and k_bc1_lane: encoder_takes_threads says whether a launch reads it.
+bool encoder_takes_threads(int format, int quality, long long nblocks);
 // `transformed`: some job applies an output transform to float texels as it gathers them.
 int launch_bc1(const EncJob *d_jobs, int njobs, long long nblocks, int quality, int threads, bool transformed, cudaStream_t s);
 int launch_bc3(const EncJob *d_jobs, int njobs, long long nblocks, int quality, int threads, cudaStream_t s);

@@ -289,3 +289,33 @@ def test_count_work_orderings(ctx, tmp_path, monkeypatch):
         assert b.count_work() == (968 + 968, 152 + 44)
     finally:
         b.close()
+
+
+@pytest.mark.parametrize("fastest", [False, True])
+def test_autotune_leaves_unread_shapes(ctx, tmp_path, monkeypatch, fastest):
+    """Encoder shapes that no launch of the batch reads are neither swept nor replaced: a cached one that the sweep would not
+    choose (96 blocks per CTA) survives for BC1 at Normal and small BC3 launches, but not where Fastest ones read it."""
+    cache = tmp_path / "tune.json"
+    monkeypatch.setenv("NTG_TUNE_CACHE", str(cache))
+    plain = {1: (1, 2), 2: (1, 2), 4: (1, 2), 6: (1, 2), 7: (1, 2)}
+    _, textures, refs = make_batch(ctx, [c for c in MIXED if fastest or c[3] in plain[c[2]]], 600)
+    b = ntg.Batch(ctx, textures)
+    b.autotune()
+    b.close()
+    doc = json.loads(cache.read_text())
+    doc["entries"][0].update(bc1=96, bc3=96, bc5=96)
+    cache.write_text(json.dumps(doc))
+    b = ntg.Batch(ctx, textures)
+    try:
+        shape = [b.info()["shape"][k] for k in ("bc1_blocks_per_cta", "bc3_blocks_per_cta", "bc5_blocks_per_cta")]
+        assert shape == [96, 96, 96]
+        b.autotune()
+        shape = [b.info()["shape"][k] for k in ("bc1_blocks_per_cta", "bc3_blocks_per_cta", "bc5_blocks_per_cta")]
+        assert [v == 96 for v in shape] == [not fastest, not fastest, False]
+        for t in textures:
+            t[4].zero_()
+        b.launch()
+        for t, r in zip(textures, refs):
+            assert np.array_equal(host(t[4]), r)
+    finally:
+        b.close()
