@@ -797,10 +797,11 @@ void chain_jobs(const ChainPlan &P, const uint32_t *d_bgra, const ntg_chain_opti
 //   else: levels 0 and 1, as soon as level 1 is there, beside all the other levels' filters and their encoding, which go
 //     to the side stream. (Level 0 alone, from the start: the filters' large CTAs then wait for SMs that the encoder
 //     keeps full; 2048x2048 BC1 with Kaiser mips gained 14 us of 1,838 that way and 41 this way.)
-// Measured, BC1 unless stated, one after the other / beside the tail / beside the filters, us: 64x64 40 / 35 / 37, 256x256
-// 65 / 56 / 74, 384x384 106 / 98 / 98, 512x512 155 / 145 / 135, 1024x1024 473 / 461 / 451; BC3 256x256 101 / 80 / 92, 512x512
+// Measured, BC1 unless stated, one after the other / beside the tail / beside the filters, us: 256x256 65 / 56 / 74, 384x384 106 / 98 / 98, 512x512 155 / 145 / 135, 1024x1024 473 / 461 / 451; BC3 256x256 101 / 80 / 92, 512x512
 // 177 / 157 / 148, 2048x2048 (k_bc3, whose CTAs hold their SM for 0.4 ms) 1,542 / 1,543 / 1,579; BC5 1024x1024 107 / 100 /
 // 109, 1500x1500 163 / 157 / 154, 2048x2048 235 / 227 / 195; Fastest BC1 1024x1024 73 / 66 / 74.
+// Small ones with box, triangle and Kaiser mips, one after the other / beside the tail: 64x64 34 / 34, 40 / 40, 48 / 44,
+// 96x96 37 / 34, 45 / 42, 53 / 45; BC5 64x64 45 / 43, 51 / 46, 59 / 48, 96x96 46 / 39, 55 / 44, 62 / 48; 32x32 within 1 us.
 struct Overlap {
     size_t split = 0;  // levels of the first launch; 0: no overlap
     bool beside_tail = false;
@@ -816,7 +817,9 @@ Overlap chain_overlap(const ChainPlan &P, const ntg_chain_options &o, size_t tai
     else
         deep = first >= 131072;
     Overlap v;
-    if (first < 1024) return v;  // smaller ones gain nothing: tail and encoder are one CTA's and one warp's time either way
+    // smaller ones gain nothing: one CTA's time in the tail, one warp's in a fit, and the event between the streams
+    const bool fit = o.format == NTG_FORMAT_BC1 || o.format == NTG_FORMAT_BC1A || o.format == NTG_FORMAT_BC3;
+    if (first < (fit && narrow_filter(P) ? 400 : 200)) return v;
     v.beside_tail = !deep;
     v.split = deep ? std::min<size_t>(tail, 2) : tail;
     if (v.split >= P.lv.size()) v.split = 0;

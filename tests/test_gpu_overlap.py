@@ -162,3 +162,15 @@ def test_levels_over_the_image(ctx, filt, where):
         inside = buf[at:at + w * h]
         inside.copy_(img.reshape(-1).view(torch.float32))
         assert torch.equal(ctx.mip_chain(inside, w, h, opt, out=buf), want), (w, h)
+
+
+@pytest.mark.parametrize("fmt", [ntg.FORMAT_BC1, ntg.FORMAT_BC1A, ntg.FORMAT_BC3, ntg.FORMAT_BC4, ntg.FORMAT_BC5])
+@pytest.mark.parametrize("filt", [ntg.FILTER_BOX, ntg.FILTER_KAISER])
+def test_small(ctx, fmt, filt):
+    """Both sides of the smallest overlapped chains, 200 and 400 blocks."""
+    for i, (w, h) in enumerate([(56, 55), (57, 53), (79, 80), (81, 76), (97, 66), (800, 4), (3, 801)]):
+        img = image(w, h, i)
+        for x, levels in [(ntg.XFORM_SRGB, 0), (ntg.XFORM_NONE, 3)]:
+            opt = ntg.ChainOptions.make(format=fmt, filter=filt, alpha_mode=ntg.ALPHA_TRANSPARENCY, in_xform=x, out_xform=x,
+                                        max_levels=levels)
+            assert torch.equal(ctx.compress_chain(img, w, h, opt), serial(ctx, img, w, h, opt)), (w, h, levels)
