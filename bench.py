@@ -781,10 +781,12 @@ def run_gpu_batch(args):
             ops = n4 * OPS_PER_ORDERING4 + n3 * OPS_PER_ORDERING3
             ach = ops / (phases["bc1"] / 1000.0)
             nb1 = blocks["bc1"]
+            # as launch_bc1 chooses: one block per thread from 150,000 blocks on, without a transform on float levels
+            bc1_kernel = "k_bc1_lane" if nb1 >= 150000 and not any(o[5] for _w, _h, f, o, _i in specs if f == 1) else "k_bc1<7>"
             roof = {"bound": "fp32", "achieved": ach / 1e12, "peak": peak_b / 1e12, "unit": "TFLOP/s",
                     "frac": ach / peak_b,
                     "traffic": BC1_TRAFFIC_PER_BLOCK * nb1 if nb1 and BC1_TRAFFIC_PER_BLOCK else None,
-                    "kernel": "k_bc1_lane (icbc Level8 cluster fit)",
+                    "kernel": f"{bc1_kernel} (icbc Level8 cluster fit)",
                     "note": f"peak = 152 SMs x 128 FP32 lanes x median SM clock {sm_mhz_b:.0f} MHz; {n4} four-cluster x "
                             f"{OPS_PER_ORDERING4} + {n3} three-cluster x {OPS_PER_ORDERING3} FP32 instructions of the scan over the BC1 phase "
                             f"({phases['bc1']:.3f} ms, one run outside the graph, CUDA events); traffic: DRAM bytes per "

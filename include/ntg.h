@@ -295,7 +295,8 @@ int ntg_batch_destroy(ntg_batch *batch);
  * W3 [8 x 256], b3 [8] (weights row-major, out x in). Training is Adam (beta 0.9 / 0.999, eps 1e-8)
  * on the weighted mean squared error of the outputs (weights 1 for the endpoints, 0.25 for the
  * error, 0 for output 7). Device buffers: x [batch x 48], targets [batch x 8], y [batch x 16]
- * (columns 8-15 zero), all FP32 row-major; batch a multiple of 8. */
+ * (columns 8-15 zero), all FP32 row-major; training batches are multiples of 8 (others are refused
+ * with NTG_ERROR_INVALID_INPUT). */
 typedef struct ntg_mlp ntg_mlp;
 int ntg_mlp_create(int device, unsigned long long seed, ntg_mlp **out);
 int ntg_mlp_destroy(ntg_mlp *mlp);
@@ -305,7 +306,7 @@ int ntg_mlp_set_params(ntg_mlp *mlp, const float *h_params);
 /* Inference: one persistent kernel per call, the weights resident in shared memory and the three
  * layers chained through TMEM; any batch size. */
 int ntg_mlp_infer(ntg_mlp *mlp, const float *d_x, int batch, float *d_y, void *stream);
-/* The same forward pass as three separate tensor-core products (the training path). */
+/* The same forward pass as three separate tensor-core products, for testing; any batch size. */
 int ntg_mlp_infer_unfused(ntg_mlp *mlp, const float *d_x, int batch, float *d_y, void *stream);
 /* One forward + backward pass: the flat gradient (parameter layout) into d_grads (may be NULL) and
  * the loss into *h_loss (may be NULL); synchronises `stream`. */

@@ -1069,7 +1069,7 @@ __device__ __noinline__ void lane_fit(const Lane<float4> &col, int n, bool prepa
     const int start = four ? g_lane_pairs.start4[n] : g_lane_pairs.start3[n];
     int end = 0;
     if (n > 0)
-        end = lane_scan<UNIT, kLaneThreads>(table, words, blk->mu[0], blk->mu[1], blk->mu[2], blk->W, blk->eta, 0.5f * k * blk->slack, n, start, 1, k,
+        end = lane_scan<UNIT, kLaneThreads>(table, words, blk->mu[0], blk->mu[1], blk->mu[2], blk->W, blk->eta, 0.5f * k * blk->slack, n, start, k,
                                             make_float3(metric.x, metric.y, metric.z));
     constexpr uint32_t stride = 16 * kLaneThreads;
     const uint32_t table0 = table - 16 * lane;
@@ -1556,7 +1556,7 @@ __global__ void __launch_bounds__(64) k_bc1_learned(const EncJob *__restrict__ j
     if (gblk >= nblocks) return;
     const EncJob &J = jobs[find_job(jobs, njobs, gblk)];
     const int blk = (int)(gblk - J.first_block);
-    // the layout of k_bc1: colours reduced over the texels in place, the ZERO SAT built over the
+    // the layout of k_bc1_lane: colours reduced over the texels in place, the ZERO SAT built over the
     // colours in place, texels gathered again for the output stage, weights derived from the texels
     Lane<float4> in{smem + t, T};
     Lane<float4> col = in;
@@ -1639,7 +1639,7 @@ __global__ void __launch_bounds__(64) k_bc1_learned(const EncJob *__restrict__ j
 
 // Work of the Level8 fit (measurement only, outside the encoder): per block the orderings that
 // cluster_fit_four and cluster_fit_three evaluate (over the non-black colours when the block has
-// black ones), from the same gather and reduce_colors as k_bc1; summed into work[0] and work[1].
+// black ones), from the gather and reduce_colors of k_bc1_lane; summed into work[0] and work[1].
 __global__ void __launch_bounds__(64) k_bc1_work(const EncJob *__restrict__ jobs, int njobs, long long nblocks,
                                                  unsigned long long *__restrict__ work) {
     extern __shared__ float4 smem[];
@@ -1673,8 +1673,8 @@ __global__ void __launch_bounds__(64) k_bc1_work(const EncJob *__restrict__ jobs
     }
 }
 
-// Shared memory of k_bc1 and k_bc1_learned: per thread 17 float4 slots, the texels, then the
-// reduced colours, then the SAT (its weights are derived from the texels).
+// Shared memory of k_bc1_box and k_bc1_learned: per thread 17 float4 slots, the texels, then the learned fit's
+// reduced colours, then its SAT (weights are derived from the texels).
 static size_t bc1_fit_smem(int T) { return (size_t)T * 17 * sizeof(float4); }
 // k_bc1_work: per thread the texels and 16 stored weights.
 static size_t bc1_work_smem(int T) { return (size_t)T * (16 * sizeof(float4) + 16 * sizeof(float)); }
@@ -1718,7 +1718,7 @@ int launch_bc1_features(const EncJob *d_jobs, int njobs, long long nblocks, floa
 
 int launch_bc1_targets(const EncJob *d_jobs, int njobs, long long nblocks, float *tg, cudaStream_t s) {
     if (nblocks == 0) return 0;
-    const int T = 64;  // texels, colours, summed-area table and weights per thread, as k_bc1
+    const int T = 64;  // texels, colours, summed-area table and weights per thread
     static std::atomic<unsigned long long> configured{0};
     allow_smem(k_bc1_targets, bc1_smem(T), configured);
     k_bc1_targets<<<(unsigned)((nblocks + T - 1) / T), T, bc1_smem(T), s>>>(d_jobs, njobs, nblocks, tg);

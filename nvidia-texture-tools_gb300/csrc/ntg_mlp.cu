@@ -1076,7 +1076,7 @@ int ntg_mlp_infer(ntg_mlp *m, const float *d_x, int batch, float *d_y, void *str
     return mlp_forward_device(m, d_x, batch, d_y, (cudaStream_t)stream);
 }
 
-// The unfused forward pass (three k_gemm launches), as training runs it; for testing.
+// The unfused forward pass (three k_gemm launches), for testing.
 int ntg_mlp_infer_unfused(ntg_mlp *m, const float *d_x, int batch, float *d_y, void *stream) {
     if (!m || !d_x || !d_y || batch <= 0) return mlp_fail(NTG_ERROR_INVALID_INPUT, "bad arguments");
     cudaStream_t s = (cudaStream_t)stream;

@@ -424,11 +424,11 @@ __device__ __forceinline__ void store_word(uint32_t a, uint32_t v) { asm volatil
 // The scan of a block's orderings by one thread, scan_rows' arithmetic on pairs that differ in the first end only, so that
 // two of the three table entries stay in registers. `table`: the thread's summed-area table (17 entries, 16 T bytes apart);
 // `words`: its flags (4 T bytes apart): bit 2 i + h for ordering h of a word's pair i, set where the ordering's scanned error
-// is within `slack` of the lowest so far or it is hard. `start`: the walk's first pair; `last`: the lowest last end. Returns
-// the number of words, from start / 16 on.
+// is within `slack` of the lowest so far or it is hard. `start`: the walk's first pair. Returns the number of words, from
+// start / 16 on.
 template <bool UNIT, int T>
 __device__ __noinline__ int lane_scan(uint32_t table, uint32_t words, float mux, float muy, float muz, float W, float eta,
-                                        float slack, int n, int start, int last, float k, float3 metric) {
+                                        float slack, int n, int start, float k, float3 metric) {
     const uint32_t stride = 16 * T;
     const float kW = k * W, cm = 0.5f * kW, ca = rcp_approx(kW), cd = 0.5f * ca;
     const float u0 = 2.0f * k - 1.0f;
@@ -442,7 +442,7 @@ __device__ __noinline__ int lane_scan(uint32_t table, uint32_t words, float mux,
     words += 4 * T * (uint32_t)done;
     const bool three = k == 2.0f;
 #pragma unroll 1
-    for (int c2 = n; c2 >= last; c2--) {
+    for (int c2 = n; c2 >= 1; c2--) {  // the last end is never 0
         const float4 p2 = load_shared(table + c2 * stride);
 #pragma unroll 1
         for (int c1 = three ? c2 : 0; c1 <= c2; c1++) {
