@@ -28,7 +28,8 @@ inline int launch_status() {
 // How a kernel of a sequence is launched. EARLY: it may begin while the kernel before it on the stream is running, so that
 // its CTAs are resident, past their launch latency, when that one ends; that one has LETS_IN. Such kernels' first statement
 // is after_previous (ntg_device.cuh), in every thread, so that nothing they read or write is earlier than in plain stream
-// order, and they read what the kernels before them wrote through load_level, never __ldg. (Letting others in where none follows early costs a few per cent.)
+// order, and they read what the kernels before them wrote through load_level, never __ldg. (Letting others in where none
+// follows early costs a few per cent.)
 enum LaunchOrder { PLAIN = 0, LETS_IN = 1, EARLY = 2 };
 
 template <typename... P, typename... A>
